@@ -334,6 +334,71 @@ __device__ __forceinline__ unsigned warp_match_digit(unsigned d) {
     return peers;
 }
 
+// Ordered scan of tile counts inside one launch (decoupled look-back): a
+// word per tile, zeroed before the launch. Tiles are taken in launch order by
+// tickets, so a tile only waits for tiles whose blocks already run; every
+// wait is bounded, and a tile that gives up poisons its own word, so later
+// tiles stop too.
+constexpr unsigned long long LB_AGG = 1ull << 62;      // tile published its own count
+constexpr unsigned long long LB_PREFIX = 2ull << 62;   // tile published its inclusive prefix
+constexpr unsigned long long LB_POISON = 3ull << 62;   // tile gave up: everything after stops
+constexpr unsigned long long LB_VALUE = (1ull << 62) - 1;
+constexpr long long LB_WAIT_CYCLES = 1ll << 31;        // ~1 s at 2 GHz
+
+// By one (full) warp: lane l reads the word of tile p - l, so each step covers
+// 32 predecessors. (Reading 8 words per lane, 256 per step, measured slower:
+// 0.73 against 0.43 ms on the 200k x 8 SpGEMM with 2048-product tiles.)
+// Returns false if the tile had to give up (timeout, or an earlier tile gave
+// up); on a timeout `status_bit` is set in *status. Lane 0 publishes.
+__device__ __forceinline__ bool lookback_scan(unsigned long long *tstate, uint64_t t, uint64_t total, uint64_t *base,
+                                              int lane, unsigned int *status, unsigned status_bit,
+                                              long long wait_cycles) {
+    if (t == 0) {
+        if (lane == 0) atomicExch(tstate, LB_PREFIX | total);
+        *base = 0;
+        return true;
+    }
+    if (lane == 0) atomicExch(tstate + t, LB_AGG | total);
+    uint64_t excl = 0;
+    int64_t p = (int64_t)t - 1;  // nearest predecessor of the window
+    const long long t0 = clock64();
+    while (true) {
+        const int64_t q = p - lane;
+        const unsigned long long v = q >= 0 ? *(volatile unsigned long long *)(tstate + q) : 0ull;
+        const unsigned long long st = v & ~LB_VALUE;
+        const unsigned pref = __ballot_sync(0xffffffffu, q >= 0 && st == LB_PREFIX);
+        // lanes up to the nearest prefix (tile 0 always publishes one, so a
+        // window reaching q < 0 holds it at a lower lane)
+        const unsigned need = pref ? (pref & (0u - pref)) * 2u - 1u : 0xffffffffu;
+        const unsigned waiting = __ballot_sync(0xffffffffu, q >= 0 && st == 0) & need;
+        const unsigned poison = __ballot_sync(0xffffffffu, q >= 0 && st == LB_POISON) & need;
+        if (poison) {
+            if (lane == 0) atomicExch(tstate + t, LB_POISON);
+            return false;
+        }
+        if (waiting) {
+            if (clock64() - t0 > wait_cycles) {
+                if (lane == 0) {
+                    atomicOr(status, status_bit);
+                    atomicExch(tstate + t, LB_POISON);
+                }
+                return false;
+            }
+            __nanosleep(32);
+            continue;
+        }
+        unsigned long long add = ((need >> lane) & 1u) ? (v & LB_VALUE) : 0ull;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+        excl += add;
+        if (pref) break;
+        p -= 32;
+    }
+    if (lane == 0) atomicExch(tstate + t, LB_PREFIX | (excl + total));
+    *base = excl;
+    return true;
+}
+
 inline unsigned grid_for(uint64_t n, unsigned block, unsigned cap = 1u << 30) {
     uint64_t g = (n + block - 1) / block;
     if (g == 0) g = 1;
@@ -369,6 +434,19 @@ int dedup_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
                        cudaStream_t s);
 int sort_grouped_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const uint64_t *s_off, uint64_t m,
                       uint64_t n_rows, int cbits, uint64_t *keys_out, uint32_t *idx_out, bool *done, cudaStream_t s);
+
+// Row-grouped entries (row r's are [s_off[r], s_off[r+1]), columns in any
+// order) as CSR: the last write of every key in (row, column) order, zeros
+// dropped unless keep_zeros (spg_rowtiles.cu). The output arrays are sized
+// for m entries; n of them are used. *done = false when a row has more than
+// 12 288 entries; the outputs are then undefined.
+struct GroupedOut {
+    DevBuf off, cols, vals;
+    uint64_t n = 0;
+};
+int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off,
+                       uint64_t m, uint64_t n_rows, int cbits, bool keep_zeros, GroupedOut *out, bool *done,
+                       cudaStream_t s);
 
 // SpGEMM pieces shared by its variants (spg_spgemm.cu, spg_spgemm_sort.cu).
 // Expand - sort - compress output: kept entries in (row, column) order.

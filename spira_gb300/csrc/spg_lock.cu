@@ -64,10 +64,12 @@ struct RowGap {
 // VEC: rows and cols 16-byte aligned; each thread reads 4 rows and 4
 // columns per step in two 16-byte loads (the successor of its last pair
 // comes from the next lane, or one more load at the warp's edge).
+// stats[5] += a sample of the inserts that 32 others of their row follow: every
+// fourth insert, by 24 lanes of each warp's 32 (3 / 16 of all).
 template <bool VEC>
 __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, uint64_t m,
                              int cbits, unsigned *__restrict__ stats) {
-    unsigned mr = 0, mc = 0;
+    unsigned mr = 0, mc = 0, hits = 0;
     bool d = false, g = false, e = false;
     if constexpr (VEC) {
         const uint64_t n4 = m / 4;  // whole groups of 4; the tail below
@@ -81,6 +83,8 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
                 r4 = reinterpret_cast<const uint4 *>(rows)[q];
                 c4 = reinterpret_cast<const uint4 *>(cols)[q];
             }
+            const uint32_t r32 = __shfl_down_sync(0xffffffffu, r4.x, 8);
+            if (4 * q + 32 < 4 * n4 && (threadIdx.x & 31) < 24) hits += r32 == r4.x ? 1u : 0u;
             uint32_t rn = __shfl_down_sync(0xffffffffu, r4.x, 1), cn = __shfl_down_sync(0xffffffffu, c4.x, 1);
             const bool have_next = ok && 4 * q + 4 < m;
             if (have_next && ((threadIdx.x & 31) == 31 || q + 1 >= n4)) {
@@ -110,6 +114,7 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
         const uint64_t k = ((uint64_t)r << cbits) | c;
         mr = max(mr, r);
         mc = max(mc, c);
+        if (!VEC && (i & 3) == 0 && ((i >> 2) & 31) < 24 && i + 32 < m) hits += rows[i + 32] == r ? 1u : 0u;
         if (i + 1 < m) {
             const uint32_t r2 = rows[i + 1];
             const uint64_t k2 = ((uint64_t)r2 << cbits) | cols[i + 1];
@@ -123,27 +128,31 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
         mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, o));
         mc = max(mc, __shfl_xor_sync(0xffffffffu, mc, o));
     }
+    hits = __reduce_add_sync(0xffffffffu, hits);
     const unsigned flags = (__any_sync(0xffffffffu, d) ? 1u : 0u) | (__any_sync(0xffffffffu, g) ? 2u : 0u) |
                            (__any_sync(0xffffffffu, e) ? 4u : 0u);
     // one set of atomics per block: per-warp atomics on the same two words
     // serialise at L2 and cost more than the pass itself
-    __shared__ unsigned s_mr[LB / 32], s_mc[LB / 32], s_fl[LB / 32];
+    __shared__ unsigned s_mr[LB / 32], s_mc[LB / 32], s_fl[LB / 32], s_hits[LB / 32];
     const int w = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) {
         s_mr[w] = mr;
         s_mc[w] = mc;
         s_fl[w] = flags;
+        s_hits[w] = hits;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned bm = 0, bc = 0, bf = 0;
+        unsigned bm = 0, bc = 0, bf = 0, bh = 0;
         for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
             bm = max(bm, s_mr[i]);
             bc = max(bc, s_mc[i]);
             bf |= s_fl[i];
+            bh += s_hits[i];
         }
         atomicMax(stats, bm);
         atomicMax(stats + 1, bc);
+        if (bh) atomicAdd(stats + 5, bh);
         if (bf & 1u) stats[2] = 1u;
         if (bf & 2u) stats[3] = 1u;
         if (bf & 4u) stats[4] = 1u;
@@ -664,6 +673,7 @@ first_keep_gather(const uint64_t *__restrict__ keys, const uint32_t *__restrict_
 // alongside the range check.
 struct Prepared {
     unsigned unsorted = 1, ungrouped = 1, not_strict = 1;
+    uint64_t long_hits = 0;  // sampled inserts that 32 others of their row follow (3 / 16 of the inserts looked at)
     bool ready = false;
 };
 
@@ -749,6 +759,32 @@ int row_offsets(Ctx *c, const uint32_t *srows, uint64_t u, uint64_t n_rows, DevB
     return SPG_OK;
 }
 
+// Installs a first lock's CSR built in arrays sized for m entries; when more
+// than an eighth of them stayed unused the entries move to arrays of their
+// own size (build_csr: exact capacity).
+int first_install(Ctx *c, Csr *A, GroupedOut &&o, uint64_t m, cudaStream_t s) {
+    const uint64_t nnz = o.n;
+    if (nnz < m - m / 8) {
+        DevBuf cols, vals;
+        SPG_TRY(cols.alloc(csr_alloc_elems(nnz) * sizeof(uint32_t), s));
+        SPG_TRY(vals.alloc(csr_alloc_elems(nnz) * sizeof(double), s));
+        SPG_CUDA_TRY(cudaMemcpyAsync(cols.ptr, o.cols.ptr, nnz * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+        SPG_CUDA_TRY(cudaMemcpyAsync(vals.ptr, o.vals.ptr, nnz * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        o.cols = std::move(cols);
+        o.vals = std::move(vals);
+        SPG_TRY(c->phase_sync(s));
+    }
+    A->invalidate_derived();
+    A->off = std::move(o.off);
+    A->cols = std::move(o.cols);
+    A->vals = std::move(o.vals);
+    A->nnz = nnz;
+    A->capacity = nnz;  // build_csr: exact
+    A->built = true;
+    A->may_have_zeros = false;
+    return SPG_OK;
+}
+
 // First lock: sort, keep the last write of every key unless it is zero, and
 // take the offsets from the kept rows.
 int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const double *vals, uint64_t m,
@@ -792,17 +828,34 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
     }
     if (m && pre && pre->ready && pre->unsorted && !pre->ungrouped) {
         // Row-grouped inserts (rows non-decreasing, columns in any order, as
-        // row-by-row assembly stages them): every row is sorted, its last
-        // write per column kept unless zero, and compacted on chip in one
-        // pass, in place at the row's input positions; a scan of the kept
-        // counts gives the offsets, and entries move only if some were dropped.
+        // row-by-row assembly stages them). Two ways to the same CSR:
+        //   tiles    (spg_rowtiles.cu) sort, reduce and write the CSR in one pass,
+        //            whatever the rows' lengths;
+        //   classes  every row is sorted, its last write per column kept unless
+        //            zero, and compacted by its length class's kernel, in place
+        //            at the row's input positions; a scan of the kept counts
+        //            gives the offsets, and entries move only if some were
+        //            dropped.
+        // Tiles are faster where rows are long (100k rows of 300 uniform
+        // columns: 0.67 against 1.17 ms; 10k of 3000: 0.83 / 1.00), and below
+        // 4 M inserts, where the classes' ten launches are what is paid (100 k
+        // inserts from the host: 0.174 / 0.235 ms). Rows of up to 32 entries are
+        // the networks' case (27-point stencil, 1 M rows in any column order:
+        // 0.53 / 0.68 ms). So: tiles when a quarter of the entries follow more
+        // than 32 others of their row, or for few inserts.
+        const bool tiles = m <= (4u << 20) || 64 * pre->long_hits > 3 * m;
         DevBuf s_off, kept, scols, svals;
         SPG_TRY(s_off.alloc((n + 1) * sizeof(uint64_t), s));
         SPG_TRY(launch_row_offsets(c, rows, m, n, s_off.as<uint64_t>(), s));
+        bool done = false;
+        if (tiles) {
+            GroupedOut o;
+            SPG_TRY(build_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, cbits, false, &o, &done, s));
+            if (done) return first_install(c, A, std::move(o), m, s);
+        }
         SPG_TRY(kept.alloc(csr_off_elems(n) * sizeof(uint64_t), s));
         SPG_TRY(scols.alloc(csr_alloc_elems(m) * sizeof(uint32_t), s));
         SPG_TRY(svals.alloc(csr_alloc_elems(m) * sizeof(double), s));
-        bool done = false;
         SPG_TRY(dedup_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, cbits, scols.as<uint32_t>(),
                                    svals.as<double>(), kept.as<uint64_t>(), &done, s));
         if (done) {
@@ -882,8 +935,8 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
     Prepared pre;
     if (m) {
         DevBuf stats;
-        SPG_TRY(stats.alloc(5 * sizeof(unsigned), s));
-        SPG_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, 5 * sizeof(unsigned), s));
+        SPG_TRY(stats.alloc(6 * sizeof(unsigned), s));
+        SPG_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, 6 * sizeof(unsigned), s));
         if (((uintptr_t)rows | (uintptr_t)cols) % 16 == 0)
             lock_prepare<true><<<grid_for((m + 3) / 4, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
                 rows, cols, m, bits_for(A->n_cols), stats.as<unsigned>());
@@ -891,8 +944,8 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
             lock_prepare<false><<<grid_for(m, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
                 rows, cols, m, bits_for(A->n_cols), stats.as<unsigned>());
         SPG_LAUNCH_CHECK();
-        unsigned h[5] = {0u, 0u, 1u, 1u, 1u};
-        SPG_CUDA_TRY(cudaMemcpyAsync(h, stats.ptr, 5 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+        unsigned h[6] = {0u, 0u, 1u, 1u, 1u, 0u};
+        SPG_CUDA_TRY(cudaMemcpyAsync(h, stats.ptr, 6 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         SPG_TRY(c->phase_sync(s));
         if ((uint64_t)h[0] >= A->n_rows)
             return set_error(SPG_ERR_OUT_OF_RANGE, "spira::matrix: row_index out of range (%u >= %llu)", h[0],
@@ -903,6 +956,7 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
         pre.unsorted = h[2];
         pre.ungrouped = h[3];
         pre.not_strict = h[4];
+        pre.long_hits = h[5];
         pre.ready = true;
     }
     const uint64_t n = A->n_rows;

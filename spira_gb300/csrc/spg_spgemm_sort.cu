@@ -46,12 +46,7 @@ constexpr int SGS_WARPS = 4;
 constexpr int SGS_THREADS = 32 * SGS_WARPS;
 constexpr uint32_t SGS_RB = SGS_THREADS;  // rows per tile at most: one thread each in the block scan
 constexpr unsigned SGS_STATUS_TIMEOUT = 0x10u;
-constexpr long long SGS_WAIT_CYCLES = 1ll << 31;  // ~1 s at 2 GHz
-
-constexpr unsigned long long LB_AGG = 1ull << 62;      // tile published its own count
-constexpr unsigned long long LB_PREFIX = 2ull << 62;   // tile published its inclusive prefix
-constexpr unsigned long long LB_POISON = 3ull << 62;   // tile gave up: everything after stops
-constexpr unsigned long long LB_VALUE = (1ull << 62) - 1;
+constexpr long long SGS_WAIT_CYCLES = LB_WAIT_CYCLES;
 
 struct SgsArgs {
     const uint64_t *aoff;
@@ -367,56 +362,9 @@ __device__ __forceinline__ uint32_t sgs_row(const SgsArgs &g, uint64_t i, uint32
     return kept;
 }
 
-// Ordered scan of the tiles' counts, by one warp: lane l reads the word of
-// tile p - l, so each step covers 32 predecessors. (Reading 8 words per lane,
-// 256 per step, measured slower: 0.73 against 0.43 ms on the 200k x 8
-// product with 2048-product tiles.) Returns false if the tile had to give up
-// (timeout, or an earlier tile gave up). Lane 0 publishes.
+// Ordered scan of the tiles' counts (lookback_scan: one warp, lane 0 publishes).
 __device__ bool sgs_lookback(const SgsArgs &g, uint64_t t, uint64_t total, uint64_t *base, int lane) {
-    if (t == 0) {
-        if (lane == 0) atomicExch(g.tstate, LB_PREFIX | total);
-        *base = 0;
-        return true;
-    }
-    if (lane == 0) atomicExch(g.tstate + t, LB_AGG | total);
-    uint64_t excl = 0;
-    int64_t p = (int64_t)t - 1;  // nearest predecessor of the window
-    const long long t0 = clock64();
-    while (true) {
-        const int64_t q = p - lane;
-        const unsigned long long v = q >= 0 ? *(volatile unsigned long long *)(g.tstate + q) : 0ull;
-        const unsigned long long st = v & ~LB_VALUE;
-        const unsigned pref = __ballot_sync(0xffffffffu, q >= 0 && st == LB_PREFIX);
-        // lanes up to the nearest prefix (tile 0 always publishes one, so a
-        // window reaching q < 0 holds it at a lower lane)
-        const unsigned need = pref ? (pref & (0u - pref)) * 2u - 1u : 0xffffffffu;
-        const unsigned waiting = __ballot_sync(0xffffffffu, q >= 0 && st == 0) & need;
-        const unsigned poison = __ballot_sync(0xffffffffu, q >= 0 && st == LB_POISON) & need;
-        if (poison) {
-            if (lane == 0) atomicExch(g.tstate + t, LB_POISON);
-            return false;
-        }
-        if (waiting) {
-            if (clock64() - t0 > g.wait_cycles) {
-                if (lane == 0) {
-                    atomicOr(g.status, SGS_STATUS_TIMEOUT);
-                    atomicExch(g.tstate + t, LB_POISON);
-                }
-                return false;
-            }
-            __nanosleep(32);
-            continue;
-        }
-        unsigned long long add = ((need >> lane) & 1u) ? (v & LB_VALUE) : 0ull;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
-        excl += add;
-        if (pref) break;
-        p -= 32;
-    }
-    if (lane == 0) atomicExch(g.tstate + t, LB_PREFIX | (excl + total));
-    *base = excl;
-    return true;
+    return lookback_scan(g.tstate, t, total, base, lane, g.status, SGS_STATUS_TIMEOUT, g.wait_cycles);
 }
 
 template <int HB, class K>

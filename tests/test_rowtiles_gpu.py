@@ -1,0 +1,56 @@
+"""lock() of row-grouped inserts through the one-pass tile kernel
+(spira_gb300/csrc/spg_rowtiles.cu) at the places where it can go wrong: tiles
+filled exactly and overfilled by one, rows longer than a tile, long stretches
+of empty rows, buckets that must be split again (clustered columns, many
+duplicates) and the widest columns. Bit-exact against the oracle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import oracle
+import spira_gb300 as sg
+from spira_gb300 import gen
+from conftest import assert_csr_equal
+
+pytestmark = pytest.mark.gpu
+
+
+def _columns(kind, rows, n_cols, seed):
+    h = gen.hash3(seed, 1, np.arange(len(rows), dtype=np.uint64))
+    if kind == "uniform":
+        return gen.below(h, n_cols)
+    if kind == "equal":  # one column per row
+        return (rows.astype(np.uint64) * 7 % n_cols).astype(np.uint32)
+    if kind == "few":  # ten columns next to each other
+        return (rows.astype(np.uint64) % (n_cols - 10) + h % np.uint64(10)).astype(np.uint32)
+    if kind == "band":  # a band around the diagonal
+        return ((rows.astype(np.uint64) * 31 + h % np.uint64(400)) % n_cols).astype(np.uint32)
+    # geometric clusters: columns 2^k and a few after, so that every split of a
+    # bucket leaves one crowded part
+    k = (h >> np.uint64(8)) % np.uint64(int(n_cols).bit_length() - 1)
+    return np.minimum((np.uint64(1) << k) + h % np.uint64(3), n_cols - 1).astype(np.uint32)
+
+
+LENGTHS = {
+    "edges": [4096, 4095, 1, 1, 4095, 2048, 2048, 2049, 2047, 0, 4097, 31, 32, 33, 0, 12288, 5000, 1, 4064, 32],
+    "short": [0, 1, 2, 5, 10, 17, 31, 32, 33] * 700,
+    "empty": [3] + [0] * 5000 + [40] + [0] * 2047 + [700] + [0] * 3000,
+    "one": [100],
+}
+
+
+@pytest.mark.parametrize("kind", ["uniform", "equal", "few", "band", "geometric"])
+@pytest.mark.parametrize("lengths", sorted(LENGTHS))
+def test_lock_row_tiles(ctx, lengths, kind):
+    L = np.asarray(LENGTHS[lengths], np.int64)
+    for n_cols in (1000, (1 << 32) - 5):
+        rows = np.repeat(np.arange(len(L), dtype=np.uint32), L)
+        cols = _columns(kind, rows, n_cols, seed=len(rows))
+        vals = gen.sym_unit(gen.hash3(len(rows), 2, np.arange(len(rows), dtype=np.uint64)))
+        vals[::11] = 0.0
+        vals[5::37] = -0.0
+        vals[3::101] = np.nan
+        A = sg.Csr(ctx, len(L), n_cols)
+        A.lock(rows, cols, vals)
+        assert_csr_equal(A.download(), oracle.lock_epochs(len(L), n_cols, [(rows, cols, vals)]))
