@@ -58,9 +58,24 @@ struct RowGap {
     uint64_t lo, hi, pos;
 };
 
-// (Writing the staged rows' offsets in this pass as well, speculatively, was
-// tried and removed: on inserts in random order every rising step between
-// neighbours would write its whole gap of rows, ~m n / 3 stores.)
+// With off (a first lock), the pass also writes the staged rows' offsets, in
+// case the rows turn out to be grouped: at a step from row r1 up to row r2
+// after insert i, off[r1 + 1 .. r2] = i + 1. Only steps of at most OFF_STEP
+// rows are written: inserts in random order, whose steps are long, then write
+// next to nothing (writing every rising step's rows took ~m n / 3 stores
+// there); a longer one sets stats[6], and launch_row_offsets writes the
+// offsets after all. A pass of its own over the 64 M rows of the 4M-row Zipf
+// matrix took 106 us, the stores here 32 (lock 1.64 -> 1.54 ms).
+constexpr uint32_t OFF_STEP = 8;
+
+__device__ __forceinline__ bool offsets_step(uint64_t *__restrict__ off, uint64_t lo, uint64_t hi, uint64_t n_rows,
+                                             uint64_t pos) {  // off[lo .. hi] = pos; true if left to the other pass
+    if (hi > n_rows || hi - lo >= OFF_STEP) return true;  // (rows are not range-checked yet)
+    off[hi] = pos;
+    for (uint64_t r = lo; r < hi; ++r) off[r] = pos;  // (steps of one row, by far the most: none)
+    return false;
+}
+
 // VEC: rows and cols 16-byte aligned; each thread reads 4 rows and 4
 // columns per step in two 16-byte loads (the successor of its last pair
 // comes from the next lane, or one more load at the warp's edge).
@@ -68,9 +83,13 @@ struct RowGap {
 // fourth insert, by 24 lanes of each warp's 32 (3 / 16 of all).
 template <bool VEC>
 __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, uint64_t m,
-                             int cbits, unsigned *__restrict__ stats) {
+                             int cbits, uint64_t n_rows, uint64_t *__restrict__ off, unsigned *__restrict__ stats) {
     unsigned mr = 0, mc = 0, hits = 0;
-    bool d = false, g = false, e = false;
+    bool d = false, g = false, e = false, gap = false;
+    if (off && blockIdx.x == 0 && threadIdx.x == 0) {  // the rows up to the first insert's and after the last one's
+        gap |= offsets_step(off, 0, rows[0], n_rows, 0);
+        gap |= offsets_step(off, (uint64_t)rows[m - 1] + 1, n_rows, n_rows, m);
+    }
     if constexpr (VEC) {
         const uint64_t n4 = m / 4;  // whole groups of 4; the tail below
         const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -103,6 +122,8 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
                         d |= k1 > k2;
                         e |= k1 >= k2;
                         g |= rr[k] > rr[k + 1];
+                        if (off && rr[k] < rr[k + 1])
+                            gap |= offsets_step(off, (uint64_t)rr[k] + 1, rr[k + 1], n_rows, 4 * q + k + 1);
                     }
                 }
             }
@@ -111,16 +132,16 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
     for (uint64_t i = (VEC ? (m & ~3ull) : 0) + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t r = rows[i], c = cols[i];
-        const uint64_t k = ((uint64_t)r << cbits) | c;
         mr = max(mr, r);
         mc = max(mc, c);
         if (!VEC && (i & 3) == 0 && ((i >> 2) & 31) < 24 && i + 32 < m) hits += rows[i + 32] == r ? 1u : 0u;
         if (i + 1 < m) {
             const uint32_t r2 = rows[i + 1];
-            const uint64_t k2 = ((uint64_t)r2 << cbits) | cols[i + 1];
+            const uint64_t k = ((uint64_t)r << cbits) | c, k2 = ((uint64_t)r2 << cbits) | cols[i + 1];
             d |= k > k2;
             e |= k >= k2;
             g |= r > r2;
+            if (off && r < r2) gap |= offsets_step(off, (uint64_t)r + 1, r2, n_rows, i + 1);
         }
     }
 #pragma unroll
@@ -130,7 +151,7 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
     }
     hits = __reduce_add_sync(0xffffffffu, hits);
     const unsigned flags = (__any_sync(0xffffffffu, d) ? 1u : 0u) | (__any_sync(0xffffffffu, g) ? 2u : 0u) |
-                           (__any_sync(0xffffffffu, e) ? 4u : 0u);
+                           (__any_sync(0xffffffffu, e) ? 4u : 0u) | (__any_sync(0xffffffffu, gap) ? 8u : 0u);
     // one set of atomics per block: per-warp atomics on the same two words
     // serialise at L2 and cost more than the pass itself
     __shared__ unsigned s_mr[LB / 32], s_mc[LB / 32], s_fl[LB / 32], s_hits[LB / 32];
@@ -156,6 +177,7 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
         if (bf & 1u) stats[2] = 1u;
         if (bf & 2u) stats[3] = 1u;
         if (bf & 4u) stats[4] = 1u;
+        if (bf & 8u) stats[6] = 1u;
     }
 }
 
@@ -675,7 +697,19 @@ struct Prepared {
     unsigned unsorted = 1, ungrouped = 1, not_strict = 1;
     uint64_t long_hits = 0;  // sampled inserts that 32 others of their row follow (3 / 16 of the inserts looked at)
     bool ready = false;
+    DevBuf off;             // a first lock: the staged rows' offsets ...
+    bool have_off = false;  // ... when the rows are grouped and no step between them was long
 };
+
+// The staged (grouped) rows' offsets.
+int staged_offsets(Ctx *c, Prepared *pre, const uint32_t *rows, uint64_t m, uint64_t n_rows, DevBuf &off,
+                   cudaStream_t s) {
+    const bool have = pre && pre->off.ptr && pre->have_off;
+    if (pre && pre->off.ptr) off = std::move(pre->off);
+    else SPG_TRY(off.alloc(csr_off_elems(n_rows) * sizeof(uint64_t), s));
+    if (!have) SPG_TRY(launch_row_offsets(c, rows, m, n_rows, off.as<uint64_t>(), s));
+    return SPG_OK;
+}
 
 int sort_keys(Ctx *c, const uint32_t *rows, const uint32_t *cols, uint64_t m, uint64_t n_rows, uint64_t n_cols,
               DevBuf &keys, DevBuf &idx, Prepared *pre, cudaStream_t s) {
@@ -806,8 +840,7 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
                                            zero.as<unsigned>());
         SPG_LAUNCH_CHECK();
         // the offsets go out before the zero check comes back: one host sync
-        SPG_TRY(new_off.alloc(csr_off_elems(n) * sizeof(uint64_t), s));
-        SPG_TRY(launch_row_offsets(c, rows, m, n, new_off.as<uint64_t>(), s));
+        SPG_TRY(staged_offsets(c, pre, rows, m, n, new_off, s));
         unsigned hz = 1;
         SPG_CUDA_TRY(cudaMemcpyAsync(&hz, zero.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         SPG_TRY(c->phase_sync(s));
@@ -845,8 +878,7 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
         // than 32 others of their row, or for few inserts.
         const bool tiles = m <= (4u << 20) || 64 * pre->long_hits > 3 * m;
         DevBuf s_off, kept, scols, svals;
-        SPG_TRY(s_off.alloc((n + 1) * sizeof(uint64_t), s));
-        SPG_TRY(launch_row_offsets(c, rows, m, n, s_off.as<uint64_t>(), s));
+        SPG_TRY(staged_offsets(c, pre, rows, m, n, s_off, s));
         bool done = false;
         if (tiles) {
             GroupedOut o;
@@ -935,17 +967,18 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
     Prepared pre;
     if (m) {
         DevBuf stats;
-        SPG_TRY(stats.alloc(6 * sizeof(unsigned), s));
-        SPG_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, 6 * sizeof(unsigned), s));
+        SPG_TRY(stats.alloc(7 * sizeof(unsigned), s));
+        SPG_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, 7 * sizeof(unsigned), s));
+        if (!A->built) SPG_TRY(pre.off.alloc(csr_off_elems(A->n_rows) * sizeof(uint64_t), s));
         if (((uintptr_t)rows | (uintptr_t)cols) % 16 == 0)
             lock_prepare<true><<<grid_for((m + 3) / 4, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
-                rows, cols, m, bits_for(A->n_cols), stats.as<unsigned>());
+                rows, cols, m, bits_for(A->n_cols), A->n_rows, pre.off.as<uint64_t>(), stats.as<unsigned>());
         else
             lock_prepare<false><<<grid_for(m, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
-                rows, cols, m, bits_for(A->n_cols), stats.as<unsigned>());
+                rows, cols, m, bits_for(A->n_cols), A->n_rows, pre.off.as<uint64_t>(), stats.as<unsigned>());
         SPG_LAUNCH_CHECK();
-        unsigned h[6] = {0u, 0u, 1u, 1u, 1u, 0u};
-        SPG_CUDA_TRY(cudaMemcpyAsync(h, stats.ptr, 6 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+        unsigned h[7] = {0u, 0u, 1u, 1u, 1u, 0u, 1u};
+        SPG_CUDA_TRY(cudaMemcpyAsync(h, stats.ptr, 7 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         SPG_TRY(c->phase_sync(s));
         if ((uint64_t)h[0] >= A->n_rows)
             return set_error(SPG_ERR_OUT_OF_RANGE, "spira::matrix: row_index out of range (%u >= %llu)", h[0],
@@ -957,6 +990,7 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
         pre.ungrouped = h[3];
         pre.not_strict = h[4];
         pre.long_hits = h[5];
+        pre.have_off = pre.off.ptr && !h[3] && !h[6];
         pre.ready = true;
     }
     const uint64_t n = A->n_rows;

@@ -54,3 +54,20 @@ def test_lock_row_tiles(ctx, lengths, kind):
         A = sg.Csr(ctx, len(L), n_cols)
         A.lock(rows, cols, vals)
         assert_csr_equal(A.download(), oracle.lock_epochs(len(L), n_cols, [(rows, cols, vals)]))
+
+
+@pytest.mark.parametrize("order", ["sorted", "grouped"])
+@pytest.mark.parametrize("step", [1, 8, 9, 40])
+@pytest.mark.parametrize("first,after", [(0, 0), (7, 7), (8, 8), (300, 300)])
+def test_lock_offsets_of_spaced_rows(ctx, order, step, first, after):
+    """Row offsets written beside the range check up to steps of 8 rows, by a
+    pass of their own beyond; empty rows before, between and after."""
+    r = first + step * np.arange(700, dtype=np.int64)
+    n_rows = int(r[-1]) + 1 + after
+    rows = np.repeat(r.astype(np.uint32), 3)
+    cols = np.tile(np.array([1, 5, 9] if order == "sorted" else [9, 1, 5], np.uint32), len(r))
+    vals = gen.sym_unit(gen.hash3(9, 2, np.arange(len(rows), dtype=np.uint64)))
+    for cut in (len(rows), len(rows) - 1, 2):  # whole and ragged 16-byte groups
+        A = sg.Csr(ctx, n_rows, 12)
+        A.lock(rows[:cut], cols[:cut], vals[:cut])
+        assert_csr_equal(A.download(), oracle.lock_epochs(n_rows, 12, [(rows[:cut], cols[:cut], vals[:cut])]))
