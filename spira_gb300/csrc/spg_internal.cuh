@@ -399,6 +399,75 @@ __device__ __forceinline__ bool lookback_scan(unsigned long long *tstate, uint64
     return true;
 }
 
+// The same by a whole block of T threads, for a tile whose count is already
+// published (its own word holds LB_AGG | total, or LB_PREFIX | total for tile
+// 0): thread t reads the word of tile id - 1 - t, so a window covers T tiles,
+// about what is in flight, and the nearest published prefix is mostly found in
+// one step of one L2 round trip (one warp's windows of 32 took 14 of them in
+// the row-tile kernel). Publishes the inclusive prefix. All threads call;
+// false in every thread if the tile had to give up.
+template <int T>
+struct BlockLookback {
+    uint64_t sum[T / 32];
+    uint32_t state[T / 32];
+};
+
+template <int T>
+__device__ __forceinline__ bool block_lookback(BlockLookback<T> &S, unsigned long long *tstate, uint64_t id,
+                                               uint64_t total, uint64_t &base, unsigned int *status,
+                                               unsigned status_bit) {
+    constexpr int W = T / 32;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    base = 0;
+    if (id == 0) return true;
+    const long long t0 = clock64();
+    int64_t p = (int64_t)id - 1;
+    while (true) {
+        const int64_t q = p - t;
+        const unsigned long long v = q >= 0 ? *(volatile unsigned long long *)(tstate + q) : 0ull + LB_PREFIX;
+        const unsigned long long st = v & ~LB_VALUE;
+        // up to the warp's nearest prefix (tile 0 always publishes one)
+        const unsigned pref = __ballot_sync(0xffffffffu, st == LB_PREFIX);
+        const unsigned need = pref ? (pref & (0u - pref)) * 2u - 1u : 0xffffffffu;
+        const unsigned waiting = __ballot_sync(0xffffffffu, st == 0) & need;
+        const unsigned poison = __ballot_sync(0xffffffffu, st == LB_POISON) & need;
+        uint64_t add = (need >> lane) & 1u ? v & LB_VALUE : 0ull;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+        if (lane == 0) {
+            S.sum[warp] = add;
+            S.state[warp] = (pref ? 1u : 0u) | (waiting ? 2u : 0u) | (poison ? 4u : 0u);
+        }
+        const bool late = __syncthreads_or(t == 0 && clock64() - t0 > LB_WAIT_CYCLES);
+        bool found = false, wait = false, bad = false;
+        uint64_t sum = 0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            if (!found) {
+                const uint32_t x = S.state[w];
+                sum += S.sum[w];
+                found = x & 1u;
+                wait |= (x & 2u) != 0;
+                bad |= (x & 4u) != 0;
+            }
+        }
+        __syncthreads();  // the parts are read
+        if (bad || (wait && late)) {
+            if (t == 0) {
+                if (!bad) atomicOr(status, status_bit);
+                atomicExch(tstate + id, 0ull + LB_POISON);
+            }
+            return false;
+        }
+        if (wait) continue;
+        base += sum;
+        if (found) break;
+        p -= T;
+    }
+    if (t == 0) atomicExch(tstate + id, LB_PREFIX | (base + total));
+    return true;
+}
+
 inline unsigned grid_for(uint64_t n, unsigned block, unsigned cap = 1u << 30) {
     uint64_t g = (n + block - 1) / block;
     if (g == 0) g = 1;
@@ -462,6 +531,21 @@ int spgemm_warpsort(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, int variant, cu
 int spgemm_run(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, int variant, cudaStream_t s);
 // SPG_SPGEMM_AUTO resolved by the context's policy (spg_tune.cu).
 int spgemm_resolve_auto(Ctx *c, const Csr *A, const Csr *B, int *variant);
+
+// C = the row-wise merge of two CSRs of the same shape (spg_merge.cu). Sum: equal
+// columns add up (one IEEE add), zeros of the result and stored zeros are
+// dropped. Replace: B's entry replaces A's, a zero of B deletes; A's other
+// entries stay as they are. off_out has n_rows + 1 entries; cols_out / vals_out
+// at least nnz(A) + nnz(B). *nnz is read back (the call synchronises).
+enum class MergeMode { Sum, Replace };
+struct CsrView {
+    const uint64_t *off;
+    const uint32_t *cols;
+    const double *vals;
+    uint64_t nnz;
+};
+int merge_csr(Ctx *c, const CsrView &A, const CsrView &B, uint64_t n_rows, MergeMode mode, uint64_t *off_out,
+              uint32_t *cols_out, double *vals_out, uint64_t *nnz, cudaStream_t s);
 
 // CSR helpers used by several ops (spg_lock.cu).
 int csr_alloc(Csr *A, uint64_t capacity, cudaStream_t s);

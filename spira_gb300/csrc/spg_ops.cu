@@ -16,19 +16,7 @@
 //   bounds   parallel/partition.hpp:78-126: first row whose nnz prefix
 //            reaches max(1, t * nnz / T); a uniform split when nnz == 0.
 //
-// Addition on the GPU, entry-parallel with no per-row loop (any row-length
-// mix balances): every entry of A finds by binary search the first entry of
-// B's row at or after its column (and whether it collides), every entry of B
-// the same in A's row. Keep flags of A (sum or own value non-zero) and of B
-// (no collision, value non-zero) are scanned separately into SA and SB. With
-// ja the absolute position found in B for A entry e, and ib the one found in
-// A for B entry f:
-//     position of A entry e in C = SA[e] + SB[ja]
-//     position of B entry f in C = SB[f] + SA[ib]
-//     C offsets: off_C[r] = SA[off_A[r]] + SB[off_B[r]]
-// since the kept entries before e in C are the kept A entries before e plus
-// the kept B entries of earlier rows and of e's row below its column. Values
-// are copied or summed once (__dadd_rn), so C is bit-exact.
+// Addition is a merge of the two CSRs (spg_merge.cu).
 #include <algorithm>
 #include <vector>
 
@@ -38,20 +26,6 @@ namespace spg {
 namespace {
 
 constexpr int OB = 256;
-constexpr uint64_t COLLIDE = 1ull << 63;  // high bit of a found position: the columns are equal
-
-
-// Row holding entry e: the last r with off[r] <= e (rows before it end at or
-// before e, empty rows share their successor's offset).
-__device__ __forceinline__ uint64_t row_of(const uint64_t *__restrict__ off, uint64_t n_rows, uint64_t e) {
-    uint64_t lo = 0, hi = n_rows - 1;
-    while (lo < hi) {
-        const uint64_t mid = (lo + hi + 1) >> 1;
-        if (off[mid] <= e) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
 
 // First position in [b, e) whose column is >= c.
 __device__ __forceinline__ uint64_t lower_col(const uint32_t *__restrict__ cols, uint64_t b, uint64_t e, uint32_t c) {
@@ -61,116 +35,6 @@ __device__ __forceinline__ uint64_t lower_col(const uint32_t *__restrict__ cols,
         else e = mid;
     }
     return b;
-}
-
-// Keep flag and partner position of every entry of X against Y's rows; for X
-// = A the kept value is the sum on a collision, for X = B a collision drops
-// the entry (A's side holds the sum). A block takes a tile of PT consecutive
-// entries: two searches find the rows of its first and last entry, the
-// offsets of the rows in between go to shared memory (when they fit), and
-// every entry finds its row there.
-constexpr int PT = 2048, PROWS = 2048;
-
-template <bool X_IS_A>
-__global__ void __launch_bounds__(OB)
-add_probe(const uint64_t *__restrict__ xoff, const uint32_t *__restrict__ xcols, const double *__restrict__ xvals,
-          uint64_t nx, const uint64_t *__restrict__ yoff, const uint32_t *__restrict__ ycols,
-          const double *__restrict__ yvals, uint64_t n_rows, uint64_t *__restrict__ keep,
-          uint64_t *__restrict__ partner) {
-    __shared__ uint64_t s_off[PROWS + 1];
-    __shared__ uint64_t s_win[2];
-    for (uint64_t e0 = blockIdx.x * (uint64_t)PT; e0 < nx; e0 += (uint64_t)gridDim.x * PT) {
-        const uint64_t e1 = min(nx, e0 + PT);
-        if (threadIdx.x == 0) s_win[0] = row_of(xoff, n_rows, e0);
-        if (threadIdx.x == 32) s_win[1] = row_of(xoff, n_rows, e1 - 1);
-        __syncthreads();
-        const uint64_t r_lo = s_win[0], r_hi = s_win[1];
-        const bool in_smem = r_hi - r_lo < PROWS;
-        if (in_smem)
-            for (uint64_t j = threadIdx.x; j <= r_hi - r_lo + 1; j += OB) s_off[j] = xoff[r_lo + j];
-        __syncthreads();
-        for (uint64_t e = e0 + threadIdx.x; e < e1; e += OB) {
-            uint64_t r;
-            if (in_smem) {  // last j with s_off[j] <= e
-                uint64_t lo = 0, hi = r_hi - r_lo;
-                while (lo < hi) {
-                    const uint64_t mid = (lo + hi + 1) >> 1;
-                    if (s_off[mid] <= e) lo = mid;
-                    else hi = mid - 1;
-                }
-                r = r_lo + lo;
-            } else {
-                uint64_t lo = r_lo, hi = r_hi;
-                while (lo < hi) {
-                    const uint64_t mid = (lo + hi + 1) >> 1;
-                    if (xoff[mid] <= e) lo = mid;
-                    else hi = mid - 1;
-                }
-                r = lo;
-            }
-            const uint32_t c = xcols[e];
-            const uint64_t yb = yoff[r], ye = yoff[r + 1];
-            const uint64_t p = lower_col(ycols, yb, ye, c);
-            const bool coll = p < ye && ycols[p] == c;
-            bool k;
-            if (X_IS_A) k = !is_zero(coll ? __dadd_rn(xvals[e], yvals[p]) : xvals[e]);
-            else k = !coll && !is_zero(xvals[e]);
-            keep[e] = k ? 1u : 0u;
-            partner[e] = p | (coll ? COLLIDE : 0);
-        }
-        __syncthreads();
-    }
-}
-
-__global__ void add_offsets(const uint64_t *__restrict__ aoff, const uint64_t *__restrict__ boff,
-                            const uint64_t *__restrict__ sa, const uint64_t *__restrict__ sb, uint64_t n_rows,
-                            uint64_t *__restrict__ coff) {
-    for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r <= n_rows;
-         r += (uint64_t)gridDim.x * blockDim.x)
-        coff[r] = sa[aoff[r]] + sb[boff[r]];
-}
-
-// Writes X's kept entries into C. sx = X's scanned keep flags (nx + 1
-// entries), sy = Y's; X = A sums on a collision. A thread handles SI entries
-// per step with their loads issued together.
-template <bool X_IS_A>
-__global__ void __launch_bounds__(OB)
-add_scatter(const uint32_t *__restrict__ xcols, const double *__restrict__ xvals, uint64_t nx,
-            const double *__restrict__ yvals, const uint64_t *__restrict__ sx, const uint64_t *__restrict__ sy,
-            const uint64_t *__restrict__ partner, uint32_t *__restrict__ ccols, double *__restrict__ cvals) {
-    constexpr int SI = 4;
-    for (uint64_t e0 = blockIdx.x * (uint64_t)(OB * SI); e0 < nx; e0 += (uint64_t)gridDim.x * OB * SI) {
-        uint64_t s0[SI], s1[SI], pp[SI];
-#pragma unroll
-        for (int q = 0; q < SI; ++q) {
-            const uint64_t e = e0 + threadIdx.x + (uint64_t)q * OB;
-            s0[q] = e < nx ? sx[e] : 0;
-            s1[q] = e < nx ? sx[e + 1] : 0;
-            pp[q] = e < nx ? partner[e] : 0;
-        }
-        uint64_t pos[SI];
-        double v[SI], yv[SI];
-        uint32_t c[SI];
-#pragma unroll
-        for (int q = 0; q < SI; ++q) {
-            const uint64_t e = e0 + threadIdx.x + (uint64_t)q * OB;
-            const bool kept = e < nx && s1[q] != s0[q];
-            const uint64_t p = pp[q] & ~COLLIDE;
-            pos[q] = kept ? s0[q] + sy[p] : 0;
-            c[q] = kept ? xcols[e] : 0u;
-            v[q] = kept ? xvals[e] : 0.0;
-            yv[q] = (kept && X_IS_A && (pp[q] & COLLIDE)) ? yvals[p] : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < SI; ++q) {
-            const uint64_t e = e0 + threadIdx.x + (uint64_t)q * OB;
-            if (e >= nx || s1[q] == s0[q]) continue;  // dropped
-            double val = v[q];
-            if (X_IS_A && (pp[q] & COLLIDE)) val = __dadd_rn(val, yv[q]);
-            ccols[pos[q]] = c[q];
-            cvals[pos[q]] = val;
-        }
-    }
 }
 
 // scale: v * s or v / s into out (may alias vals); zero results counted per
@@ -437,46 +301,17 @@ void install(Csr *C, uint64_t n_rows, uint64_t n_cols, DevBuf &off, DevBuf &cols
     C->may_have_zeros = false;
 }
 
+// C's arrays have room for every entry of both sides; nnz(C) of it is used, at
+// least half (an equal pair becomes one entry) but for cancellations.
 int add_impl(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, cudaStream_t s) {
-    const uint64_t n = A->n_rows, na = A->nnz, nb = B->nnz;
-    const unsigned cap = (unsigned)c->n_sms * 16;
-    DevBuf ka, kb, pa, pb, off, cols, vals;
-    SPG_TRY(ka.alloc((na + 1) * sizeof(uint64_t), s));
-    SPG_TRY(kb.alloc((nb + 1) * sizeof(uint64_t), s));
-    SPG_TRY(pa.alloc(std::max<uint64_t>(na, 1) * sizeof(uint64_t), s));
-    SPG_TRY(pb.alloc(std::max<uint64_t>(nb, 1) * sizeof(uint64_t), s));
-    if (na)
-        add_probe<true><<<grid_for(na, PT, cap), OB, 0, s>>>(A->d_off(), A->d_cols(), A->d_vals(), na, B->d_off(),
-                                                             B->d_cols(), B->d_vals(), n, ka.as<uint64_t>(),
-                                                             pa.as<uint64_t>());
-    if (nb)
-        add_probe<false><<<grid_for(nb, PT, cap), OB, 0, s>>>(B->d_off(), B->d_cols(), B->d_vals(), nb, A->d_off(),
-                                                              A->d_cols(), A->d_vals(), n, kb.as<uint64_t>(),
-                                                              pb.as<uint64_t>());
-    SPG_LAUNCH_CHECK();
-    if (na) SPG_TRY(exclusive_scan_u64(c, ka.as<uint64_t>(), na, ka.as<uint64_t>() + na, s));
-    else SPG_CUDA_TRY(cudaMemsetAsync(ka.ptr, 0, sizeof(uint64_t), s));
-    if (nb) SPG_TRY(exclusive_scan_u64(c, kb.as<uint64_t>(), nb, kb.as<uint64_t>() + nb, s));
-    else SPG_CUDA_TRY(cudaMemsetAsync(kb.ptr, 0, sizeof(uint64_t), s));
+    const uint64_t n = A->n_rows;
+    DevBuf off, cols, vals;
     SPG_TRY(off.alloc(csr_off_elems(n) * sizeof(uint64_t), s));
-    add_offsets<<<grid_for(n + 1, OB, cap), OB, 0, s>>>(A->d_off(), B->d_off(), ka.as<uint64_t>(), kb.as<uint64_t>(),
-                                                        n, off.as<uint64_t>());
-    SPG_LAUNCH_CHECK();
+    SPG_TRY(cols.alloc(csr_alloc_elems(A->nnz + B->nnz) * sizeof(uint32_t), s));
+    SPG_TRY(vals.alloc(csr_alloc_elems(A->nnz + B->nnz) * sizeof(double), s));
     uint64_t nnz = 0;
-    SPG_TRY(read_word(c, off.as<uint64_t>() + n, s, &nnz));
-    SPG_TRY(cols.alloc(csr_alloc_elems(nnz) * sizeof(uint32_t), s));
-    SPG_TRY(vals.alloc(csr_alloc_elems(nnz) * sizeof(double), s));
-    if (na)
-        add_scatter<true><<<grid_for(na, OB * 4, cap), OB, 0, s>>>(A->d_cols(), A->d_vals(), na, B->d_vals(),
-                                                               ka.as<uint64_t>(), kb.as<uint64_t>(), pa.as<uint64_t>(),
-                                                               cols.as<uint32_t>(), vals.as<double>());
-    if (nb)
-        add_scatter<false><<<grid_for(nb, OB * 4, cap), OB, 0, s>>>(B->d_cols(), B->d_vals(), nb, A->d_vals(),
-                                                                kb.as<uint64_t>(), ka.as<uint64_t>(),
-                                                                pb.as<uint64_t>(), cols.as<uint32_t>(),
-                                                                vals.as<double>());
-    SPG_LAUNCH_CHECK();
-    SPG_TRY(c->phase_sync(s));
+    SPG_TRY(merge_csr(c, {A->d_off(), A->d_cols(), A->d_vals(), A->nnz}, {B->d_off(), B->d_cols(), B->d_vals(), B->nnz},
+                      n, MergeMode::Sum, off.as<uint64_t>(), cols.as<uint32_t>(), vals.as<double>(), &nnz, s));
     install(Cm, n, A->n_cols, off, cols, vals, nnz);
     return SPG_OK;
 }

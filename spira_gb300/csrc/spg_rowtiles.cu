@@ -169,7 +169,7 @@ struct RtSmem : RtArrays<CAP, APART> {
     uint16_t wbeg[CAP / 32 + 2];   // start of the row that entry 32 w continues
     uint16_t wend[CAP / 32 + 2];   // end of the row that holds entry 32 w + 31
     uint32_t wsum[32];
-    uint32_t lb_sum[32], lb_state[32];  // look-back: each warp's part of the window
+    BlockLookback<T> lb;
     struct Tile {
         uint64_t id, r0, r1, s0, s1;  // its rows and their entries
         uint32_t total;               // kept entries
@@ -483,59 +483,6 @@ __global__ void __launch_bounds__(RT_BIG_T, 1) rt_big_rows(RtArgs a) {
     }
 }
 
-// Kept entries before tile id (counts fit 32 bits: an epoch has fewer than
-// 2^32 entries), by the whole block: thread t reads the word of tile
-// p - t, so a window covers T tiles, more than there are in flight, and the
-// nearest published prefix is found in one step. (One warp's windows of 32
-// took 14 steps of an L2 round trip each.) False if the tile had to give up.
-template <int T, class Smem>
-__device__ __forceinline__ bool rt_lookback(Smem &S, const RtArgs &a, uint64_t id, uint32_t total, uint32_t &base) {
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    base = 0;
-    if (id == 0) return true;  // published with its count
-    const long long t0 = clock64();
-    int64_t p = (int64_t)id - 1;
-    while (true) {
-        const int64_t q = p - t;
-        const unsigned long long v = q >= 0 ? *(volatile unsigned long long *)(a.tile_state + q) : 0ull + LB_PREFIX;
-        const unsigned long long st = v & ~LB_VALUE;
-        // up to the warp's nearest prefix (tile 0 always publishes one)
-        const unsigned pref = __ballot_sync(0xffffffffu, st == LB_PREFIX);
-        const unsigned need = pref ? (pref & (0u - pref)) * 2u - 1u : 0xffffffffu;
-        const unsigned waiting = __ballot_sync(0xffffffffu, st == 0) & need;
-        const unsigned poison = __ballot_sync(0xffffffffu, st == LB_POISON) & need;
-        const uint32_t sum = __reduce_add_sync(0xffffffffu, (need >> lane) & 1u ? (uint32_t)v : 0u);
-        if (lane == 0) {
-            S.lb_sum[warp] = sum;
-            S.lb_state[warp] = (pref ? 1u : 0u) | (waiting ? 2u : 0u) | (poison ? 4u : 0u);
-        }
-        const bool late = __syncthreads_or(t == 0 && clock64() - t0 > LB_WAIT_CYCLES);
-        // the same combination of the warps' parts in every warp
-        const uint32_t ws = lane < T / 32 ? S.lb_state[lane] : 1u;
-        const unsigned wp = __ballot_sync(0xffffffffu, ws & 1u);
-        const unsigned wneed = (wp & (0u - wp)) * 2u - 1u;  // (lanes past T / 32 count as prefixes)
-        const unsigned wmask = T / 32 < 32 ? (1u << (T / 32 % 32)) - 1u : 0xffffffffu;
-        const bool wait = (__ballot_sync(0xffffffffu, ws & 2u) & wneed & wmask) != 0;
-        const bool bad = (__ballot_sync(0xffffffffu, ws & 4u) & wneed & wmask) != 0;
-        const uint32_t wsum = __reduce_add_sync(0xffffffffu, (wneed & wmask) >> lane & 1u ? S.lb_sum[lane] : 0u);
-        const bool found = (wp & wmask) != 0;
-        __syncthreads();  // the parts are read
-        if (bad || (wait && late)) {
-            if (t == 0) {
-                if (!bad) atomicOr(a.status, RT_STATUS_TIMEOUT);
-                atomicExch(a.tile_state + id, LB_POISON);
-            }
-            return false;
-        }
-        if (wait) continue;
-        base += wsum;
-        if (found) break;
-        p -= T;
-    }
-    if (t == 0) atomicExch(a.tile_state + id, LB_PREFIX | ((unsigned long long)base + total));
-    return true;
-}
-
 // Tiles in ticket order. A tile's place in the CSR is known once every tile
 // before it is sorted, and waiting for that idled the block for as long as the
 // sort took (tiles differ, and the slowest of all in flight holds up the
@@ -581,13 +528,13 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
             }
         }
         if (it > 0) {
-            uint32_t base = 0;
-            if (!rt_lookback<T>(S, a, prev.id, prev.total, base)) return;
+            uint64_t base = 0;
+            if (!block_lookback<T>(S.lb, a.tile_state, prev.id, prev.total, base, a.status, RT_STATUS_TIMEOUT)) return;
             const uint32_t n = prev.total;
             if (prev.s1 - prev.s0 <= (uint64_t)CAP) {
                 for (uint32_t k = t; k < n; k += T) {
-                    a.out_cols[(uint64_t)base + k] = S.col[k];
-                    a.out_vals[(uint64_t)base + k] = S.val[k];
+                    a.out_cols[base + k] = S.col[k];
+                    a.out_vals[base + k] = S.val[k];
                 }
                 for (uint64_t r = prev.r0 + t; r < prev.r1; r += T) {
                     const uint64_t p = a.off[r];  // within the tile: this thread's own
@@ -595,12 +542,12 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
                 }
             } else {  // one row
                 for (uint32_t k = t; k < n; k += T) {
-                    a.out_cols[(uint64_t)base + k] = a.big_cols[prev.s0 + k];
-                    a.out_vals[(uint64_t)base + k] = a.big_vals[prev.s0 + k];
+                    a.out_cols[base + k] = a.big_cols[prev.s0 + k];
+                    a.out_vals[base + k] = a.big_vals[prev.s0 + k];
                 }
                 if (t == 0) a.off[prev.r0] = base;
             }
-            if (t == 0 && prev.r1 == a.n_rows) a.off[a.n_rows] = (uint64_t)base + n;
+            if (t == 0 && prev.r1 == a.n_rows) a.off[a.n_rows] = base + n;
         }
         if (!have) return;
         if (t == 32) rt_take(S.tile[(it + 1) % 3], a, n_tiles);
