@@ -34,7 +34,7 @@ int Ctx::phase_sync(cudaStream_t s) {
         timer_ms += ms;
         SPG_CUDA_TRY(cudaEventRecord(timer_ev[0], s));  // the next phase starts with the next work
     }
-    return SPG_OK;
+    return take_status();  // a wait that gave up: nothing after it may be used
 }
 
 int Ctx::ensure_pinned(size_t bytes) {

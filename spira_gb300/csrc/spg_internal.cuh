@@ -504,6 +504,29 @@ int dedup_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
 int sort_grouped_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const uint64_t *s_off, uint64_t m,
                       uint64_t n_rows, int cbits, uint64_t *keys_out, uint32_t *idx_out, bool *done, cudaStream_t s);
 
+// A CSR's device arrays.
+struct CsrView {
+    const uint64_t *off;
+    const uint32_t *cols;
+    const double *vals;
+    uint64_t nnz;
+};
+// Staged inserts stably sorted by row (spg_rowsort.cu). *abort != 0 (and the
+// context's status word is set) if a wait gave up: whatever runs on the outputs
+// before the next phase_sync has to look at it first.
+struct StagedSorted {
+    DevBuf rows, cols, vals, abort;
+};
+int sort_staged_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const double *vals, uint64_t m, int rbits,
+                     StagedSorted &out, cudaStream_t s);
+// A later lock's delta, small against the matrix, merged into it
+// (spg_delta.cu): rows non-decreasing, the last write of each key wins, zeros
+// delete. The outputs have room for nnz(A) + m entries (off_out: n_rows + 1).
+// *u = distinct keys of the delta. *done = false when a row has too many of
+// the inserts; the outputs are then undefined. abort: as above, may be null.
+int merge_small_delta(Ctx *c, const CsrView &A, uint64_t n_rows, const uint32_t *rows, const uint32_t *cols,
+                      const double *vals, uint64_t m, const unsigned long long *abort, uint64_t *off_out,
+                      uint32_t *cols_out, double *vals_out, uint64_t *nnz, uint64_t *u, bool *done, cudaStream_t s);
 // Row-grouped entries (row r's are [s_off[r], s_off[r+1]), columns in any
 // order) as CSR: the last write of every key in (row, column) order, zeros
 // dropped unless keep_zeros (spg_rowtiles.cu). The output arrays are sized
@@ -514,8 +537,8 @@ struct GroupedOut {
     uint64_t n = 0;
 };
 int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off,
-                       uint64_t m, uint64_t n_rows, int cbits, bool keep_zeros, GroupedOut *out, bool *done,
-                       cudaStream_t s);
+                       uint64_t m, uint64_t n_rows, int cbits, bool keep_zeros, const unsigned long long *abort,
+                       GroupedOut *out, bool *done, cudaStream_t s);
 
 // SpGEMM pieces shared by its variants (spg_spgemm.cu, spg_spgemm_sort.cu).
 // Expand - sort - compress output: kept entries in (row, column) order.
@@ -538,12 +561,6 @@ int spgemm_resolve_auto(Ctx *c, const Csr *A, const Csr *B, int *variant);
 // entries stay as they are. off_out has n_rows + 1 entries; cols_out / vals_out
 // at least nnz(A) + nnz(B). *nnz is read back (the call synchronises).
 enum class MergeMode { Sum, Replace };
-struct CsrView {
-    const uint64_t *off;
-    const uint32_t *cols;
-    const double *vals;
-    uint64_t nnz;
-};
 int merge_csr(Ctx *c, const CsrView &A, const CsrView &B, uint64_t n_rows, MergeMode mode, uint64_t *off_out,
               uint32_t *cols_out, double *vals_out, uint64_t *nnz, cudaStream_t s);
 

@@ -342,8 +342,7 @@ int merge_csr(Ctx *c, const CsrView &A, const CsrView &B, uint64_t n_rows, Merge
     k<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)c->n_sms * MT_PER_SM), MT_T, sizeof(MtSmem), s>>>(a);
     SPG_LAUNCH_CHECK();
     SPG_CUDA_TRY(cudaMemcpyAsync(nnz, off_out + n_rows, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-    SPG_TRY(c->phase_sync(s));
-    return c->take_status();
+    return c->phase_sync(s);
 }
 
 }  // namespace spg

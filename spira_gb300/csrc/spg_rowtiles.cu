@@ -61,6 +61,7 @@ struct RtArgs {
     uint64_t *off;         // out; off[r] holds a big row's kept count until its tile is written
     uint32_t *out_cols;
     double *out_vals;
+    const unsigned long long *abort;  // may be null: the inputs are not to be read if set
     unsigned int *status;
 };
 
@@ -81,6 +82,10 @@ __global__ void __launch_bounds__(RP_T) rt_plan(RtArgs a) {
     __shared__ uint64_t s_t, s_base;
     __shared__ int s_ok;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (a.abort && *a.abort) {
+        a.ctr[RC_OVERFLOW] = 1ull;
+        return;
+    }
     if (t == 0) s_t = atomicAdd(a.ctr + RC_PLAN_TICKET, 1ull);
     __syncthreads();
     const uint64_t blk = s_t, r0 = blk * RP_ROWS;
@@ -573,8 +578,8 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
 }  // namespace
 
 int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off,
-                       uint64_t m, uint64_t n_rows, int cbits, bool keep_zeros, GroupedOut *out, bool *done,
-                       cudaStream_t s) {
+                       uint64_t m, uint64_t n_rows, int cbits, bool keep_zeros, const unsigned long long *abort,
+                       GroupedOut *out, bool *done, cudaStream_t s) {
     *done = false;
     const uint64_t plan_tiles = (n_rows + RP_ROWS - 1) / RP_ROWS;
     // two neighbouring tiles of one part hold more than RT_CAP entries together
@@ -613,6 +618,7 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     a.off = out->off.as<uint64_t>();
     a.out_cols = out->cols.as<uint32_t>();
     a.out_vals = out->vals.as<double>();
+    a.abort = abort;
     a.status = c->d_status;
     rt_plan<<<(unsigned)plan_tiles, RP_T, 0, s>>>(a);
     SPG_LAUNCH_CHECK();
@@ -631,7 +637,6 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     SPG_CUDA_TRY(cudaMemcpyAsync(&h_over, a.ctr + RC_OVERFLOW, 8, cudaMemcpyDeviceToHost, s));
     SPG_CUDA_TRY(cudaMemcpyAsync(&out->n, a.off + n_rows, 8, cudaMemcpyDeviceToHost, s));
     SPG_TRY(c->phase_sync(s));
-    SPG_TRY(c->take_status());
     *done = h_over == 0;
     return SPG_OK;
 }
