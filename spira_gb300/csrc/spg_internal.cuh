@@ -315,8 +315,14 @@ __device__ __forceinline__ void warp_bitonic(K (&key)[E], int lane, int k0 = 2) 
 // zero, NaN is not; also exactly Spira's SpGEMM drop test `v != V{}`
 // (spgemm.hpp:44) negated. Tested on the bit pattern (every bit but the sign
 // clear): integer ALU work instead of an FP64 compare, which costs as much
-// FP64 pipe time as a multiply on GB300.
-__device__ __forceinline__ bool is_zero(double v) { return (__double_as_longlong(v) << 1) == 0; }
+// FP64 pipe time as a multiply on GB300. The words are taken apart in assembly:
+// written as (bits << 1) == 0, the compiler turns the test back into the FP64
+// compare (the FP64 pipe of kernels without any arithmetic was 8-22 % busy).
+__device__ __forceinline__ bool is_zero(double v) {
+    uint32_t lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(v));
+    return (lo | (hi << 1)) == 0;
+}
 
 // Lanes of the (full) warp whose NB-bit value d (a radix digit, or 256 for
 // "no key" when NB = 9) equals this lane's: NB ballots on the ALU pipe,
