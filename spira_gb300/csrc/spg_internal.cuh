@@ -556,6 +556,10 @@ int spgemm_esc(Ctx *c, const Csr *A, const Csr *B, const uint64_t *hp, uint64_t 
                EscOut *out, cudaStream_t s);
 void spgemm_install(Csr *Cm, uint64_t m, uint64_t n, DevBuf &&off, DevBuf &&cols, DevBuf &&vals, uint64_t nnz);
 uint64_t read_u64(Ctx *c, const uint64_t *d, cudaStream_t s, int *rc);
+// ROWMERGE's way when no row has more than SPGEMM_HASH_MAX products
+// (spg_spgemm_hash.cu).
+constexpr int SPGEMM_HASH_MAX = 64;
+int spgemm_hash_rows(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, uint64_t P, cudaStream_t s);
 int spgemm_warpsort(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, int variant, cudaStream_t s);
 int spgemm_run(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, int variant, cudaStream_t s);
 // SPG_SPGEMM_AUTO resolved by the context's policy (spg_tune.cu).
