@@ -494,21 +494,16 @@ int exclusive_scan_i64(Ctx *c, int64_t *d_data, uint64_t n, cudaStream_t s);
 // `key_bits` bits. Inputs are consumed; results land in (keys, vals) again.
 int radix_sort_pairs_u64(Ctx *c, uint64_t *d_keys, uint32_t *d_vals, uint64_t n,
                          int key_bits, cudaStream_t s);
-// Stable (row, col) order of m pairs whose rows are non-decreasing, sorted
-// row by row on chip (rows of up to 32 entries in registers, longer ones in
-// shared memory): keys_out = row << cbits | col, idx_out = input position.
-// s_off[r] = first position of row r (n_rows + 1 entries). *done = false when
-// a row has more than 12 288 entries or columns need more than 26 bits; the
-// outputs are then undefined.
-// The first lock of row-grouped inserts in one pass of the same sort: every
-// row's last write per column, unless zero, in column order at the row's
-// first input positions (out_cols / out_vals[s_off[r] + k], k < kept[r]);
-// kept[r] for every row r < n_rows. *done as for sort_grouped_rows.
+// A first lock's row-grouped inserts, sorted row by row on chip (rows of up to
+// 32 entries in registers, longer ones in shared memory): every row's last
+// write per column, unless zero, in column order at the row's first input
+// positions (out_cols / out_vals[s_off[r] + k], k < kept[r]); s_off[r] = first
+// position of row r (n_rows + 1 entries), kept[r] for every row r < n_rows.
+// *done = false when a row has more than 12 288 entries or columns need more
+// than 26 bits; the outputs are then undefined.
 int dedup_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off, uint64_t m,
                        uint64_t n_rows, int cbits, uint32_t *out_cols, double *out_vals, uint64_t *kept, bool *done,
                        cudaStream_t s);
-int sort_grouped_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const uint64_t *s_off, uint64_t m,
-                      uint64_t n_rows, int cbits, uint64_t *keys_out, uint32_t *idx_out, bool *done, cudaStream_t s);
 
 // A CSR's device arrays.
 struct CsrView {

@@ -461,15 +461,10 @@ __device__ __forceinline__ int seg_class(uint64_t L) {
     return 10;
 }
 
-// Where the sort puts a row's entries. Key mode (DEDUP = false): keys[p] =
-// row << cbits | col and idx[p] = input position, p over the row's input
-// positions in sorted order. Dedup mode (a first lock): the row's last write
-// per column, unless zero, in column order at the row's first input
-// positions (cols[s_off[r] + k], vals[s_off[r] + k]) and kept[r] = their
-// number.
+// Where the sort puts a row's entries: the row's last write per column, unless
+// zero, in column order at the row's first input positions
+// (cols[s_off[r] + k], vals[s_off[r] + k]) and kept[r] = their number.
 struct SegOut {
-    uint64_t *keys;
-    uint32_t *idx;
     const double *in_vals;
     uint32_t *cols;
     double *vals;
@@ -495,7 +490,6 @@ __global__ void __launch_bounds__(256) seg_count(const uint64_t *__restrict__ s_
 // Writes single-entry rows through and lists the rows of classes 6..9:
 // lists[base_c + k] for class c (base_c = the rows of the listed classes
 // below it; classes 7..9 are the tile kernels' lists). cur[c]: fill cursors.
-template <bool DEDUP>
 __global__ void __launch_bounds__(256) seg_place(const uint32_t *__restrict__ cols, const uint64_t *__restrict__ s_off,
                                                  uint64_t n_rows, int cbits, const unsigned *__restrict__ ctr,
                                                  unsigned *__restrict__ cur, uint32_t *__restrict__ lists, SegOut o) {
@@ -516,17 +510,12 @@ __global__ void __launch_bounds__(256) seg_place(const uint32_t *__restrict__ co
             const uint64_t b = s_off[r], L = s_off[r + 1] - b;
             c = seg_class(L);
             if (L == 1) {
-                if constexpr (DEDUP) {
-                    const double v = o.in_vals[b];
-                    o.cols[b] = cols[b];
-                    o.vals[b] = v;
-                    o.kept[r] = is_zero(v) ? 0 : 1;
-                } else {
-                    o.keys[b] = ((uint64_t)r << cbits) | cols[b];
-                    o.idx[b] = (uint32_t)b;
-                }
+                const double v = o.in_vals[b];
+                o.cols[b] = cols[b];
+                o.vals[b] = v;
+                o.kept[r] = is_zero(v) ? 0 : 1;
             } else if (L == 0) {
-                if constexpr (DEDUP) o.kept[r] = 0;
+                o.kept[r] = 0;
             } else if (c >= 6 && c <= 9) {
                 slot = atomicAdd(&sc[c], 1u);
             }
@@ -558,47 +547,37 @@ __device__ __forceinline__ uint32_t segment_bitonic(uint32_t key, int lane) {
 }
 
 // Rows (b, L, r) of one class, one per P-lane segment (L = 0: no row).
-template <int P, bool DEDUP>
+template <int P>
 __device__ __forceinline__ void sort_short_group(const uint32_t *__restrict__ cols, uint64_t b, uint64_t L,
                                                  uint64_t r, int cbits, const SegOut &o, int lane) {
     const int j = lane % P;
     uint32_t key = 0xFFFFFFFFu;  // real keys stay below 2^31: cbits <= 26
     double v_in = 0.0;
-    {
-        if ((uint64_t)j < L) {
-            key = (cols[b + j] << 5) | (uint32_t)j;
-            if constexpr (DEDUP) v_in = o.in_vals[b + j];  // in input order: coalesced
-        }
+    if ((uint64_t)j < L) {
+        key = (cols[b + j] << 5) | (uint32_t)j;
+        v_in = o.in_vals[b + j];  // in input order: coalesced
     }
     key = segment_bitonic<P>(key, lane);
-    if constexpr (!DEDUP) {
-        if ((uint64_t)j < L) {
-            o.keys[b + j] = (r << cbits) | (key >> 5);
-            o.idx[b + j] = (uint32_t)(b + (key & 31u));
-        }
-    } else {
-        // the last of a run of equal columns is the last write; kept unless
-        // zero. Its value comes from the lane that loaded it.
-        const uint32_t nxt = __shfl_down_sync(0xffffffffu, key, 1);
-        const double v = __shfl_sync(0xffffffffu, v_in, (lane & ~(P - 1)) | (int)(key & (uint32_t)(P - 1)));
-        bool keep = false;
-        if ((uint64_t)j < L && ((uint64_t)(j + 1) == L || (nxt >> 5) != (key >> 5))) keep = !is_zero(v);
-        const unsigned seg = P == 32 ? 0xffffffffu : ((1u << (P & 31)) - 1u) << (lane & ~(P - 1));
-        const unsigned bal = __ballot_sync(0xffffffffu, keep) & seg;
-        if (keep) {
-            const uint64_t w = b + (uint64_t)__popc(bal & ((1u << lane) - 1u));
-            o.cols[w] = key >> 5;
-            o.vals[w] = v;
-        }
-        if (j == 0 && L) o.kept[r] = (uint64_t)__popc(bal);
+    // the last of a run of equal columns is the last write; kept unless
+    // zero. Its value comes from the lane that loaded it.
+    const uint32_t nxt = __shfl_down_sync(0xffffffffu, key, 1);
+    const double v = __shfl_sync(0xffffffffu, v_in, (lane & ~(P - 1)) | (int)(key & (uint32_t)(P - 1)));
+    bool keep = false;
+    if ((uint64_t)j < L && ((uint64_t)(j + 1) == L || (nxt >> 5) != (key >> 5))) keep = !is_zero(v);
+    const unsigned seg = P == 32 ? 0xffffffffu : ((1u << (P & 31)) - 1u) << (lane & ~(P - 1));
+    const unsigned bal = __ballot_sync(0xffffffffu, keep) & seg;
+    if (keep) {
+        const uint64_t w = b + (uint64_t)__popc(bal & ((1u << lane) - 1u));
+        o.cols[w] = key >> 5;
+        o.vals[w] = v;
     }
+    if (j == 0 && L) o.kept[r] = (uint64_t)__popc(bal);
 }
 
 // Short rows: warp w takes rows [32 w, 32 w + 32) (grid-stride), reads
 // their offsets in one coalesced access, and sorts the rows of each short
 // class among them, 32 / P at a time (segment g of P lanes takes the class's
 // g-th remaining row).
-template <bool DEDUP>
 __global__ void __launch_bounds__(256) seg_short_sort(const uint32_t *__restrict__ cols,
                                                       const uint64_t *__restrict__ s_off, uint64_t n_rows, int cbits,
                                                       SegOut o) {
@@ -624,11 +603,11 @@ __global__ void __launch_bounds__(256) seg_short_sort(const uint32_t *__restrict
                 const uint64_t gr = w * 32 + (uint64_t)sl;
                 const uint64_t len = src < 32 ? gL : 0;
                 switch (cls) {
-                    case 1: sort_short_group<2, DEDUP>(cols, gb, len, gr, cbits, o, lane); break;
-                    case 2: sort_short_group<4, DEDUP>(cols, gb, len, gr, cbits, o, lane); break;
-                    case 3: sort_short_group<8, DEDUP>(cols, gb, len, gr, cbits, o, lane); break;
-                    case 4: sort_short_group<16, DEDUP>(cols, gb, len, gr, cbits, o, lane); break;
-                    default: sort_short_group<32, DEDUP>(cols, gb, len, gr, cbits, o, lane); break;
+                    case 1: sort_short_group<2>(cols, gb, len, gr, cbits, o, lane); break;
+                    case 2: sort_short_group<4>(cols, gb, len, gr, cbits, o, lane); break;
+                    case 3: sort_short_group<8>(cols, gb, len, gr, cbits, o, lane); break;
+                    case 4: sort_short_group<16>(cols, gb, len, gr, cbits, o, lane); break;
+                    default: sort_short_group<32>(cols, gb, len, gr, cbits, o, lane); break;
                 }
                 (void)P;
                 for (int k = 0; k < per && mask; ++k) mask &= mask - 1;  // drop the rows just sorted
@@ -685,7 +664,7 @@ __device__ __forceinline__ void warp_bitonic_looped(K (&key)[E], int lane) {
 // (Holding E consecutive elements per lane instead, so that near partners
 // meet in registers, measured 2.6x slower: strided loads and stores, and
 // twice the registers.)
-template <int E, class K, bool DEDUP>
+template <int E, class K>
 __device__ __forceinline__ void sort_medium_row(const uint32_t *__restrict__ cols, uint64_t b, uint32_t L, uint64_t r,
                                                 int cbits, const SegOut &o, int lane) {
     K key[E];
@@ -695,47 +674,36 @@ __device__ __forceinline__ void sort_medium_row(const uint32_t *__restrict__ col
         key[e] = p < L ? (((K)cols[b + p] << 9) | (K)p) : ~(K)0;
     }
     warp_bitonic_looped<E, K>(key, lane);
-    if constexpr (!DEDUP) {
+    uint32_t kept = 0;
+    const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const uint32_t p = 32u * e + lane;
-            if (p < L) {
-                o.keys[b + p] = (r << cbits) | (uint64_t)(key[e] >> 9);
-                o.idx[b + p] = (uint32_t)(b + (uint32_t)(key[e] & 511u));
-            }
+    for (int e = 0; e < E; ++e) {
+        const uint32_t p = 32u * e + lane;
+        // the next element: lane + 1 of the same register, or lane 0 of the next
+        K nx = __shfl_down_sync(0xffffffffu, key[e], 1);
+        if (e + 1 < E) {
+            const K f = __shfl_sync(0xffffffffu, key[e + 1 < E ? e + 1 : e], 0);
+            if (lane == 31) nx = f;
         }
-    } else {
-        uint32_t kept = 0;
-        const unsigned lt = (1u << lane) - 1u;
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const uint32_t p = 32u * e + lane;
-            // the next element: lane + 1 of the same register, or lane 0 of the next
-            K nx = __shfl_down_sync(0xffffffffu, key[e], 1);
-            if (e + 1 < E) {
-                const K f = __shfl_sync(0xffffffffu, key[e + 1 < E ? e + 1 : e], 0);
-                if (lane == 31) nx = f;
-            }
-            bool keep = false;
-            double v = 0.0;
-            if (p < L && (p + 1 == L || (nx >> 9) != (key[e] >> 9))) {  // last write of its column
-                v = o.in_vals[b + (uint32_t)(key[e] & 511u)];
-                keep = !is_zero(v);
-            }
-            const unsigned bal = __ballot_sync(0xffffffffu, keep);
-            if (keep) {
-                const uint64_t w = b + kept + (uint32_t)__popc(bal & lt);
-                o.cols[w] = (uint32_t)(key[e] >> 9);
-                o.vals[w] = v;
-            }
-            kept += (uint32_t)__popc(bal);
+        bool keep = false;
+        double v = 0.0;
+        if (p < L && (p + 1 == L || (nx >> 9) != (key[e] >> 9))) {  // last write of its column
+            v = o.in_vals[b + (uint32_t)(key[e] & 511u)];
+            keep = !is_zero(v);
         }
-        if (lane == 0) o.kept[r] = kept;
+        const unsigned bal = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+            const uint64_t w = b + kept + (uint32_t)__popc(bal & lt);
+            o.cols[w] = (uint32_t)(key[e] >> 9);
+            o.vals[w] = v;
+        }
+        kept += (uint32_t)__popc(bal);
     }
+    if (lane == 0) o.kept[r] = kept;
 }
 
 // Medium rows: a warp per row from the class-6 list.
-template <class K, bool DEDUP>
+template <class K>
 __global__ void __launch_bounds__(256, sizeof(K) == 8 ? 2 : 4) seg_medium_sort(const uint32_t *__restrict__ cols,
                                                        const uint64_t *__restrict__ s_off,
                                                        const uint32_t *__restrict__ lists,
@@ -747,10 +715,10 @@ __global__ void __launch_bounds__(256, sizeof(K) == 8 ? 2 : 4) seg_medium_sort(c
         const uint64_t r = lists[k];
         const uint64_t b = s_off[r];
         const uint32_t L = (uint32_t)(s_off[r + 1] - b);
-        if (L <= 64) sort_medium_row<2, K, DEDUP>(cols, b, L, r, cbits, o, lane);
-        else if (L <= 128) sort_medium_row<4, K, DEDUP>(cols, b, L, r, cbits, o, lane);
-        else if (L <= 256) sort_medium_row<8, K, DEDUP>(cols, b, L, r, cbits, o, lane);
-        else sort_medium_row<16, K, DEDUP>(cols, b, L, r, cbits, o, lane);
+        if (L <= 64) sort_medium_row<2, K>(cols, b, L, r, cbits, o, lane);
+        else if (L <= 128) sort_medium_row<4, K>(cols, b, L, r, cbits, o, lane);
+        else if (L <= 256) sort_medium_row<8, K>(cols, b, L, r, cbits, o, lane);
+        else sort_medium_row<16, K>(cols, b, L, r, cbits, o, lane);
     }
 }
 
@@ -761,31 +729,31 @@ constexpr uint16_t IDX_ZERO = 0x8000;  // row positions are < 2^14
 // consecutive entries, hit distinct banks.
 __device__ __forceinline__ uint32_t pad33(uint32_t p) { return p + (p >> 5); }
 
-template <int T, int I, bool DEDUP>
+template <int T, int I>
 struct TileSmem {
     static constexpr int MAXE = T * I;
     static constexpr int NCTR = RS_WORDS * T;
-    static constexpr bool VSTAGE = DEDUP && MAXE <= 4096;  // values staged in shared memory
+    static constexpr bool VSTAGE = MAXE <= 4096;  // values staged in shared memory
     union {  // the counters live only inside a radix pass, the exchange arrays between passes
         uint32_t ctr[NCTR + NCTR / 32];  // counter word w of thread t at pad33(w T + t)
         struct {
             uint32_t key[MAXE + MAXE / 32];
-            uint16_t idx[MAXE + MAXE / 32];  // row position; dedup mode: | IDX_ZERO if the value is zero
-            uint32_t ex[MAXE + MAXE / 32 + 2];  // dedup mode: kept entries before each position
+            uint16_t idx[MAXE + MAXE / 32];  // row position; | IDX_ZERO if the value is zero
+            uint32_t ex[MAXE + MAXE / 32 + 2];  // kept entries before each position
         } x;
     } u;
-    double val[VSTAGE ? MAXE : 1];  // dedup mode: values by row position, kept through every pass
+    double val[VSTAGE ? MAXE : 1];  // values by row position, kept through every pass
     uint32_t wsum[T / 32];
 };
 
 // Rows of tile kernel KI's list (class 7 + KI, T * I entries at most), a
 // block per row; persistent blocks take rows in a grid-stride loop.
-template <int T, int I, bool DEDUP>
+template <int T, int I>
 __global__ void __launch_bounds__(T, T <= 128 ? 6 : T <= 256 ? 3 : 1)
 seg_tile_sort(const uint32_t *__restrict__ cols, const uint64_t *__restrict__ s_off,
               const uint32_t *__restrict__ lists, const unsigned *__restrict__ ctr, int ki, int cbits, SegOut o,
               unsigned *__restrict__ overflow) {
-    using Sm = TileSmem<T, I, DEDUP>;
+    using Sm = TileSmem<T, I>;
     constexpr int W = T / 32;
     extern __shared__ __align__(16) unsigned char ts_raw[];
     Sm &S = *reinterpret_cast<Sm *>(ts_raw);
@@ -803,16 +771,14 @@ seg_tile_sort(const uint32_t *__restrict__ cols, const uint64_t *__restrict__ s_
             continue;
         }
         const int passes = (cbits + RS_DBITS - 1) / RS_DBITS;
-        // coalesced load in input order into the exchange arrays (dedup mode:
-        // each value read once; its zero test rides in the position's top bit)
+        // coalesced load in input order into the exchange arrays (each
+        // value read once; its zero test rides in the position's top bit)
         for (int e = t; e < E; e += T) {
             S.u.x.key[pad33(e)] = cols[b + e];
             uint16_t ix = (uint16_t)e;
-            if constexpr (DEDUP) {
-                const double v = o.in_vals[b + e];
-                if (is_zero(v)) ix |= IDX_ZERO;
-                if constexpr (Sm::VSTAGE) S.val[e] = v;
-            }
+            const double v = o.in_vals[b + e];
+            if (is_zero(v)) ix |= IDX_ZERO;
+            if constexpr (Sm::VSTAGE) S.val[e] = v;
             S.u.x.idx[pad33(e)] = ix;
         }
         __syncthreads();
@@ -911,73 +877,66 @@ seg_tile_sort(const uint32_t *__restrict__ cols, const uint64_t *__restrict__ s_
                 }
             }
         }
-        if constexpr (!DEDUP) {
-            for (int q = t; q < E; q += T) {
-                o.keys[b + q] = ((uint64_t)r << cbits) | S.u.x.key[pad33(q)];
-                o.idx[b + q] = (uint32_t)(b + S.u.x.idx[pad33(q)]);
-            }
-        } else {
-            // keep = last of a run of equal columns (the last write) and not
-            // zero; ex = exclusive count of kept entries
-            uint32_t keepm = 0, cnt = 0;
+        // keep = last of a run of equal columns (the last write) and not
+        // zero; ex = exclusive count of kept entries
+        uint32_t keepm = 0, cnt = 0;
 #pragma unroll
-            for (int i = 0; i < I; ++i) {
-                const int q = t * I + i;
-                if (q < E) {
-                    const uint32_t k = S.u.x.key[pad33(q)];
-                    if ((q + 1 == E || S.u.x.key[pad33(q + 1)] != k) && !(S.u.x.idx[pad33(q)] & IDX_ZERO)) {
-                        keepm |= 1u << i;
-                        ++cnt;
-                    }
+        for (int i = 0; i < I; ++i) {
+            const int q = t * I + i;
+            if (q < E) {
+                const uint32_t k = S.u.x.key[pad33(q)];
+                if ((q + 1 == E || S.u.x.key[pad33(q + 1)] != k) && !(S.u.x.idx[pad33(q)] & IDX_ZERO)) {
+                    keepm |= 1u << i;
+                    ++cnt;
                 }
             }
-            uint32_t inc = cnt;
+        }
+        uint32_t inc = cnt;
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t x = __shfl_up_sync(0xffffffffu, inc, d);
-                if (lane >= d) inc += x;
-            }
-            if (lane == 31) S.wsum[warp] = inc;
-            __syncthreads();
-            uint32_t run = inc - cnt, total = 0;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += x;
+        }
+        if (lane == 31) S.wsum[warp] = inc;
+        __syncthreads();
+        uint32_t run = inc - cnt, total = 0;
 #pragma unroll
-            for (int w = 0; w < W; ++w) {
-                const uint32_t x = S.wsum[w];
-                if (w < warp) run += x;
-                total += x;
-            }
+        for (int w = 0; w < W; ++w) {
+            const uint32_t x = S.wsum[w];
+            if (w < warp) run += x;
+            total += x;
+        }
 #pragma unroll
-            for (int i = 0; i < I; ++i) {
-                const int q = t * I + i;
-                if (q < E) {
-                    S.u.x.ex[pad33(q)] = run;
-                    run += (keepm >> i) & 1u;
-                }
+        for (int i = 0; i < I; ++i) {
+            const int q = t * I + i;
+            if (q < E) {
+                S.u.x.ex[pad33(q)] = run;
+                run += (keepm >> i) & 1u;
             }
-            if (t == 0) {
-                S.u.x.ex[pad33(E)] = total;
-                o.kept[r] = total;
-            }
-            __syncthreads();
-            for (int q = t; q < E; q += T) {
-                const uint32_t e0 = S.u.x.ex[pad33(q)];
-                if (S.u.x.ex[pad33(q + 1)] != e0) {
-                    const unsigned tp = S.u.x.idx[pad33(q)] & ~IDX_ZERO;
-                    o.cols[b + e0] = S.u.x.key[pad33(q)];
-                    if constexpr (Sm::VSTAGE) o.vals[b + e0] = S.val[tp];
-                    else o.vals[b + e0] = o.in_vals[b + tp];
-                }
+        }
+        if (t == 0) {
+            S.u.x.ex[pad33(E)] = total;
+            o.kept[r] = total;
+        }
+        __syncthreads();
+        for (int q = t; q < E; q += T) {
+            const uint32_t e0 = S.u.x.ex[pad33(q)];
+            if (S.u.x.ex[pad33(q + 1)] != e0) {
+                const unsigned tp = S.u.x.idx[pad33(q)] & ~IDX_ZERO;
+                o.cols[b + e0] = S.u.x.key[pad33(q)];
+                if constexpr (Sm::VSTAGE) o.vals[b + e0] = S.val[tp];
+                else o.vals[b + e0] = o.in_vals[b + tp];
             }
         }
         __syncthreads();  // shared state is rebuilt by the next row
     }
 }
 
-template <int T, int I, bool DEDUP>
+template <int T, int I>
 int launch_tile_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, const uint32_t *lists, const unsigned *ctr,
                      int ki, uint64_t max_rows, int cbits, const SegOut &o, unsigned *overflow, cudaStream_t s) {
-    auto k = seg_tile_sort<T, I, DEDUP>;
-    constexpr size_t smem = sizeof(TileSmem<T, I, DEDUP>);
+    auto k = seg_tile_sort<T, I>;
+    constexpr size_t smem = sizeof(TileSmem<T, I>);
     SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     SPG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, T, smem));
@@ -989,7 +948,6 @@ int launch_tile_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, const 
     return SPG_OK;
 }
 
-template <bool DEDUP>
 int seg_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, uint64_t m, uint64_t n_rows, int cbits,
              const SegOut &o, bool *done, cudaStream_t s) {
     *done = false;
@@ -1003,21 +961,21 @@ int seg_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, uint64_t m, ui
     const unsigned gr = grid_for(n_rows, 256, (unsigned)c->n_sms * 8);
     seg_count<<<gr, 256, 0, s>>>(s_off, n_rows, ctr);
     SPG_LAUNCH_CHECK();
-    seg_place<DEDUP><<<gr, 256, 0, s>>>(cols, s_off, n_rows, cbits, ctr, cur, lists, o);
+    seg_place<<<gr, 256, 0, s>>>(cols, s_off, n_rows, cbits, ctr, cur, lists, o);
     SPG_LAUNCH_CHECK();
-    seg_short_sort<DEDUP><<<grid_for((n_rows + 31) / 32, 8, (unsigned)c->n_sms * 16), 256, 0, s>>>(cols, s_off, n_rows,
+    seg_short_sort<<<grid_for((n_rows + 31) / 32, 8, (unsigned)c->n_sms * 16), 256, 0, s>>>(cols, s_off, n_rows,
                                                                                                 cbits, o);
     SPG_LAUNCH_CHECK();
     // (8 blocks per SM: twice what fits at once, which balanced rows of
     // unequal length better than one wave)
-    if (cbits <= 22) seg_medium_sort<uint32_t, DEDUP><<<(unsigned)c->n_sms * 8, 256, 0, s>>>(cols, s_off, lists, ctr, cbits, o);
-    else seg_medium_sort<uint64_t, DEDUP><<<(unsigned)c->n_sms * 8, 256, 0, s>>>(cols, s_off, lists, ctr, cbits, o);
+    if (cbits <= 22) seg_medium_sort<uint32_t><<<(unsigned)c->n_sms * 8, 256, 0, s>>>(cols, s_off, lists, ctr, cbits, o);
+    else seg_medium_sort<uint64_t><<<(unsigned)c->n_sms * 8, 256, 0, s>>>(cols, s_off, lists, ctr, cbits, o);
     SPG_LAUNCH_CHECK();
-    SPG_TRY((launch_tile_sort<TS0_T, TS0_I, DEDUP>(c, cols, s_off, lists, ctr, 0, m / (SEG_MEDIUM + 1) + 1, cbits,
+    SPG_TRY((launch_tile_sort<TS0_T, TS0_I>(c, cols, s_off, lists, ctr, 0, m / (SEG_MEDIUM + 1) + 1, cbits,
                                                    o, ovf, s)));
-    SPG_TRY((launch_tile_sort<TS1_T, TS1_I, DEDUP>(c, cols, s_off, lists, ctr, 1, m / (TS0 + 1) + 1, cbits, o, ovf,
+    SPG_TRY((launch_tile_sort<TS1_T, TS1_I>(c, cols, s_off, lists, ctr, 1, m / (TS0 + 1) + 1, cbits, o, ovf,
                                                    s)));
-    SPG_TRY((launch_tile_sort<TS2_T, TS2_I, DEDUP>(c, cols, s_off, lists, ctr, 2, m / (TS1 + 1) + 1, cbits, o, ovf,
+    SPG_TRY((launch_tile_sort<TS2_T, TS2_I>(c, cols, s_off, lists, ctr, 2, m / (TS1 + 1) + 1, cbits, o, ovf,
                                                    s)));
     unsigned h = 1u;
     SPG_CUDA_TRY(cudaMemcpyAsync(&h, ovf, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
@@ -1027,19 +985,6 @@ int seg_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, uint64_t m, ui
 }
 
 }  // namespace
-
-int sort_grouped_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const uint64_t *s_off, uint64_t m,
-                      uint64_t n_rows, int cbits, uint64_t *keys_out, uint32_t *idx_out, bool *done, cudaStream_t s) {
-    (void)rows;  // the rows are s_off's
-    if (m == 0) {
-        *done = true;
-        return SPG_OK;
-    }
-    SegOut o{};
-    o.keys = keys_out;
-    o.idx = idx_out;
-    return seg_sort<false>(c, cols, s_off, m, n_rows, cbits, o, done, s);
-}
 
 int dedup_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off, uint64_t m,
                        uint64_t n_rows, int cbits, uint32_t *out_cols, double *out_vals, uint64_t *kept, bool *done,
@@ -1054,7 +999,7 @@ int dedup_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
         *done = true;
         return SPG_OK;
     }
-    return seg_sort<true>(c, cols, s_off, m, n_rows, cbits, o, done, s);
+    return seg_sort(c, cols, s_off, m, n_rows, cbits, o, done, s);
 }
 
 }  // namespace spg

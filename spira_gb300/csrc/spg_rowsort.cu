@@ -252,8 +252,8 @@ int sort_staged_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const d
     SPG_TRY(out.abort.alloc(sizeof(unsigned long long), s));
     SPG_CUDA_TRY(cudaMemsetAsync(out.abort.ptr, 0, sizeof(unsigned long long), s));
     SPG_TRY(out.rows.alloc(m * sizeof(uint32_t), s));
-    SPG_TRY(out.cols.alloc(m * sizeof(uint32_t), s));
-    SPG_TRY(out.vals.alloc(m * sizeof(double), s));
+    SPG_TRY(out.cols.alloc(csr_alloc_elems(m) * sizeof(uint32_t), s));  // (a CSR's arrays, for the transpose)
+    SPG_TRY(out.vals.alloc(csr_alloc_elems(m) * sizeof(double), s));
     if (passes > 1) {
         SPG_TRY(rows2.alloc(m * sizeof(uint32_t), s));
         SPG_TRY(cols2.alloc(m * sizeof(uint32_t), s));

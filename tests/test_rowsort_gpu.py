@@ -79,3 +79,18 @@ def test_lock_small_later_epoch(ctx, n_rows, per_row, m, order):
     A.lock(*first)
     A.lock(r, c, v)
     assert_csr_equal(A.download(), oracle.lock_epochs(n_rows, n_cols, [first, (r, c, v)]))
+
+
+@pytest.mark.parametrize("n_rows,n_cols,m", [
+    (3000, 90, 50_000),            # every column above 32 entries
+    (5, 40_000, 60_000),           # source rows of 12 000, columns of one or two
+    (20_000, 20_000, 400_000),     # a few columns above 32
+    (9000, 1, 9000),               # one column
+    (70_000, 300, 2_500_000),      # the large tiles
+])
+def test_transpose_by_column_sort(ctx, n_rows, n_cols, m):
+    first = _inserts(m, n_rows, n_cols, seed=m)
+    H = oracle.lock_epochs(n_rows, n_cols, [first])
+    A = sg.Csr(ctx, n_rows, n_cols)
+    A.load(H.off, H.cols, H.vals)
+    assert_csr_equal(A.transpose().download(), oracle.transpose(H))
