@@ -324,6 +324,9 @@ __device__ __forceinline__ bool is_zero(double v) {
     return (lo | (hi << 1)) == 0;
 }
 
+// Brings p's line into the L2 (no fault, no wait).
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Lanes of the (full) warp whose NB-bit value d (a radix digit, or 256 for
 // "no key" when NB = 9) equals this lane's: NB ballots on the ALU pipe,
 // cheaper on GB300 than match.any, which issues on the narrow

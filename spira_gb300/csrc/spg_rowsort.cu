@@ -12,7 +12,11 @@
 // to their digit-ordered places in shared memory (cp.async), from where every
 // digit's run goes out on consecutive addresses.
 //
-// Bound: 32 bytes per entry and pass of HBM traffic. Sorting only the row bits
+// Bound: 32 bytes per entry and pass of HBM traffic, half of the time taken (a
+// pass over 10 M entries: 101 us, 47 at the copy rate); the rest is latency
+// between the barriers of three blocks an SM. 116 us before the columns and
+// values were prefetched into the L2 during the ranking and the digit's bits
+// were a constant of the code. Sorting only the row bits
 // and leaving each row to the row kernels takes 3 passes for 2 M rows where
 // the (row, column) keys took 6, of three launches each and with an index that
 // fetched every value at random afterwards.
@@ -70,10 +74,10 @@ struct RsSmem {
     uint64_t tile;
 };
 
-template <int T, int I, int PER_SM>
+template <int T, int I, int PER_SM, int BITS>
 __global__ void __launch_bounds__(T, PER_SM)
 rs_pass(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, const double *__restrict__ vals,
-        uint64_t m, int shift, int bits, const unsigned long long *__restrict__ hist,
+        uint64_t m, int shift, const unsigned long long *__restrict__ hist,
         unsigned long long *__restrict__ ticket, unsigned long long *__restrict__ state,
         uint32_t *__restrict__ out_rows, uint32_t *__restrict__ out_cols, double *__restrict__ out_vals,
         unsigned int *__restrict__ status, unsigned long long *__restrict__ abort) {
@@ -88,7 +92,10 @@ rs_pass(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, co
     __syncthreads();
     const uint64_t tile = S.tile, t0 = tile * TILE;
     const int n = (int)min((uint64_t)TILE, m - t0);
-    const uint32_t mask = (1u << bits) - 1u;
+    // the columns and values are wanted once the ranks are known: into the L2 meanwhile
+    for (int i = t * 32; i < n; i += T * 32) prefetch_l2(cols + t0 + i);
+    for (int i = t * 16; i < n; i += T * 16) prefetch_l2(vals + t0 + i);
+    constexpr uint32_t mask = (1u << BITS) - 1u;
     // warp w owns entries [w 32 I, (w + 1) 32 I) of the tile and walks them in order
     const int base = warp * (I * 32) + lane;
     uint32_t r[I], rank[I];
@@ -104,11 +111,9 @@ rs_pass(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, co
         const uint32_t d = (r[j] >> shift) & mask;
         unsigned peers = valid;
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            if (b < bits) {
-                const unsigned bit = (d >> b) & 1u, bal = __ballot_sync(0xffffffffu, bit);
-                peers &= bit ? bal : ~bal;
-            }
+        for (int b = 0; b < BITS; ++b) {
+            const unsigned bit = (d >> b) & 1u, bal = __ballot_sync(0xffffffffu, bit);
+            peers &= bit ? bal : ~bal;
         }
         uint32_t before = 0;
         if (ok) before = S.cnt[warp][d];
@@ -120,7 +125,7 @@ rs_pass(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, co
     __syncthreads();
     // digit t: exclusive prefix over the warps, its tile count published, and
     // exclusive scans over the digits of the tile's and the global counts
-    const bool digit = t < RS_RADIX;  // whole warps
+    const bool digit = t < max(32, 1 << BITS);  // whole warps
     uint32_t tot = 0, place = 0;
     uint64_t gplace = 0;
     unsigned long long *mine = state + tile * RS_RADIX + t;
@@ -221,25 +226,37 @@ rs_pass(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, co
     }
 }
 
-template <int T, int I, int PER_SM>
-int rs_launch(const uint32_t *rows, const uint32_t *cols, const double *vals, uint64_t m, int shift, int bits,
+template <int T, int I, int PER_SM, int BITS>
+int rs_launch(const uint32_t *rows, const uint32_t *cols, const double *vals, uint64_t m, int shift,
               const unsigned long long *hist, unsigned long long *ticket, unsigned long long *state, uint32_t *orows,
               uint32_t *ocols, double *ovals, unsigned int *status, unsigned long long *abort, cudaStream_t s) {
-    auto k = rs_pass<T, I, PER_SM>;
+    auto k = rs_pass<T, I, PER_SM, BITS>;
     constexpr size_t smem = sizeof(RsSmem<T, I>);
     SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint64_t tiles = (m + T * I - 1) / (T * I);
-    k<<<(unsigned)tiles, T, smem, s>>>(rows, cols, vals, m, shift, bits, hist, ticket, state, orows, ocols, ovals,
+    k<<<(unsigned)tiles, T, smem, s>>>(rows, cols, vals, m, shift, hist, ticket, state, orows, ocols, ovals,
                                        status, abort);
     SPG_LAUNCH_CHECK();
     return SPG_OK;
+}
+
+using RsLaunch = decltype(&rs_launch<RS_LT, RS_LI, RS_LB, 8>);
+
+template <int T, int I, int PER_SM>
+RsLaunch rs_launch_of(int bits) {
+    switch (bits) {
+        case 5: return rs_launch<T, I, PER_SM, 5>;
+        case 6: return rs_launch<T, I, PER_SM, 6>;
+        case 7: return rs_launch<T, I, PER_SM, 7>;
+        default: return rs_launch<T, I, PER_SM, 8>;
+    }
 }
 
 }  // namespace
 
 int sort_staged_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const double *vals, uint64_t m, int rbits,
                      StagedSorted &out, cudaStream_t s) {
-    const int passes = std::max(1, (rbits + 7) / 8), bits = std::max(1, (rbits + passes - 1) / passes);
+    const int passes = std::max(1, (rbits + 7) / 8), bits = std::max(5, (rbits + passes - 1) / passes);
     // tiles of RS_LT x RS_LI entries, or of 1024 while those are too few to fill the chip
     const bool large = m >= (uint64_t)c->n_sms * RS_LB * RS_LT * RS_LI;
     const uint64_t tile = large ? RS_LT * RS_LI : 256 * 4, tiles = (m + tile - 1) / tile;
@@ -261,14 +278,14 @@ int sort_staged_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const d
     }
     rs_hist<<<grid_for(m, RS_T * 16, (unsigned)c->n_sms * 4), RS_T, 0, s>>>(rows, m, passes, bits, hist);
     SPG_LAUNCH_CHECK();
+    const RsLaunch launch = large ? rs_launch_of<RS_LT, RS_LI, RS_LB>(bits) : rs_launch_of<256, 4, 6>(bits);
     const uint32_t *ir = rows, *ic = cols;
     const double *iv = vals;
     for (int p = 0; p < passes; ++p) {
         const bool to_out = (passes - 1 - p) % 2 == 0;  // the last pass ends in the outputs
         uint32_t *orr = (to_out ? out.rows : rows2).as<uint32_t>(), *oc = (to_out ? out.cols : cols2).as<uint32_t>();
         double *ov = (to_out ? out.vals : vals2).as<double>();
-        auto launch = large ? rs_launch<RS_LT, RS_LI, RS_LB> : rs_launch<256, 4, 6>;
-        SPG_TRY(launch(ir, ic, iv, m, p * bits, bits, hist + p * RS_RADIX, ticket + p, state + p * tiles * RS_RADIX, orr,
+        SPG_TRY(launch(ir, ic, iv, m, p * bits, hist + p * RS_RADIX, ticket + p, state + p * tiles * RS_RADIX, orr,
                        oc, ov, c->d_status, out.abort.as<unsigned long long>(), s));
         ir = orr;
         ic = oc;

@@ -40,10 +40,12 @@ def test_lock_rows_in_no_order(ctx, n_rows, m):
 
 
 @pytest.mark.parametrize("n_rows,n_cols,m,skew", [
-    (300_000, 300_000, 2_000_003, False),   # the large tiles
+    (300_000, 300_000, 2_000_003, False),   # the large tiles, digits of 7 bits
+    (300, 400_000, 1_500_003, False),       # of 5
+    (4000, 400_000, 1_500_003, False),      # of 6
     (9_000, 500_000, 4_500_000, False),     # more than the few-inserts rule: rows of 500
     (50_000, 1000, 30_000, True),           # one row too long for the row kernels, runs of one row
-    (50_000, 100_000, 2_000_003, True),
+    (50_000, 100_000, 2_000_003, True),     # of 8
 ])
 def test_lock_rows_in_no_order_large(ctx, n_rows, n_cols, m, skew):
     first, later = _inserts(m, n_rows, n_cols, 5, skew), _inserts(m // 7, n_rows, n_cols, 6, skew)
