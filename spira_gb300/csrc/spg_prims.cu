@@ -405,7 +405,7 @@ int radix_sort_pairs_u64(Ctx *c, uint64_t *d_keys, uint32_t *d_vals, uint64_t n,
 // Rows are sorted by length class:
 //   * one entry: written through by the planning pass;
 //   * 2..32 entries: a bitonic network in registers, 32 / P rows of padded
-//     length P (2, 4, 8, 16, 32) per warp, keys (col << 5 | position); a warp
+//     length P (2, 4, 8, 16, 32) per warp and step, keys (col << 5 | position); a warp
 //     takes 32 consecutive rows (their offsets in one coalesced read) and
 //     sorts each class present among them in turn;
 //   * 33..SEG_MEDIUM entries: one warp per row, a bitonic network over the
@@ -546,73 +546,92 @@ __device__ __forceinline__ uint32_t segment_bitonic(uint32_t key, int lane) {
     return key;
 }
 
-// Rows (b, L, r) of one class, one per P-lane segment (L = 0: no row).
-template <int P>
-__device__ __forceinline__ void sort_short_group(const uint32_t *__restrict__ cols, uint64_t b, uint64_t L,
-                                                 uint64_t r, int cbits, const SegOut &o, int lane) {
-    const int j = lane % P;
-    uint32_t key = 0xFFFFFFFFu;  // real keys stay below 2^31: cbits <= 26
-    double v_in = 0.0;
-    if ((uint64_t)j < L) {
-        key = (cols[b + j] << 5) | (uint32_t)j;
-        v_in = o.in_vals[b + j];  // in input order: coalesced
+// n rows of one class, U x 32 / P at a time (one per P-lane segment): lane
+// ord[k] of the warp holds row k's first entry b and length L, and its row is
+// r0 + ord[k].
+template <int P, int U>
+__device__ __forceinline__ void sort_short_class(const uint32_t *__restrict__ cols, const uint8_t *ord, int n,
+                                                 uint64_t b, uint32_t L, uint64_t r0, const SegOut &o, int lane) {
+    constexpr int PER = 32 / P;
+    const int j = lane % P, g = lane / P;
+    for (int k0 = 0; k0 < n; k0 += U * PER) {
+        uint32_t key[U], len[U];
+        uint64_t first[U];
+        double v_in[U];
+        int src[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + u * PER + g;
+            src[u] = k < n ? ord[k] : 0;
+            first[u] = __shfl_sync(0xffffffffu, b, src[u]);
+            len[u] = __shfl_sync(0xffffffffu, L, src[u]);
+            if (k >= n) len[u] = 0;
+            key[u] = 0xFFFFFFFFu;  // real keys stay below 2^31: cbits <= 26
+            v_in[u] = 0.0;
+            if ((uint32_t)j < len[u]) {
+                key[u] = (cols[first[u] + j] << 5) | (uint32_t)j;
+                v_in[u] = o.in_vals[first[u] + j];  // in input order: coalesced
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (u > 0 && k0 + u * PER >= n) break;  // (the same for the whole warp)
+            key[u] = segment_bitonic<P>(key[u], lane);
+            // the last of a run of equal columns is the last write; kept unless
+            // zero. Its value comes from the lane that loaded it.
+            const uint32_t nxt = __shfl_down_sync(0xffffffffu, key[u], 1);
+            const double v = __shfl_sync(0xffffffffu, v_in[u], (lane & ~(P - 1)) | (int)(key[u] & (uint32_t)(P - 1)));
+            bool keep = false;
+            if ((uint32_t)j < len[u] && ((uint32_t)(j + 1) == len[u] || (nxt >> 5) != (key[u] >> 5))) keep = !is_zero(v);
+            const unsigned seg = P == 32 ? 0xffffffffu : ((1u << (P & 31)) - 1u) << (lane & ~(P - 1));
+            const unsigned bal = __ballot_sync(0xffffffffu, keep) & seg;
+            if (keep) {
+                const uint64_t w = first[u] + (uint64_t)__popc(bal & ((1u << lane) - 1u));
+                o.cols[w] = key[u] >> 5;
+                o.vals[w] = v;
+            }
+            if (j == 0 && len[u]) o.kept[r0 + src[u]] = (uint64_t)__popc(bal);
+        }
     }
-    key = segment_bitonic<P>(key, lane);
-    // the last of a run of equal columns is the last write; kept unless
-    // zero. Its value comes from the lane that loaded it.
-    const uint32_t nxt = __shfl_down_sync(0xffffffffu, key, 1);
-    const double v = __shfl_sync(0xffffffffu, v_in, (lane & ~(P - 1)) | (int)(key & (uint32_t)(P - 1)));
-    bool keep = false;
-    if ((uint64_t)j < L && ((uint64_t)(j + 1) == L || (nxt >> 5) != (key >> 5))) keep = !is_zero(v);
-    const unsigned seg = P == 32 ? 0xffffffffu : ((1u << (P & 31)) - 1u) << (lane & ~(P - 1));
-    const unsigned bal = __ballot_sync(0xffffffffu, keep) & seg;
-    if (keep) {
-        const uint64_t w = b + (uint64_t)__popc(bal & ((1u << lane) - 1u));
-        o.cols[w] = key >> 5;
-        o.vals[w] = v;
-    }
-    if (j == 0 && L) o.kept[r] = (uint64_t)__popc(bal);
 }
 
 // Short rows: warp w takes rows [32 w, 32 w + 32) (grid-stride), reads
-// their offsets in one coalesced access, and sorts the rows of each short
-// class among them, 32 / P at a time (segment g of P lanes takes the class's
-// g-th remaining row).
+// their offsets in one coalesced access, orders its lanes by their rows' class
+// and sorts each class's rows. Bound: latency, so the loads of up to four
+// rows per segment are issued together (five entries a row, 10 M entries: 81
+// us; two 104, eight 125 for the registers). Finding a class's g-th row in its
+// ballot with __fns and one row per segment at a time took 130.
 __global__ void __launch_bounds__(256) seg_short_sort(const uint32_t *__restrict__ cols,
-                                                      const uint64_t *__restrict__ s_off, uint64_t n_rows, int cbits,
-                                                      SegOut o) {
+                                                      const uint64_t *__restrict__ s_off, uint64_t n_rows, SegOut o) {
+    __shared__ uint8_t s_ord[256 / 32][32];  // the warp's lanes by class
     const int lane = threadIdx.x & 31;
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    uint8_t *const ord = s_ord[threadIdx.x >> 5];
     for (uint64_t w = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); w * 32 < n_rows; w += warps) {
-        const uint64_t r = w * 32 + lane;
-        uint64_t b = 0, L = 0;
-        if (r < n_rows) {
-            b = s_off[r];
-            L = s_off[r + 1] - b;
+        const uint64_t r0 = w * 32;
+        uint64_t b = 0, len = 0;
+        if (r0 + lane < n_rows) {
+            b = s_off[r0 + lane];
+            len = s_off[r0 + lane + 1] - b;
         }
-        const int c = (L >= 2 && L <= 32) ? 32 - __clz((unsigned)(L - 1)) : 0;
+        const uint32_t L = len <= 32 ? (uint32_t)len : 0u;
+        const int c = L >= 2 ? 32 - __clz((int)(L - 1)) : 0;
+        int n[6], at = 0;  // rows of each class
 #pragma unroll
         for (int cls = 1; cls <= 5; ++cls) {
-            unsigned mask = __ballot_sync(0xffffffffu, c == cls);
-            const int P = 1 << cls, per = 32 >> cls;
-            while (mask) {
-                const int g = lane >> cls;  // this lane's segment
-                const unsigned src = __fns(mask, 0, g + 1);  // the segment's row: g-th set lane of mask
-                const int sl = src < 32 ? (int)src : 0;
-                const uint64_t gb = __shfl_sync(0xffffffffu, b, sl), gL = __shfl_sync(0xffffffffu, L, sl);
-                const uint64_t gr = w * 32 + (uint64_t)sl;
-                const uint64_t len = src < 32 ? gL : 0;
-                switch (cls) {
-                    case 1: sort_short_group<2>(cols, gb, len, gr, cbits, o, lane); break;
-                    case 2: sort_short_group<4>(cols, gb, len, gr, cbits, o, lane); break;
-                    case 3: sort_short_group<8>(cols, gb, len, gr, cbits, o, lane); break;
-                    case 4: sort_short_group<16>(cols, gb, len, gr, cbits, o, lane); break;
-                    default: sort_short_group<32>(cols, gb, len, gr, cbits, o, lane); break;
-                }
-                (void)P;
-                for (int k = 0; k < per && mask; ++k) mask &= mask - 1;  // drop the rows just sorted
-            }
+            const unsigned mask = __ballot_sync(0xffffffffu, c == cls);
+            n[cls] = __popc(mask);
+            if (c == cls) ord[at + __popc(mask & ((1u << lane) - 1u))] = (uint8_t)lane;
+            at += n[cls];
         }
+        __syncwarp();
+        const uint8_t *p = ord;
+        sort_short_class<2, 4>(cols, p, n[1], b, L, r0, o, lane);
+        sort_short_class<4, 4>(cols, p += n[1], n[2], b, L, r0, o, lane);
+        sort_short_class<8, 4>(cols, p += n[2], n[3], b, L, r0, o, lane);
+        sort_short_class<16, 2>(cols, p += n[3], n[4], b, L, r0, o, lane);
+        sort_short_class<32, 1>(cols, p += n[4], n[5], b, L, r0, o, lane);
+        __syncwarp();  // the next rows' order overwrites this one
     }
 }
 
@@ -963,8 +982,7 @@ int seg_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, uint64_t m, ui
     SPG_LAUNCH_CHECK();
     seg_place<<<gr, 256, 0, s>>>(cols, s_off, n_rows, cbits, ctr, cur, lists, o);
     SPG_LAUNCH_CHECK();
-    seg_short_sort<<<grid_for((n_rows + 31) / 32, 8, (unsigned)c->n_sms * 16), 256, 0, s>>>(cols, s_off, n_rows,
-                                                                                                cbits, o);
+    seg_short_sort<<<grid_for((n_rows + 31) / 32, 8, (unsigned)c->n_sms * 16), 256, 0, s>>>(cols, s_off, n_rows, o);
     SPG_LAUNCH_CHECK();
     // (8 blocks per SM: twice what fits at once, which balanced rows of
     // unequal length better than one wave)
