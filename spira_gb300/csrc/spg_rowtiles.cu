@@ -14,17 +14,24 @@
 //      clustered in a long row, or many duplicates) are split again over
 //      their own column range until none is left;
 //   3. an entry's sorted place is its bucket's first slot plus the bucket's
-//      entries before it by (column, input position): a few compares;
+//      entries before it by (column, input position): a few compares, for
+//      four entries at a time;
 //   4. the last entry of a run of equal columns is the last write; its keep
 //      bit is a ballot, the tile's kept count goes through an ordered scan
 //      (look-back), and the tile writes its rows' offsets and entries into
 //      the CSR, consecutive threads on consecutive entries.
 // Rows of more than RT_CAP entries are ordered beforehand by larger blocks
-// (the same steps) into scratch at their input positions; their tiles copy.
+// (the same steps, two sizes) into scratch at their input positions; their
+// tiles copy.
 //
-// Bound: 24 bytes per entry of HBM traffic (12 in, 12 out) and about 120
-// thread-instructions per entry. It replaces per-class sorting kernels (a
-// segmented bitonic network up to 32 entries, a warp bitonic network up to
+// Floor: 24 bytes per entry of HBM traffic (12 in, 12 out). Bound: latency
+// between the fifteen barriers of a tile, at half of the issue slots: on the
+// 64 M entries of the 4M-row Zipf(1.8) matrix 0.75 ms for the tiles, 0.38 for
+// the longer rows (0.23 at the copy rate). Hence small blocks, four of 256
+// threads an SM: two of 512 threads with 4096 entries took 1.03 + 0.26 ms,
+// of which walking one bucket at a time (step 3; four entries' walks now run
+// side by side) 0.13 and copying long rows one load at a time 0.06. It
+// replaces per-class sorting kernels (a segmented bitonic network up to 32 entries, a warp bitonic network up to
 // 512, LSD radix blocks up to 12 288: 145 instructions per entry and radix
 // pass) followed by a compaction pass over all entries.
 #include <algorithm>
@@ -34,16 +41,16 @@
 namespace spg {
 namespace {
 
-constexpr int RT_CAP = 4096;            // entries of a tile
-constexpr int RT_T = 512, RT_PER_SM = 2;
-constexpr int RT_BIG = 12288;           // longest row a block takes
-constexpr int RT_BIG_T = 1024;
+constexpr int RT_CAP = 2048;            // entries of a tile
+constexpr int RT_T = 256, RT_PER_SM = 4;
+constexpr int RT_MID = 4096, RT_MID_T = 512, RT_MID_PER_SM = 2;  // longer rows: blocks for up to RT_MID entries ...
+constexpr int RT_BIG = 12288, RT_BIG_T = 1024;                   // ... and for up to RT_BIG, the longest a block takes
 constexpr int RT_LONG = 64;             // rows above it spread over their own column range
-constexpr int RT_LIM = 32;              // longest bucket ordered by counting (the bitmap search spans two words)
+constexpr int RT_LIM = 32;              // longest bucket ordered by counting
 constexpr unsigned RT_STATUS_TIMEOUT = 0x20u;
 
 // Counters at the head of the scratch words.
-enum : int { RC_PLAN_TICKET = 0, RC_TICKET = 1, RC_TILES = 2, RC_BIG = 3, RC_OVERFLOW = 4, RC_N = 8 };
+enum : int { RC_PLAN_TICKET = 0, RC_TICKET = 1, RC_TILES = 2, RC_BIG = 3, RC_OVERFLOW = 4, RC_MID = 5, RC_MID_TICKET = 6, RC_BIG_TICKET = 7, RC_N = 8 };
 
 struct RtArgs {
     const uint32_t *cols;
@@ -55,7 +62,8 @@ struct RtArgs {
     unsigned long long *ctr;
     unsigned long long *plan_state, *tile_state;
     uint32_t *tile_start;  // first row of each tile, then n_rows
-    uint32_t *big;         // rows of RT_CAP+1 .. RT_BIG entries
+    uint32_t *longer;      // rows of RT_CAP+1 .. RT_MID entries from the front, longer ones from the back
+    uint64_t n_longer;
     uint32_t *big_cols;    // their ordered entries, at the rows' input positions
     double *big_vals;
     uint64_t *off;         // out; off[r] holds a big row's kept count until its tile is written
@@ -110,7 +118,8 @@ __global__ void __launch_bounds__(RP_T) rt_plan(RtArgs a) {
             const uint64_t L = s_off[r + 1] - s_off[r];
             if (lane == 0) {
                 if (L > (uint64_t)RT_BIG) a.ctr[RC_OVERFLOW] = 1ull;
-                else a.big[atomicAdd(a.ctr + RC_BIG, 1ull)] = (uint32_t)(r0 + r);
+                else if (L > (uint64_t)RT_MID) a.longer[a.n_longer - 1 - atomicAdd(a.ctr + RC_BIG, 1ull)] = (uint32_t)(r0 + r);
+                else a.longer[atomicAdd(a.ctr + RC_MID, 1ull)] = (uint32_t)(r0 + r);
             }
             ++e;
         }
@@ -243,7 +252,7 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
                                              const double *__restrict__ vals, int E, int cbits, bool keep_zeros,
                                              uint32_t (&pk)[CAP / T], double (&v)[CAP / T]) {
     constexpr int I = CAP / T, CW = I / 2, P = CAP / 1024;
-    static_assert(CAP % T == 0 && I % 2 == 0 && CAP % 1024 == 0, "whole words per thread");
+    static_assert(CAP % T == 0 && (I % 4 == 0) && CAP % 1024 == 0, "whole words per thread");
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int shift = cbits ? 32 - cbits : 0;  // (cbits == 0: the only column is 0)
     uint16_t *cnt16 = reinterpret_cast<uint16_t *>(S.cnt);
@@ -392,21 +401,48 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
     __syncthreads();
     // place: the bucket's first slot plus the bucket's entries before this one;
     // dropped if the bucket has a later write of its column
+    // (four entries' walks side by side, as a walk alone waits for every load;
+    // but not with the few registers of a thread of RT_BIG_T)
+    constexpr int G = T == RT_BIG_T ? 1 : 4;
 #pragma unroll
-    for (int i = 0; i < I; ++i) {
-        const int e = t + i * T;
-        if (e < E) {
-            const uint32_t lo = pk[i] >> 16, hi = pk[i] & 0xFFFFu;
-            uint32_t f = lo;
-            bool kept = !((dropped >> i) & 1u) && (keep_zeros || !is_zero(v[i]));
-            if (hi - lo > 1) {
-                uint32_t same = 0;
-                for (uint32_t j = lo; j < hi; ++j) {
+    for (int i0 = 0; i0 < I; i0 += G) {
+        uint32_t acc[G], most = 0;  // entries before | entries of the same column << 16
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            if (t + (i0 + g) * T >= E) pk[i0 + g] = 0;
+            const uint32_t len = (pk[i0 + g] & 0xFFFFu) - (pk[i0 + g] >> 16);
+            most = max(most, len);
+            acc[g] = 0;
+        }
+        if (G == 1) {
+            if (most > 1) {
+                for (uint32_t j = pk[i0] >> 16; j < (pk[i0] & 0xFFFFu); ++j) {
                     const uint32_t cj = S.scol[j];
-                    f += cj < c[i] ? 1u : 0u;
-                    same += cj == c[i] ? 1u : 0u;
+                    acc[0] += cj < c[i0] ? 1u : 0u;
+                    acc[0] += cj == c[i0] ? 0x10000u : 0u;
                 }
-                if (same > 1) {
+            }
+        } else if (most > 1) {
+            for (uint32_t j = 0; j < most; ++j) {
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    const uint32_t q = (pk[i0 + g] >> 16) + j;
+                    if (q < (pk[i0 + g] & 0xFFFFu)) {
+                        const uint32_t cj = S.scol[q];
+                        acc[g] += cj < c[i0 + g] ? 1u : 0u;
+                        acc[g] += cj == c[i0 + g] ? 0x10000u : 0u;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const int i = i0 + g, e = t + i * T;
+            if (e < E) {
+                const uint32_t lo = pk[i] >> 16, hi = pk[i] & 0xFFFFu;
+                uint32_t f = lo + (acc[g] & 0xFFFFu);
+                bool kept = !((dropped >> i) & 1u) && (keep_zeros || !is_zero(v[i]));
+                if (acc[g] >= 0x20000u) {
                     for (uint32_t j = lo; j < hi; ++j) {
                         if (S.scol[j] == c[i]) {
                             f += S.spos[j] < e ? 1u : 0u;
@@ -414,9 +450,9 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
                         }
                     }
                 }
+                pk[i] = kept ? f : ~0u;
+                if (kept) atomicOr(&S.keep[f >> 5], 1u << (f & 31));
             }
-            pk[i] = kept ? f : ~0u;
-            if (kept) atomicOr(&S.keep[f >> 5], 1u << (f & 31));
         }
     }
     __syncthreads();
@@ -448,17 +484,23 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
     return __shfl_sync(0xffffffffu, inc, 31);
 }
 
-// Rows longer than a tile, a block each (persistent over the list): ordered
-// and compacted into scratch at the row's input positions.
-__global__ void __launch_bounds__(RT_BIG_T, 1) rt_big_rows(RtArgs a) {
-    constexpr int T = RT_BIG_T, CAP = RT_BIG, I = CAP / T;
+// Rows longer than a tile, a block each (taken from the list one by one):
+// ordered and compacted into scratch at the row's input positions.
+template <int T, int CAP, int PER_SM, int COUNT, int TICKET>
+__global__ void __launch_bounds__(T, PER_SM) rt_long_rows(RtArgs a) {
+    constexpr int I = CAP / T;
+    __shared__ uint64_t s_next;
     extern __shared__ __align__(16) unsigned char rt_raw[];
     auto &S = *reinterpret_cast<RtSmem<T, CAP, false> *>(rt_raw);
     const int t = threadIdx.x;
     if (a.ctr[RC_OVERFLOW]) return;
-    const uint64_t n = a.ctr[RC_BIG];
-    for (uint64_t k = blockIdx.x; k < n; k += gridDim.x) {
-        const uint64_t r = a.big[k], s0 = a.s_off[r];
+    const uint64_t n = a.ctr[COUNT];
+    while (true) {
+        if (t == 0) s_next = atomicAdd(a.ctr + TICKET, 1ull);
+        __syncthreads();
+        const uint64_t k = s_next;
+        if (k >= n) return;
+        const uint64_t r = a.longer[COUNT == RC_BIG ? a.n_longer - 1 - k : k], s0 = a.s_off[r];
         const int E = (int)(a.s_off[r + 1] - s0);
         uint32_t c[I], o[I];
         double v[I];
@@ -503,12 +545,13 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
     const uint64_t n_tiles = a.ctr[RC_TILES];
     if (t == 0) rt_take(S.tile[0], a, n_tiles);
     __syncthreads();
+    uint32_t row_p = 0;  // the place in its tile of row r0 + t of the tile sorted last
     for (unsigned it = 0;; ++it) {
         auto &cur = S.tile[it % 3], &prev = S.tile[(it + 2) % 3];
         const bool have = cur.id < n_tiles;
-        uint32_t c[I], o[I], total = 0;
+        uint32_t c[I], o[I], total = 0, row_b = 0;
         double v[I];
-        int E = -1;  // < 0: a row ordered by rt_big_rows, or no tile
+        int E = -1;  // < 0: a row ordered by rt_long_rows, or no tile
         if (have) {
             const uint64_t r0 = cur.r0, r1 = cur.r1, s0 = cur.s0;
             if (cur.s1 - s0 <= (uint64_t)CAP) {
@@ -518,6 +561,7 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
                 for (int w = t; w < CAP / 32 + 2; w += T) S.head[w] = 0;
                 for (int w = t; w < E / 2 + 1; w += T) S.cnt[w] = 0;
                 __syncthreads();
+                row_b = (uint32_t)(b0 - s0);
                 if (r0 + t < r1 && b0 != e0) rt_mark_row(S, (int)(b0 - s0), (int)(e0 - s0));
                 for (uint64_t r = r0 + t + T; r < r1; r += T) {
                     const uint64_t b = a.s_off[r], e = a.s_off[r + 1];
@@ -541,14 +585,30 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
                     a.out_cols[base + k] = S.col[k];
                     a.out_vals[base + k] = S.val[k];
                 }
-                for (uint64_t r = prev.r0 + t; r < prev.r1; r += T) {
+                if (prev.r0 + t < prev.r1) a.off[prev.r0 + t] = base + row_p;
+                for (uint64_t r = prev.r0 + t + T; r < prev.r1; r += T) {
                     const uint64_t p = a.off[r];  // within the tile: this thread's own
                     a.off[r] = p + base;
                 }
-            } else {  // one row
-                for (uint32_t k = t; k < n; k += T) {
-                    a.out_cols[base + k] = a.big_cols[prev.s0 + k];
-                    a.out_vals[base + k] = a.big_vals[prev.s0 + k];
+            } else {  // one row, eight loads of a thread in flight (one pair at a time: 55 us more on the Zipf matrix)
+                constexpr int U = 4;
+                for (uint32_t k0 = t; k0 < n; k0 += U * T) {
+                    uint32_t cc[U];
+                    double vv[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const uint32_t k = k0 + u * T;
+                        cc[u] = k < n ? a.big_cols[prev.s0 + k] : 0u;
+                        vv[u] = k < n ? a.big_vals[prev.s0 + k] : 0.0;
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const uint32_t k = k0 + u * T;
+                        if (k < n) {
+                            a.out_cols[base + k] = cc[u];
+                            a.out_vals[base + k] = vv[u];
+                        }
+                    }
                 }
                 if (t == 0) a.off[prev.r0] = base;
             }
@@ -567,8 +627,10 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
                 }
             }
             for (uint64_t r = r0 + t; r < r1; r += T) {
-                const uint32_t p = (uint32_t)(a.s_off[r] - s0);
-                a.off[r] = p == (uint32_t)E ? total : S.kpre[p >> 5] + __popc(S.keep[p >> 5] & ((1u << (p & 31)) - 1u));
+                const uint32_t p = r == r0 + t ? row_b : (uint32_t)(a.s_off[r] - s0);
+                const uint32_t q = p == (uint32_t)E ? total : S.kpre[p >> 5] + __popc(S.keep[p >> 5] & ((1u << (p & 31)) - 1u));
+                if (r == r0 + t) row_p = q;
+                else a.off[r] = q;
             }
         }
         __syncthreads();
@@ -584,9 +646,9 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     const uint64_t plan_tiles = (n_rows + RP_ROWS - 1) / RP_ROWS;
     // two neighbouring tiles of one part hold more than RT_CAP entries together
     const uint64_t t_max = 2 * (m / RT_CAP) + 2 * (plan_tiles + m / RP_PART) + 4;
-    const bool may_big = m > (uint64_t)RT_CAP;
-    const uint64_t n_big = m / (RT_CAP + 1) + 1;
-    DevBuf state, tiles, bigs, big_cols, big_vals;
+    const bool may_long = m > (uint64_t)RT_CAP;
+    const uint64_t n_long = m / (RT_CAP + 1) + 1;
+    DevBuf state, tiles, longer, big_cols, big_vals;
     // (the outputs first: the scratch below is a little smaller, and took the
     // freed outputs of an earlier lock when it came first, so that the pool
     // mapped new memory for these at every call: 0.5 ms on the 4M-row matrix)
@@ -596,8 +658,8 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     SPG_TRY(state.alloc((RC_N + plan_tiles + t_max) * sizeof(unsigned long long), s));
     SPG_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, (RC_N + plan_tiles + t_max) * sizeof(unsigned long long), s));
     SPG_TRY(tiles.alloc((t_max + 1) * sizeof(uint32_t), s));
-    SPG_TRY(bigs.alloc(n_big * sizeof(uint32_t), s));
-    if (may_big) {
+    SPG_TRY(longer.alloc(n_long * sizeof(uint32_t), s));
+    if (may_long) {
         SPG_TRY(big_cols.alloc(m * sizeof(uint32_t), s));
         SPG_TRY(big_vals.alloc(m * sizeof(double), s));
     }
@@ -612,7 +674,8 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     a.plan_state = a.ctr + RC_N;
     a.tile_state = a.plan_state + plan_tiles;
     a.tile_start = tiles.as<uint32_t>();
-    a.big = bigs.as<uint32_t>();
+    a.longer = longer.as<uint32_t>();
+    a.n_longer = n_long;
     a.big_cols = big_cols.as<uint32_t>();
     a.big_vals = big_vals.as<double>();
     a.off = out->off.as<uint64_t>();
@@ -622,10 +685,18 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     a.status = c->d_status;
     rt_plan<<<(unsigned)plan_tiles, RP_T, 0, s>>>(a);
     SPG_LAUNCH_CHECK();
-    if (may_big) {
+    if (may_long) {
+        auto k = rt_long_rows<RT_MID_T, RT_MID, RT_MID_PER_SM, RC_MID, RC_MID_TICKET>;
+        constexpr size_t smem = sizeof(RtSmem<RT_MID_T, RT_MID, false>);
+        SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k<<<(unsigned)std::min<uint64_t>(n_long, (uint64_t)c->n_sms * RT_MID_PER_SM), RT_MID_T, smem, s>>>(a);
+        SPG_LAUNCH_CHECK();
+    }
+    if (m > (uint64_t)RT_MID) {
+        auto k = rt_long_rows<RT_BIG_T, RT_BIG, 1, RC_BIG, RC_BIG_TICKET>;
         constexpr size_t smem = sizeof(RtSmem<RT_BIG_T, RT_BIG, false>);
-        SPG_CUDA_TRY(cudaFuncSetAttribute(rt_big_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        rt_big_rows<<<(unsigned)std::min<uint64_t>(n_big, (uint64_t)c->n_sms), RT_BIG_T, smem, s>>>(a);
+        SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k<<<(unsigned)std::min<uint64_t>(m / (RT_MID + 1), (uint64_t)c->n_sms), RT_BIG_T, smem, s>>>(a);
         SPG_LAUNCH_CHECK();
     }
     constexpr size_t smem = sizeof(RtSmem<RT_T, RT_CAP, true>);

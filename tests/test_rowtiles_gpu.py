@@ -37,6 +37,7 @@ LENGTHS = {
     "short": [0, 1, 2, 5, 10, 17, 31, 32, 33] * 700,
     "empty": [3] + [0] * 5000 + [40] + [0] * 2047 + [700] + [0] * 3000,
     "one": [100],
+    "long": [2049, 3, 4096, 4097, 2048] * 170,  # more long rows than blocks
 }
 
 
