@@ -139,13 +139,18 @@ int spg_ctx_create(int device, spg_ctx **out) {
         uint64_t thr = UINT64_MAX;  // keep freed blocks cached in the pool
         e = cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }
-    // Status word in mapped pinned memory: kernels flag timeouts there and the
-    // host reads it after a synchronisation without an extra copy.
-    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void **>(&c->h_status), sizeof(unsigned),
-                                            cudaHostAllocMapped);
+    // Status word and result words in mapped pinned memory: kernels store
+    // there and the host reads after a synchronisation without an extra copy.
+    constexpr size_t WORDS_AT = 64;  // (the status word has its own line)
+    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void **>(&c->h_status),
+                                            WORDS_AT + Ctx::N_WORDS * sizeof(unsigned long long), cudaHostAllocMapped);
     if (e == cudaSuccess) {
         *c->h_status = 0;
         e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&c->d_status), c->h_status, 0);
+    }
+    if (e == cudaSuccess) {
+        c->h_words = reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(c->h_status) + WORDS_AT);
+        c->d_words = reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(c->d_status) + WORDS_AT);
     }
     if (e != cudaSuccess) {
         if (c->stream) cudaStreamDestroy(c->stream);

@@ -40,6 +40,7 @@ struct SdArgs {
     const double *vals;
     uint64_t m;
     const unsigned long long *abort;
+    unsigned long long *words;  // for the host: ctr[0], ctr[1], entries gained (signed)
     unsigned long long *ctr;   // [0] distinct keys, [1] 1: a row has more than SD_RUN inserts
     uint64_t *place;           // by sorted position, as the next four
     int64_t *P;                // contributions, then their exclusive scan (m + 1)
@@ -118,6 +119,11 @@ __device__ __forceinline__ uint64_t sd_lower(const T *__restrict__ x, uint64_t l
 }
 
 __global__ void __launch_bounds__(SD_T) sd_chunks(SdArgs a) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // final since the probe and the scan
+        store_word(a.words, 0, a.ctr[0]);
+        store_word(a.words, 1, a.ctr[1]);
+        store_word(a.words, 2, (unsigned long long)a.P[a.m]);
+    }
     if (sd_off(a)) return;
     const uint64_t k = blockIdx.x * (uint64_t)SD_T + threadIdx.x;
     if (k <= a.n_chunks) a.chunk[k] = sd_lower(a.place, 0, a.m, k * SD_CHUNK);
@@ -243,6 +249,7 @@ int merge_small_delta(Ctx *c, const CsrView &A, uint64_t n_rows, const uint32_t 
     a.vals = vals;
     a.m = m;
     a.abort = abort;
+    a.words = c->d_words;
     a.off = off_out;
     a.out_cols = cols_out;
     a.out_vals = vals_out;
@@ -255,14 +262,10 @@ int merge_small_delta(Ctx *c, const CsrView &A, uint64_t n_rows, const uint32_t 
     SPG_LAUNCH_CHECK();
     sd_merge<<<(unsigned)(a.n_chunks + a.n_rchunks + gm), SD_T, 0, s>>>(a);
     SPG_LAUNCH_CHECK();
-    uint64_t h[2] = {0, 1};
-    int64_t total = 0;
-    SPG_CUDA_TRY(cudaMemcpyAsync(h, a.ctr, 16, cudaMemcpyDeviceToHost, s));
-    SPG_CUDA_TRY(cudaMemcpyAsync(&total, a.P + m, 8, cudaMemcpyDeviceToHost, s));
     SPG_TRY(c->phase_sync(s));
-    *u = h[0];
-    *nnz = (uint64_t)((int64_t)A.nnz + total);
-    *done = h[1] == 0;
+    *u = c->word(0);
+    *nnz = (uint64_t)((int64_t)A.nnz + (int64_t)c->word(2));
+    *done = c->word(1) == 0;
     return SPG_OK;
 }
 

@@ -79,7 +79,8 @@ __device__ __forceinline__ bool offsets_step(uint64_t *__restrict__ off, uint64_
 // fourth insert, by 24 lanes of each warp's 32 (3 / 16 of all).
 template <bool VEC>
 __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, uint64_t m,
-                             int cbits, uint64_t n_rows, uint64_t *__restrict__ off, unsigned *__restrict__ stats) {
+                             int cbits, uint64_t n_rows, uint64_t *__restrict__ off, unsigned *__restrict__ stats,
+                             unsigned long long *__restrict__ words) {
     unsigned mr = 0, mc = 0, hits = 0;
     bool d = false, g = false, e = false, gap = false;
     if (off && blockIdx.x == 0 && threadIdx.x == 0) {  // the rows up to the first insert's and after the last one's
@@ -174,6 +175,9 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
         if (bf & 2u) stats[3] = 1u;
         if (bf & 4u) stats[4] = 1u;
         if (bf & 8u) stats[6] = 1u;
+        if (last_block(stats + 7)) {
+            for (int i = 0; i < 7; ++i) store_word(words, i, *(volatile unsigned *)(stats + i));
+        }
     }
 }
 
@@ -811,19 +815,21 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
     Prepared pre;
     if (m) {
         DevBuf stats;
-        SPG_TRY(stats.alloc(7 * sizeof(unsigned), s));
-        SPG_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, 7 * sizeof(unsigned), s));
+        SPG_TRY(stats.alloc(8 * sizeof(unsigned), s));
+        SPG_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, 8 * sizeof(unsigned), s));
         if (!A->built) SPG_TRY(pre.off.alloc(csr_off_elems(A->n_rows) * sizeof(uint64_t), s));
         if (((uintptr_t)rows | (uintptr_t)cols) % 16 == 0)
             lock_prepare<true><<<grid_for((m + 3) / 4, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
-                rows, cols, m, bits_for(A->n_cols), A->n_rows, pre.off.as<uint64_t>(), stats.as<unsigned>());
+                rows, cols, m, bits_for(A->n_cols), A->n_rows, pre.off.as<uint64_t>(), stats.as<unsigned>(),
+                c->d_words);
         else
             lock_prepare<false><<<grid_for(m, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
-                rows, cols, m, bits_for(A->n_cols), A->n_rows, pre.off.as<uint64_t>(), stats.as<unsigned>());
+                rows, cols, m, bits_for(A->n_cols), A->n_rows, pre.off.as<uint64_t>(), stats.as<unsigned>(),
+                c->d_words);
         SPG_LAUNCH_CHECK();
-        unsigned h[7] = {0u, 0u, 1u, 1u, 1u, 0u, 1u};
-        SPG_CUDA_TRY(cudaMemcpyAsync(h, stats.ptr, 7 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         SPG_TRY(c->phase_sync(s));
+        unsigned h[7];
+        for (int i = 0; i < 7; ++i) h[i] = (unsigned)c->word(i);
         if ((uint64_t)h[0] >= A->n_rows)
             return set_error(SPG_ERR_OUT_OF_RANGE, "spira::matrix: row_index out of range (%u >= %llu)", h[0],
                              (unsigned long long)A->n_rows);

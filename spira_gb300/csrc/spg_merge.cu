@@ -52,6 +52,7 @@ struct MtArgs {
     uint32_t *cols;
     double *vals;
     unsigned int *status;
+    unsigned long long *words;  // [0] entries kept
 };
 
 // Cut t: the row holding item t MT_TILE, and how many of A's and B's entries
@@ -289,7 +290,10 @@ __global__ void __launch_bounds__(MT_T, MT_PER_SM) mt_tiles(MtArgs a) {
                 const uint64_t p = a.off[r];  // within the tile: this thread's own
                 a.off[r] = p + base;
             }
-            if (t == 0 && prev.id + 1 == a.n_tiles) a.off[a.n_rows] = base + prev.total;
+            if (t == 0 && prev.id + 1 == a.n_tiles) {
+                a.off[a.n_rows] = base + prev.total;
+                store_word(a.words, 0, base + prev.total);
+            }
         }
         if (!have) return;
         if (t == 32) mt_take(S.tile[(it + 1) % 3], a);
@@ -335,14 +339,16 @@ int merge_csr(Ctx *c, const CsrView &A, const CsrView &B, uint64_t n_rows, Merge
     a.cols = cols_out;
     a.vals = vals_out;
     a.status = c->d_status;
+    a.words = c->d_words;
     mt_splits<<<(unsigned)((tiles + 1 + 7) / 8), 256, 0, s>>>(a, split.as<MtSplit>());
     SPG_LAUNCH_CHECK();
     auto k = mode == MergeMode::Sum ? mt_tiles<MergeMode::Sum> : mt_tiles<MergeMode::Replace>;
     SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MtSmem)));
     k<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)c->n_sms * MT_PER_SM), MT_T, sizeof(MtSmem), s>>>(a);
     SPG_LAUNCH_CHECK();
-    SPG_CUDA_TRY(cudaMemcpyAsync(nnz, off_out + n_rows, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-    return c->phase_sync(s);
+    SPG_TRY(c->phase_sync(s));
+    *nnz = c->word(0);
+    return SPG_OK;
 }
 
 }  // namespace spg

@@ -71,6 +71,7 @@ struct RtArgs {
     double *out_vals;
     const unsigned long long *abort;  // may be null: the inputs are not to be read if set
     unsigned int *status;
+    unsigned long long *words;  // [0] 1: a row is too long, nothing is built; [1] entries kept
 };
 
 // ---------------------------------------------------------------- tile plan
@@ -541,7 +542,10 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
     extern __shared__ __align__(16) unsigned char rt_raw[];
     auto &S = *reinterpret_cast<RtSmem<T, CAP, true> *>(rt_raw);
     const int t = threadIdx.x;
-    if (a.ctr[RC_OVERFLOW]) return;
+    if (a.ctr[RC_OVERFLOW]) {
+        if (blockIdx.x == 0 && t == 0) store_word(a.words, 0, 1ull);
+        return;
+    }
     const uint64_t n_tiles = a.ctr[RC_TILES];
     if (t == 0) rt_take(S.tile[0], a, n_tiles);
     __syncthreads();
@@ -612,7 +616,11 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
                 }
                 if (t == 0) a.off[prev.r0] = base;
             }
-            if (t == 0 && prev.r1 == a.n_rows) a.off[a.n_rows] = base + n;
+            if (t == 0 && prev.r1 == a.n_rows) {
+                a.off[a.n_rows] = base + n;
+                store_word(a.words, 0, 0ull);
+                store_word(a.words, 1, base + n);
+            }
         }
         if (!have) return;
         if (t == 32) rt_take(S.tile[(it + 1) % 3], a, n_tiles);
@@ -683,6 +691,7 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     a.out_vals = out->vals.as<double>();
     a.abort = abort;
     a.status = c->d_status;
+    a.words = c->d_words;
     rt_plan<<<(unsigned)plan_tiles, RP_T, 0, s>>>(a);
     SPG_LAUNCH_CHECK();
     if (may_long) {
@@ -704,11 +713,9 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     const unsigned blocks = (unsigned)std::min<uint64_t>(t_max, (uint64_t)c->n_sms * RT_PER_SM);
     rt_tiles<<<blocks, RT_T, smem, s>>>(a);
     SPG_LAUNCH_CHECK();
-    unsigned long long h_over = 1;
-    SPG_CUDA_TRY(cudaMemcpyAsync(&h_over, a.ctr + RC_OVERFLOW, 8, cudaMemcpyDeviceToHost, s));
-    SPG_CUDA_TRY(cudaMemcpyAsync(&out->n, a.off + n_rows, 8, cudaMemcpyDeviceToHost, s));
     SPG_TRY(c->phase_sync(s));
-    *done = h_over == 0;
+    *done = c->word(0) == 0;
+    out->n = *done ? c->word(1) : 0;
     return SPG_OK;
 }
 

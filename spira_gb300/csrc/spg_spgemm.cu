@@ -45,11 +45,12 @@ namespace {
 constexpr int GB = 256;
 
 // Products per row of A (thread per row); entry m is 0. ctr[0] += all of them,
-// ctr[1] += the rows of more than SPGEMM_HASH_MAX.
+// ctr[1] += the rows of more than SPGEMM_HASH_MAX; the host gets both in
+// words[0 .. 1].
 __global__ void __launch_bounds__(GB)
 sg_row_products(const uint64_t *__restrict__ aoff, const uint32_t *__restrict__ acols,
                 const uint64_t *__restrict__ boff, uint64_t m, uint64_t *__restrict__ cnt,
-                unsigned long long *__restrict__ ctr) {
+                unsigned long long *__restrict__ ctr, unsigned long long *__restrict__ words) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     unsigned long long s = 0;
     if (i < m)
@@ -77,6 +78,10 @@ sg_row_products(const uint64_t *__restrict__ aoff, const uint32_t *__restrict__ 
         }
         if (sum) atomicAdd(ctr, sum);
         if (over) atomicAdd(ctr + 1, over);
+        if (last_block(ctr + 2)) {
+            store_word(words, 0, *(volatile unsigned long long *)ctr);
+            store_word(words, 1, *(volatile unsigned long long *)(ctr + 1));
+        }
     }
 }
 
@@ -446,17 +451,15 @@ int spgemm_products(Ctx *c, const Csr *A, const Csr *B, DevBuf *pofs, uint64_t *
                     cudaStream_t s) {
     const uint64_t m = A->n_rows;
     DevBuf ctr;
-    SPG_TRY(ctr.alloc(2 * sizeof(unsigned long long), s));
-    SPG_CUDA_TRY(cudaMemsetAsync(ctr.ptr, 0, 2 * sizeof(unsigned long long), s));
+    SPG_TRY(ctr.alloc(3 * sizeof(unsigned long long), s));
+    SPG_CUDA_TRY(cudaMemsetAsync(ctr.ptr, 0, 3 * sizeof(unsigned long long), s));
     SPG_TRY(pofs->alloc((m + 1) * sizeof(uint64_t), s));
     sg_row_products<<<grid_for(m + 1, GB), GB, 0, s>>>(A->d_off(), A->d_cols(), B->d_off(), m, pofs->as<uint64_t>(),
-                                                       ctr.as<unsigned long long>());
+                                                       ctr.as<unsigned long long>(), c->d_words);
     SPG_LAUNCH_CHECK();
-    unsigned long long h[2] = {0, 0};
-    SPG_CUDA_TRY(cudaMemcpyAsync(h, ctr.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
     SPG_TRY(c->phase_sync(s));
-    *P = h[0];
-    *long_rows = h[1];
+    *P = c->word(0);
+    *long_rows = c->word(1);
     if (*P >= (1ull << 32))
         return set_error(SPG_ERR_UNSUPPORTED, "spgemm: %llu products exceed 2^32-1", (unsigned long long)*P);
     return SPG_OK;

@@ -44,6 +44,7 @@ struct ShArgs {
     uint32_t *ccols;
     double *cvals;
     unsigned int *status;
+    unsigned long long *words;  // [0] entries of C
 };
 
 struct ShSmem {
@@ -253,7 +254,10 @@ __global__ void __launch_bounds__(SH_T, 8) sh_tiles(ShArgs a) {
     uint64_t base = 0;
     if (!block_lookback<SH_T>(S.lb, a.state, tile, total, base, a.status, SH_STATUS_TIMEOUT)) return;
     if (t < SH_ROWS && row0 + t < a.m) a.coff[row0 + t] = base + before;
-    if (t == 0 && tile + 1 == a.n_tiles) a.coff[a.m] = base + total;
+    if (t == 0 && tile + 1 == a.n_tiles) {
+        a.coff[a.m] = base + total;
+        store_word(a.words, 0, base + total);
+    }
     for (int j = warp; j < SH_ROWS; j += SH_T / 32) {
         const uint32_t n = __shfl_sync(0xffffffffu, cnt, j), o = __shfl_sync(0xffffffffu, before, j);
         for (uint32_t q = lane; q < n; q += 32) {
@@ -279,7 +283,7 @@ int spgemm_hash_rows(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, uint64_t P, cu
     SPG_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, (1 + tiles) * sizeof(unsigned long long), s));
     unsigned long long *ticket = state.as<unsigned long long>();
     ShArgs a{A->d_off(), A->d_cols(), A->d_vals(), B->d_off(), B->d_cols(), B->d_vals(), m, tiles, ticket, ticket + 1,
-             off.as<uint64_t>(), cols.as<uint32_t>(), vals.as<double>(), c->d_status};
+             off.as<uint64_t>(), cols.as<uint32_t>(), vals.as<double>(), c->d_status, c->d_words};
     // 32-bit indices and sort keys (column, six slot bits) where they fit
     const bool i32 = B->nnz <= 0xFFFFFFFFull, k32 = n <= (1ull << 26);
     auto k = i32 ? (k32 ? sh_tiles<uint32_t, uint32_t> : sh_tiles<uint32_t, unsigned long long>)
@@ -287,9 +291,8 @@ int spgemm_hash_rows(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, uint64_t P, cu
     SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ShSmem)));
     k<<<(unsigned)tiles, SH_T, sizeof(ShSmem), s>>>(a);
     SPG_LAUNCH_CHECK();
-    int rc = SPG_OK;
-    const uint64_t nnz = read_u64(c, off.as<uint64_t>() + m, s, &rc);
-    SPG_TRY(rc);
+    SPG_TRY(c->phase_sync(s));
+    const uint64_t nnz = c->word(0);
     spgemm_install(Cm, m, n, std::move(off), std::move(cols), std::move(vals), nnz);
     return SPG_OK;
 }

@@ -69,6 +69,7 @@ struct SgsArgs {
     uint32_t *ccols;
     double *cvals;
     unsigned int *status;
+    unsigned long long *words;   // [0] entries of C
     uint32_t tpb;                // product budget of a tile (shared memory)
     long long wait_cycles;       // bound of every look-back wait
     uint64_t fixed_rows;         // nonzero: no heavy rows; tile t = rows [t F, t F + F), pofs = raw counts
@@ -79,14 +80,14 @@ __device__ __forceinline__ bool sgs_heavy(const uint64_t *aoff, const uint64_t *
 }
 
 // Products per row (pofs[i]) and the products of heavy rows only (hp[i], 0
-// for the others); entry m of both is 0; *n_heavy counts heavy rows and
-// *p_total sums the products (one atomic per block each).
+// for the others); entry m of both is 0; ctr[0] counts heavy rows and ctr[1]
+// sums the products (one atomic per block each), for the host in words[0 .. 1].
 __global__ void __launch_bounds__(256) sgs_products(const uint64_t *__restrict__ aoff,
                                                     const uint32_t *__restrict__ acols,
                                                     const uint64_t *__restrict__ boff, uint64_t m, uint32_t hb,
                                                     uint64_t *__restrict__ pofs, uint64_t *__restrict__ hp,
-                                                    unsigned long long *__restrict__ n_heavy,
-                                                    unsigned long long *__restrict__ p_total) {
+                                                    unsigned long long *__restrict__ ctr,
+                                                    unsigned long long *__restrict__ words) {
     __shared__ unsigned long long s_p[8], s_h[8];
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     uint64_t p = 0;
@@ -122,8 +123,12 @@ __global__ void __launch_bounds__(256) sgs_products(const uint64_t *__restrict__
             bp += s_p[w];
             bh += s_h[w];
         }
-        if (bp) atomicAdd(p_total, bp);
-        if (bh) atomicAdd(n_heavy, bh);
+        if (bp) atomicAdd(ctr + 1, bp);
+        if (bh) atomicAdd(ctr, bh);
+        if (last_block(ctr + 2)) {
+            store_word(words, 0, *(volatile unsigned long long *)ctr);
+            store_word(words, 1, *(volatile unsigned long long *)(ctr + 1));
+        }
     }
 }
 
@@ -479,7 +484,10 @@ __global__ void __launch_bounds__(SGS_THREADS) sgs_tiles(SgsArgs g) {
     if (!sh_ok) return;
     const uint64_t base = sh_base;
     if ((uint32_t)tid < nr) g.coff[row0 + tid] = base + excl;
-    if (tid == 0 && row1 == g.m) g.coff[g.m] = base + total;
+    if (tid == 0 && row1 == g.m) {
+        g.coff[g.m] = base + total;
+        store_word(g.words, 0, base + total);
+    }
     if (!heavy_tile) {
         // a warp per row, lanes over its kept entries (no search for the row)
         for (uint32_t j = warp; j < nr; j += SGS_WARPS) {
@@ -551,11 +559,12 @@ int spgemm_warpsort(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, int variant, cu
     SPG_CUDA_TRY(cudaMemsetAsync(nh_dev.ptr, 0, 3 * sizeof(uint64_t), s));
     unsigned long long *nh = reinterpret_cast<unsigned long long *>(nh_dev.as<uint64_t>());
     sgs_products<<<grid_for(m + 1, 256), 256, 0, s>>>(A->d_off(), A->d_cols(), B->d_off(), m, cf.hb,
-                                                     pofs.as<uint64_t>(), hp.as<uint64_t>(), nh, nh + 1);
+                                                     pofs.as<uint64_t>(), hp.as<uint64_t>(), nh, c->d_words);
     SPG_LAUNCH_CHECK();
     uint64_t h[3] = {0, 0, 0};  // heavy rows, products, heavy products
-    SPG_CUDA_TRY(cudaMemcpyAsync(h, nh_dev.ptr, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     SPG_TRY(c->phase_sync(s));
+    h[0] = c->word(0);
+    h[1] = c->word(1);
     // No heavy row: tiles of F consecutive rows (F rows of at most hb products fill a tile's budget
     // at most), their regions scanned inside the kernel: no scan, no tile plan.
     const uint64_t F = h[0] ? 0 : cf.tpb / cf.hb;
@@ -637,6 +646,7 @@ int spgemm_warpsort(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, int variant, cu
     g.ccols = cols.as<uint32_t>();
     g.cvals = vals.as<double>();
     g.status = c->d_status;
+    g.words = c->d_words;
     g.tpb = cf.tpb;
     g.wait_cycles = SGS_WAIT_CYCLES;
     g.fixed_rows = F;
@@ -650,9 +660,8 @@ int spgemm_warpsort(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, int variant, cu
         lrc = k32 ? launch_tiles<128, uint32_t>(g, grid, smem, s) : launch_tiles<128, uint64_t>(g, grid, smem, s);
     else lrc = k32 ? launch_tiles<256, uint32_t>(g, grid, smem, s) : launch_tiles<256, uint64_t>(g, grid, smem, s);
     SPG_TRY(lrc);
-    const uint64_t nnz = read_u64(c, off.as<uint64_t>() + m, s, &rc);
-    SPG_TRY(rc);
-    SPG_TRY(c->take_status());
+    SPG_TRY(c->phase_sync(s));
+    const uint64_t nnz = c->word(0);
     spgemm_install(Cm, m, n, std::move(off), std::move(cols), std::move(vals), nnz);
     return SPG_OK;
 }

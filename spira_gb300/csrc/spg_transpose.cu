@@ -183,7 +183,8 @@ __global__ void __launch_bounds__(TB)
 tr_sort_mid(const uint64_t *__restrict__ toff, const uint32_t *__restrict__ mid,
             const unsigned long long *__restrict__ n_mid, const uint32_t *__restrict__ tsrc,
             const double *__restrict__ tval, uint32_t *__restrict__ out_cols, double *__restrict__ out_vals,
-            const unsigned long long *__restrict__ longest) {
+            const unsigned long long *__restrict__ longest, unsigned long long *__restrict__ words) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) store_word(words, 0, *longest);
     if (*longest > NET_MAX) return;
     const unsigned lane = threadIdx.x & 31;
     const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -259,10 +260,10 @@ int transpose_impl(Ctx *c, const Csr *A, Csr *T, cudaStream_t s) {
                                                                mx);
             tr_sort_mid<<<(unsigned)c->n_sms * 8, TB, 0, s>>>(out_off.as<uint64_t>(), midbuf.as<uint32_t>(), n_mid,
                                                              tsrc.as<uint32_t>(), tval.as<double>(),
-                                                             out_cols.as<uint32_t>(), out_vals.as<double>(), mx);
+                                                             out_cols.as<uint32_t>(), out_vals.as<double>(), mx, c->d_words);
             SPG_LAUNCH_CHECK();
-            SPG_CUDA_TRY(cudaMemcpyAsync(&longest, mx, 8, cudaMemcpyDeviceToHost, s));
             SPG_TRY(c->phase_sync(s));
+            longest = c->word(0);
         }
         if (longest > NET_MAX) {
             // (column, source row, value) sorted stably by column: the rows of a
