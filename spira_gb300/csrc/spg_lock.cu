@@ -224,7 +224,7 @@ __global__ void first_grouped_compact(const uint32_t *__restrict__ rows, const u
 // caller takes the general path).
 __global__ void first_direct_copy(const uint32_t *__restrict__ cols, const double *__restrict__ vals, uint64_t m,
                                   uint32_t *__restrict__ out_cols, double *__restrict__ out_vals,
-                                  unsigned *__restrict__ zero) {
+                                  unsigned *__restrict__ zero, unsigned long long *__restrict__ words) {
     bool z = false;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
          i += (uint64_t)gridDim.x * blockDim.x) {
@@ -233,7 +233,11 @@ __global__ void first_direct_copy(const uint32_t *__restrict__ cols, const doubl
         out_cols[i] = cols[i];
         out_vals[i] = v;
     }
-    if (__any_sync(0xffffffffu, z) && (threadIdx.x & 31) == 0) *zero = 1u;
+    const bool any = __syncthreads_or(z);
+    if (threadIdx.x == 0) {
+        if (any) zero[0] = 1u;
+        if (last_block(zero + 1)) store_word(words, 0, *(volatile unsigned *)zero);
+    }
 }
 
 // flag[i] = 1 iff sorted key i is the last of its run (the last write).
@@ -514,22 +518,23 @@ constexpr uint64_t FEW_STAGED = 4u << 20;
 // Prepared::long_hits of rows sorted since lock_prepare, from 2^16 places.
 constexpr uint64_t LONG_SAMPLES = 1u << 16;
 
-__global__ void long_rows_sample(const uint32_t *__restrict__ rows, uint64_t m, unsigned *__restrict__ hits) {
+__global__ void long_rows_sample(const uint32_t *__restrict__ rows, uint64_t m, unsigned *__restrict__ hits,
+                                 unsigned long long *__restrict__ words) {
     const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, i = k * (m - 32) / LONG_SAMPLES;
     const unsigned n = __popc(__ballot_sync(0xffffffffu, rows[i] == rows[i + 32]));
     if ((threadIdx.x & 31) == 0 && n) atomicAdd(hits, n);
+    __syncthreads();
+    if (threadIdx.x == 0 && last_block(hits + 1)) store_word(words, 0, *(volatile unsigned *)hits);
 }
 
 int sample_long_rows(Ctx *c, const uint32_t *rows, uint64_t m, uint64_t *long_hits, cudaStream_t s) {
     DevBuf hits;
-    SPG_TRY(hits.alloc(sizeof(unsigned), s));
-    SPG_CUDA_TRY(cudaMemsetAsync(hits.ptr, 0, sizeof(unsigned), s));
-    long_rows_sample<<<LONG_SAMPLES / LB, LB, 0, s>>>(rows, m, hits.as<unsigned>());
+    SPG_TRY(hits.alloc(2 * sizeof(unsigned), s));
+    SPG_CUDA_TRY(cudaMemsetAsync(hits.ptr, 0, 2 * sizeof(unsigned), s));
+    long_rows_sample<<<LONG_SAMPLES / LB, LB, 0, s>>>(rows, m, hits.as<unsigned>(), c->d_words);
     SPG_LAUNCH_CHECK();
-    unsigned h = 0;
-    SPG_CUDA_TRY(cudaMemcpyAsync(&h, hits.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     SPG_TRY(c->phase_sync(s));
-    *long_hits = (uint64_t)((double)h / LONG_SAMPLES * 3.0 / 16.0 * (double)m);
+    *long_hits = (uint64_t)((double)c->word(0) / LONG_SAMPLES * 3.0 / 16.0 * (double)m);
     return SPG_OK;
 }
 
@@ -611,19 +616,17 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
         // unless a value is zero, the staged arrays are the CSR
         const unsigned g = grid_for(m, LB, (unsigned)c->n_sms * 16);
         DevBuf zero;
-        SPG_TRY(zero.alloc(sizeof(unsigned), s));
-        SPG_CUDA_TRY(cudaMemsetAsync(zero.ptr, 0, sizeof(unsigned), s));
+        SPG_TRY(zero.alloc(2 * sizeof(unsigned), s));
+        SPG_CUDA_TRY(cudaMemsetAsync(zero.ptr, 0, 2 * sizeof(unsigned), s));
         SPG_TRY(out_cols.alloc(csr_alloc_elems(m) * sizeof(uint32_t), s));
         SPG_TRY(out_vals.alloc(csr_alloc_elems(m) * sizeof(double), s));
         first_direct_copy<<<g, LB, 0, s>>>(cols, vals, m, out_cols.as<uint32_t>(), out_vals.as<double>(),
-                                           zero.as<unsigned>());
+                                           zero.as<unsigned>(), c->d_words);
         SPG_LAUNCH_CHECK();
         // the offsets go out before the zero check comes back: one host sync
         SPG_TRY(staged_offsets(c, pre, rows, m, n, new_off, s));
-        unsigned hz = 1;
-        SPG_CUDA_TRY(cudaMemcpyAsync(&hz, zero.ptr, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         SPG_TRY(c->phase_sync(s));
-        if (!hz) {
+        if (c->word(0) == 0) {
             A->invalidate_derived();
             A->off = std::move(new_off);
             A->cols = std::move(out_cols);
@@ -670,11 +673,8 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
             SPG_TRY(scols.alloc(csr_alloc_elems(m) * sizeof(uint32_t), s));
             SPG_TRY(svals.alloc(csr_alloc_elems(m) * sizeof(double), s));
             SPG_TRY(dedup_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, cbits, scols.as<uint32_t>(),
-                                       svals.as<double>(), kept.as<uint64_t>(), &done, s));
+                                       svals.as<double>(), kept.as<uint64_t>(), &nnz, &done, s));
             if (done) {
-                SPG_TRY(exclusive_scan_u64(c, kept.as<uint64_t>(), n, kept.as<uint64_t>() + n, s));
-                SPG_CUDA_TRY(cudaMemcpyAsync(&nnz, kept.as<uint64_t>() + n, 8, cudaMemcpyDeviceToHost, s));
-                SPG_TRY(c->phase_sync(s));
                 if (nnz == m) {  // nothing dropped: the staging arrays are the CSR
                     out_cols = std::move(scols);
                     out_vals = std::move(svals);

@@ -968,7 +968,7 @@ int launch_tile_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, const 
 }
 
 int seg_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, uint64_t m, uint64_t n_rows, int cbits,
-             const SegOut &o, bool *done, cudaStream_t s) {
+             const SegOut &o, uint64_t *nnz, bool *done, cudaStream_t s) {
     *done = false;
     if (cbits > SEG_MAX_CBITS || m > 0xFFFFFFFFull) return SPG_OK;
     DevBuf ctr_b, lists_b;
@@ -995,29 +995,33 @@ int seg_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, uint64_t m, ui
                                                    s)));
     SPG_TRY((launch_tile_sort<TS2_T, TS2_I>(c, cols, s_off, lists, ctr, 2, m / (TS1 + 1) + 1, cbits, o, ovf,
                                                    s)));
-    unsigned h = 1u;
-    SPG_CUDA_TRY(cudaMemcpyAsync(&h, ovf, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    // the offsets go out before the flag comes back: one host sync
+    SPG_TRY(exclusive_scan_u64(c, o.kept, n_rows, o.kept + n_rows, s));
+    SPG_CUDA_TRY(cudaMemcpyAsync(c->h_words, ovf, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    SPG_CUDA_TRY(cudaMemcpyAsync(c->h_words + 1, o.kept + n_rows, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     SPG_TRY(c->phase_sync(s));
-    *done = h == 0;
+    *done = (unsigned)c->word(0) == 0;
+    *nnz = c->word(1);
     return SPG_OK;
 }
 
 }  // namespace
 
 int dedup_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off, uint64_t m,
-                       uint64_t n_rows, int cbits, uint32_t *out_cols, double *out_vals, uint64_t *kept, bool *done,
-                       cudaStream_t s) {
+                       uint64_t n_rows, int cbits, uint32_t *out_cols, double *out_vals, uint64_t *off, uint64_t *nnz,
+                       bool *done, cudaStream_t s) {
     SegOut o{};
     o.in_vals = vals;
     o.cols = out_cols;
     o.vals = out_vals;
-    o.kept = kept;
+    o.kept = off;
     if (m == 0) {
-        SPG_CUDA_TRY(cudaMemsetAsync(kept, 0, n_rows * sizeof(uint64_t), s));
+        SPG_CUDA_TRY(cudaMemsetAsync(off, 0, (n_rows + 1) * sizeof(uint64_t), s));
+        *nnz = 0;
         *done = true;
         return SPG_OK;
     }
-    return seg_sort(c, cols, s_off, m, n_rows, cbits, o, done, s);
+    return seg_sort(c, cols, s_off, m, n_rows, cbits, o, nnz, done, s);
 }
 
 }  // namespace spg
