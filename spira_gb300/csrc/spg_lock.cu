@@ -72,16 +72,22 @@ __device__ __forceinline__ bool offsets_step(uint64_t *__restrict__ off, uint64_
     return false;
 }
 
+__device__ __forceinline__ uint32_t column_gap(uint32_t a, uint32_t b) { return a < b ? b - a : a - b; }
+
 // VEC: rows and cols 16-byte aligned; each thread reads 4 rows and 4
 // columns per step in two 16-byte loads (the successor of its last pair
 // comes from the next lane, or one more load at the warp's edge).
 // stats[5] += a sample of the inserts that 32 others of their row follow: every
-// fourth insert, by 24 lanes of each warp's 32 (3 / 16 of all).
+// fourth insert, by 24 lanes of each warp's 32 (3 / 16 of all). stats[7] += a
+// sample of the inserts whose successor in the row is nearer than `near`
+// columns, less those whose successor is not: every fourth insert.
 template <bool VEC>
 __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, uint64_t m,
-                             int cbits, uint64_t n_rows, uint64_t *__restrict__ off, unsigned *__restrict__ stats,
+                             int cbits, uint64_t n_rows, uint32_t near, uint64_t *__restrict__ off,
+                             unsigned *__restrict__ stats,
                              unsigned long long *__restrict__ words) {
     unsigned mr = 0, mc = 0, hits = 0;
+    int score = 0;
     bool d = false, g = false, e = false, gap = false;
     if (off && blockIdx.x == 0 && threadIdx.x == 0) {  // the rows up to the first insert's and after the last one's
         gap |= offsets_step(off, 0, rows[0], n_rows, 0);
@@ -107,6 +113,7 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
                 rn = rows[4 * q + 4];
                 cn = cols[4 * q + 4];
             }
+            if (ok && r4.x == r4.y) score += column_gap(c4.x, c4.y) < near ? 1 : -1;
             if (ok) {
                 const uint32_t rr[5] = {r4.x, r4.y, r4.z, r4.w, rn}, cc[5] = {c4.x, c4.y, c4.z, c4.w, cn};
 #pragma unroll
@@ -133,8 +140,9 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
         mc = max(mc, c);
         if (!VEC && (i & 3) == 0 && ((i >> 2) & 31) < 24 && i + 32 < m) hits += rows[i + 32] == r ? 1u : 0u;
         if (i + 1 < m) {
-            const uint32_t r2 = rows[i + 1];
-            const uint64_t k = ((uint64_t)r << cbits) | c, k2 = ((uint64_t)r2 << cbits) | cols[i + 1];
+            const uint32_t r2 = rows[i + 1], c2 = cols[i + 1];
+            const uint64_t k = ((uint64_t)r << cbits) | c, k2 = ((uint64_t)r2 << cbits) | c2;
+            if (!VEC && (i & 3) == 0 && r == r2) score += column_gap(c, c2) < near ? 1 : -1;
             d |= k > k2;
             e |= k >= k2;
             g |= r > r2;
@@ -147,36 +155,42 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
         mc = max(mc, __shfl_xor_sync(0xffffffffu, mc, o));
     }
     hits = __reduce_add_sync(0xffffffffu, hits);
+    score = __reduce_add_sync(0xffffffffu, score);
     const unsigned flags = (__any_sync(0xffffffffu, d) ? 1u : 0u) | (__any_sync(0xffffffffu, g) ? 2u : 0u) |
                            (__any_sync(0xffffffffu, e) ? 4u : 0u) | (__any_sync(0xffffffffu, gap) ? 8u : 0u);
     // one set of atomics per block: per-warp atomics on the same two words
     // serialise at L2 and cost more than the pass itself
     __shared__ unsigned s_mr[LB / 32], s_mc[LB / 32], s_fl[LB / 32], s_hits[LB / 32];
+    __shared__ int s_score[LB / 32];
     const int w = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) {
         s_mr[w] = mr;
         s_mc[w] = mc;
         s_fl[w] = flags;
         s_hits[w] = hits;
+        s_score[w] = score;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned bm = 0, bc = 0, bf = 0, bh = 0;
+        int bs = 0;
         for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
             bm = max(bm, s_mr[i]);
             bc = max(bc, s_mc[i]);
             bf |= s_fl[i];
             bh += s_hits[i];
+            bs += s_score[i];
         }
         atomicMax(stats, bm);
         atomicMax(stats + 1, bc);
         if (bh) atomicAdd(stats + 5, bh);
+        if (bs) atomicAdd(reinterpret_cast<int *>(stats) + 7, bs);
         if (bf & 1u) stats[2] = 1u;
         if (bf & 2u) stats[3] = 1u;
         if (bf & 4u) stats[4] = 1u;
         if (bf & 8u) stats[6] = 1u;
-        if (last_block(stats + 7)) {
-            for (int i = 0; i < 7; ++i) store_word(words, i, *(volatile unsigned *)(stats + i));
+        if (last_block(stats + 8)) {
+            for (int i = 0; i < 8; ++i) store_word(words, i, *(volatile unsigned *)(stats + i));
         }
     }
 }
@@ -498,6 +512,7 @@ struct Prepared {
     unsigned unsorted = 1, ungrouped = 1, not_strict = 1;
     bool grouped_fits = true;  // false: a row too long for the row-grouped kernels
     uint64_t long_hits = 0;  // sampled inserts that 32 others of their row follow (3 / 16 of the inserts looked at)
+    int64_t clustered = 0;   // sampled inserts with a near successor in their row, less those with a far one
     bool ready = false;
     DevBuf off;             // a first lock: the staged rows' offsets ...
     bool have_off = false;  // ... when the rows are grouped and no step between them was long
@@ -515,26 +530,41 @@ int staged_offsets(Ctx *c, Prepared *pre, const uint32_t *rows, uint64_t m, uint
 
 constexpr uint64_t FEW_STAGED = 4u << 20;
 
-// Prepared::long_hits of rows sorted since lock_prepare, from 2^16 places.
+// A sixteenth of the columns: a successor at random is nearer once in eight.
+uint32_t near_columns(uint64_t n_cols) { return (uint32_t)std::min<uint64_t>(n_cols / 16 + 1, 0xFFFFFFFFull); }
+
+// Prepared::long_hits and clustered of rows sorted since lock_prepare, from 2^16 places.
 constexpr uint64_t LONG_SAMPLES = 1u << 16;
 
-__global__ void long_rows_sample(const uint32_t *__restrict__ rows, uint64_t m, unsigned *__restrict__ hits,
-                                 unsigned long long *__restrict__ words) {
+__global__ void long_rows_sample(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, uint64_t m,
+                                 uint32_t near, unsigned *__restrict__ hits, unsigned long long *__restrict__ words) {
     const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, i = k * (m - 32) / LONG_SAMPLES;
     const unsigned n = __popc(__ballot_sync(0xffffffffu, rows[i] == rows[i + 32]));
-    if ((threadIdx.x & 31) == 0 && n) atomicAdd(hits, n);
+    const int score = rows[i] != rows[i + 1] ? 0 : column_gap(cols[i], cols[i + 1]) < near ? 1 : -1;
+    const int sum = __reduce_add_sync(0xffffffffu, score);
+    if ((threadIdx.x & 31) == 0) {
+        if (n) atomicAdd(hits, n);
+        if (sum) atomicAdd(reinterpret_cast<int *>(hits) + 1, sum);
+        __threadfence();
+    }
     __syncthreads();
-    if (threadIdx.x == 0 && last_block(hits + 1)) store_word(words, 0, *(volatile unsigned *)hits);
+    if (threadIdx.x == 0 && last_block(hits + 2)) {
+        store_word(words, 0, *(volatile unsigned *)hits);
+        store_word(words, 1, *(volatile unsigned *)(hits + 1));
+    }
 }
 
-int sample_long_rows(Ctx *c, const uint32_t *rows, uint64_t m, uint64_t *long_hits, cudaStream_t s) {
+int sample_long_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, uint64_t m, uint64_t n_cols, Prepared *pre,
+                     cudaStream_t s) {
     DevBuf hits;
-    SPG_TRY(hits.alloc(2 * sizeof(unsigned), s));
-    SPG_CUDA_TRY(cudaMemsetAsync(hits.ptr, 0, 2 * sizeof(unsigned), s));
-    long_rows_sample<<<LONG_SAMPLES / LB, LB, 0, s>>>(rows, m, hits.as<unsigned>(), c->d_words);
+    SPG_TRY(hits.alloc(3 * sizeof(unsigned), s));
+    SPG_CUDA_TRY(cudaMemsetAsync(hits.ptr, 0, 3 * sizeof(unsigned), s));
+    long_rows_sample<<<LONG_SAMPLES / LB, LB, 0, s>>>(rows, cols, m, near_columns(n_cols), hits.as<unsigned>(),
+                                                        c->d_words);
     SPG_LAUNCH_CHECK();
     SPG_TRY(c->phase_sync(s));
-    *long_hits = (uint64_t)((double)c->word(0) / LONG_SAMPLES * 3.0 / 16.0 * (double)m);
+    pre->clustered = (int)(unsigned)c->word(1);
+    pre->long_hits = (uint64_t)((double)c->word(0) / LONG_SAMPLES * 3.0 / 16.0 * (double)m);
     return SPG_OK;
 }
 
@@ -651,14 +681,19 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
         //            at the row's input positions; a scan of the kept counts
         //            gives the offsets, and entries move only if some were
         //            dropped.
-        // Tiles are faster where rows are long (100k rows of 300 uniform
-        // columns: 0.67 against 1.17 ms; 10k of 3000: 0.83 / 1.00), and below
-        // 4 M inserts, where the classes' ten launches are what is paid (100 k
-        // inserts from the host: 0.174 / 0.235 ms). Rows of up to 32 entries are
-        // the networks' case (27-point stencil, 1 M rows in any column order:
-        // 0.53 / 0.68 ms). So: tiles when a quarter of the entries follow more
-        // than 32 others of their row, or for few inserts.
-        const bool tiles = m <= FEW_STAGED || 64 * pre->long_hits > 3 * m;
+        // Tiles are faster where a row's columns spread over the matrix, so that
+        // its buckets hold an entry each (1 M rows of 24 uniform columns: 0.45
+        // against 0.60 ms; 2 M of 5: 0.26 / 0.30), where rows are long (200 k of
+        // 201 in a band: 0.99 / 1.06; 20 k of 1000 on ten columns: 0.48 / 0.61),
+        // and below 4 M inserts, where the classes' ten launches are what is paid
+        // (600 k rows of 5: 0.15 / 0.18). Short rows of columns close together
+        // crowd their buckets and are the networks' case (27-point stencil, 1 M
+        // rows in any column order: 0.67 / 0.49; 300 k rows of 64 on 200 columns:
+        // 0.54 / 0.43; 2 M of a 5-point stencil 0.27 / 0.23). So: tiles for few
+        // inserts, when about 0.7 of the entries have one of their row 32 places
+        // on, or when most have their successor a sixteenth of the columns away
+        // or more.
+        const bool tiles = m <= FEW_STAGED || 8 * pre->long_hits > m + m / 32 || pre->clustered < 0;
         DevBuf s_off, kept, scols, svals;
         SPG_TRY(staged_offsets(c, pre, rows, m, n, s_off, s));
         bool done = false;
@@ -815,21 +850,21 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
     Prepared pre;
     if (m) {
         DevBuf stats;
-        SPG_TRY(stats.alloc(8 * sizeof(unsigned), s));
-        SPG_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, 8 * sizeof(unsigned), s));
+        SPG_TRY(stats.alloc(9 * sizeof(unsigned), s));
+        SPG_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, 9 * sizeof(unsigned), s));
         if (!A->built) SPG_TRY(pre.off.alloc(csr_off_elems(A->n_rows) * sizeof(uint64_t), s));
         if (((uintptr_t)rows | (uintptr_t)cols) % 16 == 0)
             lock_prepare<true><<<grid_for((m + 3) / 4, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
-                rows, cols, m, bits_for(A->n_cols), A->n_rows, pre.off.as<uint64_t>(), stats.as<unsigned>(),
+                rows, cols, m, bits_for(A->n_cols), A->n_rows, near_columns(A->n_cols), pre.off.as<uint64_t>(), stats.as<unsigned>(),
                 c->d_words);
         else
             lock_prepare<false><<<grid_for(m, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
-                rows, cols, m, bits_for(A->n_cols), A->n_rows, pre.off.as<uint64_t>(), stats.as<unsigned>(),
+                rows, cols, m, bits_for(A->n_cols), A->n_rows, near_columns(A->n_cols), pre.off.as<uint64_t>(), stats.as<unsigned>(),
                 c->d_words);
         SPG_LAUNCH_CHECK();
         SPG_TRY(c->phase_sync(s));
-        unsigned h[7];
-        for (int i = 0; i < 7; ++i) h[i] = (unsigned)c->word(i);
+        unsigned h[8];
+        for (int i = 0; i < 8; ++i) h[i] = (unsigned)c->word(i);
         if ((uint64_t)h[0] >= A->n_rows)
             return set_error(SPG_ERR_OUT_OF_RANGE, "spira::matrix: row_index out of range (%u >= %llu)", h[0],
                              (unsigned long long)A->n_rows);
@@ -840,6 +875,7 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
         pre.ungrouped = h[3];
         pre.not_strict = h[4];
         pre.long_hits = h[5];
+        pre.clustered = (int)h[7];
         pre.have_off = pre.off.ptr && !h[3] && !h[6];
         pre.ready = true;
     }
@@ -859,7 +895,7 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
         pre.ungrouped = 0;
         pre.not_strict = 1;
         pre.have_off = false;
-        if (!has_old && m > FEW_STAGED) SPG_TRY(sample_long_rows(c, rows, m, &pre.long_hits, s));
+        if (!has_old && m > FEW_STAGED) SPG_TRY(sample_long_rows(c, rows, cols, m, A->n_cols, &pre, s));
     }
     const unsigned long long *abort = sorted.abort.as<unsigned long long>();
     if (!has_old) return first_lock(c, A, rows, cols, vals, m, &pre, abort, s);

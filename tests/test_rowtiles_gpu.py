@@ -72,3 +72,23 @@ def test_lock_offsets_of_spaced_rows(ctx, order, step, first, after):
         A = sg.Csr(ctx, n_rows, 12)
         A.lock(rows[:cut], cols[:cut], vals[:cut])
         assert_csr_equal(A.download(), oracle.lock_epochs(n_rows, 12, [(rows[:cut], cols[:cut], vals[:cut])]))
+
+
+@pytest.mark.parametrize("order", ["grouped", "shuffled"])
+@pytest.mark.parametrize("kind", ["uniform", "band"])
+def test_lock_many_short_rows(ctx, kind, order):
+    """Above the few-inserts rule: scattered columns by tiles, columns close
+    together by the row classes (rows of 0..33 entries)."""
+    L = np.tile(np.arange(34, dtype=np.int64), 7500)
+    rows = np.repeat(np.arange(len(L), dtype=np.uint32), L)
+    n_cols = 9_000_001
+    cols = _columns(kind, rows, n_cols, seed=3)
+    vals = gen.sym_unit(gen.hash3(4, 2, np.arange(len(rows), dtype=np.uint64)))
+    vals[::11] = 0.0
+    assert len(rows) > 4 << 20
+    if order == "shuffled":
+        p = np.argsort(gen.hash3(5, 2, np.arange(len(rows), dtype=np.uint64)), kind="stable")
+        rows, cols, vals = rows[p], cols[p], vals[p]
+    A = sg.Csr(ctx, len(L), n_cols)
+    A.lock(rows, cols, vals)
+    assert_csr_equal(A.download(), oracle.lock_epochs(len(L), n_cols, [(rows, cols, vals)]))
