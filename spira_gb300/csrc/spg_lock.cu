@@ -7,18 +7,21 @@
 // slice, the buffer winning on equal columns and a zero deleting
 // (csr_build.hpp:126-488). The GPU formulation computes the same CSR:
 //
-//   1. keys (row << cbits | col) with the staging index as payload go through
-//      a stable LSD radix sort; the last element of each equal-key run is the
-//      last write (stability keeps insertion order within a run);
-//   2. the deduplicated delta D (sorted by row, col; zeros kept) gets row
-//      offsets doff;
-//   3. the delta, sorted, is merged into the old CSR, sorted too, tile by tile
-//      (spg_merge.cu): an equal column takes the delta's value, a zero of the
-//      delta deletes.
+//   1. one pass checks the ranges, tells how the inserts are ordered and samples
+//      the rows' lengths and how scattered their columns are;
+//   2. inserts in any row order are sorted stably by row (spg_rowsort.cu);
+//   3. a first lock sorts, dedups and compacts the grouped rows into the CSR, in
+//      one pass over tiles of rows (spg_rowtiles.cu) or by row classes
+//      (spg_prims.cu); rows too long for either go through a global stable
+//      radix sort of the keys (row << cbits | col), in which the last element
+//      of a run of equal keys is the last write;
+//   4. a later epoch of few inserts goes insert by insert (spg_delta.cu); any
+//      other becomes a sorted delta (zeros kept) and is merged into the old
+//      CSR tile by tile (spg_merge.cu): an equal column takes the delta's
+//      value, a zero of the delta deletes.
 // Everything is integer work or a copy of the value bits, so structure and
-// values are bit-exact against Spira. The first lock is the same pass with an
-// empty old CSR. Capacity follows Spira's rule: the first build is tight;
-// a merge keeps the old capacity when old nnz + |D| fits, else grows to 1.5x
+// values are bit-exact against Spira. Capacity follows Spira's rule: the first
+// build is tight; a merge keeps the old capacity when old nnz + |D| fits, else grows to 1.5x
 // that bound (csr_build.hpp:139-145).
 #include "spg_internal.cuh"
 
@@ -26,7 +29,6 @@ namespace spg {
 namespace {
 
 constexpr int LB = 256;
-
 
 __global__ void lock_make_keys(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols,
                                uint64_t m, int cbits, uint64_t *__restrict__ keys,
@@ -38,7 +40,8 @@ __global__ void lock_make_keys(const uint32_t *__restrict__ rows, const uint32_t
     }
 }
 
-// One pass over the staged inserts: keys and staging indices, plus
+// One pass over the staged inserts, which counts (the last block stores the
+// counts for the host):
 // stats[0] = max row, stats[1] = max column (range check), stats[2] = 1 if
 // some key is greater than its successor (not sorted), stats[3] = 1 if some
 // row is (rows not grouped), stats[4] = 1 if some key is not below its
@@ -60,8 +63,9 @@ struct RowGap {
 // next to nothing (writing every rising step's rows took ~m n / 3 stores
 // there); a longer one sets stats[6], and launch_row_offsets writes the
 // offsets after all (in a matrix of few rows, where short steps are common in
-// random order too, steps of one row only). A pass of its own over the 64 M rows of the 4M-row Zipf
-// matrix took 106 us, the stores here 32 (lock 1.64 -> 1.54 ms).
+// random order too, steps of one row only). A pass of its own over the 64 M
+// inserts' rows of the 4M-row Zipf matrix took 106 us, the stores here 32
+// (lock 1.64 -> 1.54 ms).
 constexpr uint32_t OFF_STEP = 8;
 
 __device__ __forceinline__ bool offsets_step(uint64_t *__restrict__ off, uint64_t lo, uint64_t hi, uint64_t n_rows,

@@ -45,12 +45,14 @@ __global__ void __launch_bounds__(RS_T) rs_hist(const uint32_t *__restrict__ row
         const uint64_t i0 = 4 * it * stride + blockIdx.x * (uint64_t)RS_T + threadIdx.x;
         uint32_t r[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) r[u] = i0 + u * stride < m ? rows[i0 + u * stride] : 0xFFFFFFFFu;
+        for (int u = 0; u < 4; ++u) r[u] = i0 + u * stride < m ? rows[i0 + u * stride] : 0u;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            // one add for a warp of one row (runs of a row would serialise)
-            const bool one = __all_sync(0xffffffffu, r[u] == __shfl_sync(0xffffffffu, r[u], 0));
-            if (i0 + u * stride < m && (!one || (threadIdx.x & 31) == 0)) {
+            // one add for a whole warp of one row (runs of a row would serialise)
+            const bool in = i0 + u * stride < m;
+            const uint32_t r0 = __shfl_sync(0xffffffffu, r[u], 0);
+            const bool one = __all_sync(0xffffffffu, in && r[u] == r0);
+            if (in && (!one || (threadIdx.x & 31) == 0)) {
                 for (int p = 0; p < passes; ++p) atomicAdd(&s_h[p][(r[u] >> (p * bits)) & mask], one ? 32u : 1u);
             }
         }

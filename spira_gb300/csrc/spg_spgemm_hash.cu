@@ -9,8 +9,8 @@
 // C(i, j) the left-to-right sum over ascending k from its first product (+0.0 +
 // p1 = p1 whenever the sum can be kept). The loads of eight A entries' B rows
 // are in flight together. The kept sums are then compacted, put in column
-// order by a bitonic network over the row's lanes, and the tile of SH_ROWS rows goes straight into C through an ordered scan of the
-// tiles' counts.
+// order by a bitonic network over the row's lanes, and the tile of SH_ROWS rows goes straight
+// into C through an ordered scan of the tiles' counts.
 //
 // Bound: the FP64 pipe, one multiply and one add per eight-lane step (0.19 ms
 // for the 48 M products of the 3D 7-point Laplacian squared); measured there:
