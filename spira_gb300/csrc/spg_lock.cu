@@ -914,9 +914,11 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
         SPG_TRY(out_vals.alloc(elems * sizeof(double), s));
         return SPG_OK;
     };
-    // An eighth of the matrix at most goes insert by insert (at 1 M rows of 10,
-    // 100 k inserts: 0.30 ms against 0.40 for the general merge; 5 M: the merge).
-    if (!A->may_have_zeros && m <= A->nnz / 8) {
+    // A fifth of the matrix at most goes insert by insert, unless many rows get
+    // more than it takes (1 M rows of 10, insert by insert / general merge: 100 k
+    // inserts 274 / 385 us, 1.25 M 430 / 507, 2.5 M 551 / 560; 30 k rows of 1000:
+    // 300 k 466 / 663; 3 M, 100 to a row, 1216 with the attempt / 862).
+    if (!A->may_have_zeros && m <= A->nnz / 5 && m <= 32 * n && 16 * pre.long_hits <= m) {
         SPG_TRY(alloc_out(m));
         SPG_TRY(merge_small_delta(c, {A->d_off(), A->d_cols(), A->d_vals(), A->nnz}, n, rows, cols, vals, m, abort,
                                   new_off.as<uint64_t>(), out_cols.as<uint32_t>(), out_vals.as<double>(), &new_nnz, &u,

@@ -30,6 +30,7 @@ namespace {
 constexpr int RS_T = 256, RS_RADIX = 256, RS_LOOK = 8;
 constexpr int RS_MAX_PASSES = 4;
 constexpr int RS_LT = 512, RS_LI = 6, RS_LB = 3;  // large sorts: threads, entries per thread, blocks per SM
+constexpr uint64_t RS_LARGE_PER_SM = 2048;
 constexpr unsigned RS_STATUS_TIMEOUT = 0x80u;
 
 // Digit counts of every pass (hist[p * RS_RADIX + d]).
@@ -259,8 +260,10 @@ RsLaunch rs_launch_of(int bits) {
 int sort_staged_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const double *vals, uint64_t m, int rbits,
                      StagedSorted &out, cudaStream_t s) {
     const int passes = std::max(1, (rbits + 7) / 8), bits = std::max(5, (rbits + passes - 1) / passes);
-    // tiles of RS_LT x RS_LI entries, or of 1024 while those are too few to fill the chip
-    const bool large = m >= (uint64_t)c->n_sms * RS_LB * RS_LT * RS_LI;
+    // tiles of RS_LT x RS_LI entries; of 1024 while the larger ones are fewer than
+    // two for three SMs (first lock in random order into 1 M rows, large / small:
+    // 100 k inserts 153.5 / 152.6 us, 400 k 166 / 173, 1.4 M 220 / 257)
+    const bool large = m >= (uint64_t)c->n_sms * RS_LARGE_PER_SM;
     const uint64_t tile = large ? RS_LT * RS_LI : 256 * 4, tiles = (m + tile - 1) / tile;
     DevBuf work, rows2, cols2, vals2;
     const uint64_t words = passes * (RS_RADIX + 1 + tiles * RS_RADIX);
