@@ -25,7 +25,7 @@
 // tiles copy.
 //
 // Floor: 24 bytes per entry of HBM traffic (12 in, 12 out). Bound: latency
-// between the fifteen barriers of a tile, at half of the issue slots: on the
+// between the fifteen barriers of a tile, at 60 % of the issue slots: on the
 // 64 M entries of the 4M-row Zipf(1.8) matrix 0.75 ms for the tiles, 0.38 for
 // the longer rows (0.23 at the copy rate). Hence small blocks, four of 256
 // threads an SM: two of 512 threads with 4096 entries took 1.03 + 0.26 ms,
