@@ -357,6 +357,8 @@ __global__ void offsets_fill_gaps(const RowGap *__restrict__ gaps, const unsigne
     }
 }
 
+}  // namespace
+
 // off[0..n_rows] from the non-decreasing rows srows[0..u) (stream-ordered).
 int launch_row_offsets(Ctx *c, const uint32_t *srows, uint64_t u, uint64_t n_rows, uint64_t *off, cudaStream_t s) {
     DevBuf scratch;  // [counter (16 bytes)] [GAP_SLOTS gaps]
@@ -374,6 +376,8 @@ int launch_row_offsets(Ctx *c, const uint32_t *srows, uint64_t u, uint64_t n_row
     SPG_LAUNCH_CHECK();
     return SPG_OK;
 }
+
+namespace {
 
 // Explicit zeros of a loaded CSR inside rows the delta touches: Spira's merge
 // drops them (csr_build.hpp:274-276, 292-296). They become synthetic zero

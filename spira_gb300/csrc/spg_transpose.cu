@@ -23,6 +23,7 @@ namespace spg {
 namespace {
 
 constexpr int TB = 256;
+constexpr uint64_t LOOK_LARGE = 10u << 20;
 
 // rowid[k] = source row of entry k (eight lanes per row).
 __global__ void tr_expand(const uint64_t *__restrict__ off, uint64_t n_rows, uint32_t *__restrict__ rowid) {
@@ -226,9 +227,16 @@ int transpose_impl(Ctx *c, const Csr *A, Csr *T, cudaStream_t s) {
     const unsigned gmax = (unsigned)c->n_sms * 32;
     DevBuf out_off, out_cols, out_vals;
     SPG_TRY(out_off.alloc(csr_off_elems(n) * sizeof(uint64_t), s));
-    SPG_CUDA_TRY(cudaMemsetAsync(out_off.ptr, 0, csr_off_elems(n) * sizeof(uint64_t), s));
     unsigned long long longest = NET_MAX + 1;
-    if (nnz) {
+    // Whether the networks may do: source rows below their padding key, and not
+    // above 16 entries a column on average (32 from 10 M entries on), where
+    // finding out costs more than they gain. Looked at first / column sort at
+    // once: 500k x 200k with 20 to a column 267 / 219 us, 500k x 500k with 24 568 /
+    // 502 (columns above 32 both); 25 and 27 to a column, all alike: 300 k columns
+    // 344 / 363, 500 k 514 / 538, 1 M 961 / 1020; 13: 225 / 331.
+    const bool look = nnz && m < 0xFFFFFFFFull && nnz <= (nnz > LOOK_LARGE ? NET_MAX : 16) * n;
+    if (look || nnz == 0) SPG_CUDA_TRY(cudaMemsetAsync(out_off.ptr, 0, csr_off_elems(n) * sizeof(uint64_t), s));
+    if (look) {
         tr_count<<<grid_for(nnz, TB, gmax), TB, 0, s>>>(A->d_cols(), nnz,
                                                        reinterpret_cast<unsigned long long *>(out_off.ptr));
         SPG_LAUNCH_CHECK();
@@ -236,52 +244,50 @@ int transpose_impl(Ctx *c, const Csr *A, Csr *T, cudaStream_t s) {
         // The longest output row decides: up to 32 entries, an atomic scatter
         // and sorting networks per row. That path is enqueued at once, its
         // kernels checking the longest row on the device, so the common case
-        // costs no host round trip before the final one. An average above 32
-        // needs no look. Where both apply the networks are faster (3D Laplacian
-        // 100^3 221 us, 368 by the column sort; 200k x 200k with 12 a row 150 / 170;
-        // 1 M with 6 309 / 326).
-        DevBuf meta, midbuf, cursor, tsrc, tval;
-        if (m < 0xFFFFFFFFull && nnz <= NET_MAX * n) {  // source rows below the networks' padding key
-            SPG_TRY(out_cols.alloc(csr_alloc_elems(nnz) * sizeof(uint32_t), s));
-            SPG_TRY(out_vals.alloc(csr_alloc_elems(nnz) * sizeof(double), s));
-            // [longest row (8 bytes)] [rows of 17..32 entries (8 bytes)] [cursors]
-            SPG_TRY(meta.alloc(16 + n * sizeof(unsigned), s));
-            SPG_CUDA_TRY(cudaMemsetAsync(meta.ptr, 0, 16 + n * sizeof(unsigned), s));
-            unsigned long long *mx = meta.as<unsigned long long>(), *n_mid = mx + 1;
-            unsigned *cur = reinterpret_cast<unsigned *>(mx + 2);
-            tr_max_len<<<grid_for(std::max(n, m), TB, (unsigned)c->n_sms * 8), TB, 0, s>>>(out_off.as<uint64_t>(), n, A->d_off(),
-                                                                             m, mx);
-            SPG_LAUNCH_CHECK();
-            SPG_TRY(tsrc.alloc(nnz * sizeof(uint32_t), s));
-            SPG_TRY(tval.alloc(nnz * sizeof(double), s));
-            SPG_TRY(midbuf.alloc(n * sizeof(uint32_t), s));
-            tr_scatter<<<grid_for(m, TB), TB, 0, s>>>(A->d_off(), A->d_cols(), A->d_vals(), m, out_off.as<uint64_t>(),
-                                                      cur, tsrc.as<uint32_t>(), tval.as<double>(), mx);
-            tr_sort_short<<<grid_for(n, TB, gmax), TB, 0, s>>>(out_off.as<uint64_t>(), n, tsrc.as<uint32_t>(),
-                                                               tval.as<double>(), out_cols.as<uint32_t>(),
-                                                               out_vals.as<double>(), n_mid, midbuf.as<uint32_t>(),
-                                                               mx);
-            tr_sort_mid<<<(unsigned)c->n_sms * 8, TB, 0, s>>>(out_off.as<uint64_t>(), midbuf.as<uint32_t>(), n_mid,
-                                                             tsrc.as<uint32_t>(), tval.as<double>(),
-                                                             out_cols.as<uint32_t>(), out_vals.as<double>(), mx, c->d_words);
-            SPG_LAUNCH_CHECK();
-            SPG_TRY(c->phase_sync(s));
-            longest = c->word(0);
-        }
-        if (longest > NET_MAX) {
-            // (column, source row, value) sorted stably by column: the rows of a
-            // column stay in ascending order, whatever its length
-            StagedSorted o;
-            DevBuf rowid;
-            SPG_TRY(rowid.alloc(nnz * sizeof(uint32_t), s));
-            tr_expand<<<grid_for(m * 8, TB), TB, 0, s>>>(A->d_off(), m, rowid.as<uint32_t>());
-            SPG_LAUNCH_CHECK();
-            SPG_TRY(sort_staged_rows(c, A->d_cols(), rowid.as<uint32_t>(), A->d_vals(), nnz, bits_for(n), o, s));
-            out_cols = std::move(o.cols);
-            out_vals = std::move(o.vals);
-            SPG_TRY(c->phase_sync(s));
-        }
-    } else {
+        // costs no host round trip before the final one. Where both apply the
+        // networks are faster (3D Laplacian 100^3 221 us, 368 by the column sort;
+        // 200k x 200k with 12 a row 150 / 170; 1 M with 6 309 / 326).
+        DevBuf meta, midbuf, tsrc, tval;
+        SPG_TRY(out_cols.alloc(csr_alloc_elems(nnz) * sizeof(uint32_t), s));
+        SPG_TRY(out_vals.alloc(csr_alloc_elems(nnz) * sizeof(double), s));
+        // [longest row (8 bytes)] [rows of 17..32 entries (8 bytes)] [cursors]
+        SPG_TRY(meta.alloc(16 + n * sizeof(unsigned), s));
+        SPG_CUDA_TRY(cudaMemsetAsync(meta.ptr, 0, 16 + n * sizeof(unsigned), s));
+        unsigned long long *mx = meta.as<unsigned long long>(), *n_mid = mx + 1;
+        unsigned *cur = reinterpret_cast<unsigned *>(mx + 2);
+        tr_max_len<<<grid_for(std::max(n, m), TB, (unsigned)c->n_sms * 8), TB, 0, s>>>(out_off.as<uint64_t>(), n, A->d_off(),
+                                                                         m, mx);
+        SPG_LAUNCH_CHECK();
+        SPG_TRY(tsrc.alloc(nnz * sizeof(uint32_t), s));
+        SPG_TRY(tval.alloc(nnz * sizeof(double), s));
+        SPG_TRY(midbuf.alloc(n * sizeof(uint32_t), s));
+        tr_scatter<<<grid_for(m, TB), TB, 0, s>>>(A->d_off(), A->d_cols(), A->d_vals(), m, out_off.as<uint64_t>(),
+                                                  cur, tsrc.as<uint32_t>(), tval.as<double>(), mx);
+        tr_sort_short<<<grid_for(n, TB, gmax), TB, 0, s>>>(out_off.as<uint64_t>(), n, tsrc.as<uint32_t>(),
+                                                           tval.as<double>(), out_cols.as<uint32_t>(),
+                                                           out_vals.as<double>(), n_mid, midbuf.as<uint32_t>(),
+                                                           mx);
+        tr_sort_mid<<<(unsigned)c->n_sms * 8, TB, 0, s>>>(out_off.as<uint64_t>(), midbuf.as<uint32_t>(), n_mid,
+                                                         tsrc.as<uint32_t>(), tval.as<double>(),
+                                                         out_cols.as<uint32_t>(), out_vals.as<double>(), mx, c->d_words);
+        SPG_LAUNCH_CHECK();
+        SPG_TRY(c->phase_sync(s));
+        longest = c->word(0);
+    }
+    if (nnz && longest > NET_MAX) {
+        // (column, source row, value) sorted stably by column: the rows of a
+        // column stay in ascending order, whatever its length
+        StagedSorted o;
+        DevBuf rowid;
+        SPG_TRY(rowid.alloc(nnz * sizeof(uint32_t), s));
+        tr_expand<<<grid_for(m * 8, TB), TB, 0, s>>>(A->d_off(), m, rowid.as<uint32_t>());
+        SPG_LAUNCH_CHECK();
+        SPG_TRY(sort_staged_rows(c, A->d_cols(), rowid.as<uint32_t>(), A->d_vals(), nnz, bits_for(n), o, s));
+        if (!look) SPG_TRY(launch_row_offsets(c, o.rows.as<uint32_t>(), nnz, n, out_off.as<uint64_t>(), s));
+        out_cols = std::move(o.cols);
+        out_vals = std::move(o.vals);
+        SPG_TRY(c->phase_sync(s));
+    } else if (nnz == 0) {
         SPG_TRY(out_cols.alloc(csr_alloc_elems(0) * sizeof(uint32_t), s));
         SPG_TRY(out_vals.alloc(csr_alloc_elems(0) * sizeof(double), s));
         SPG_TRY(c->phase_sync(s));

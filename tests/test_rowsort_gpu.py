@@ -89,6 +89,9 @@ def test_lock_small_later_epoch(ctx, n_rows, per_row, m, order):
     (20_000, 20_000, 400_000),     # a few columns above 32
     (9000, 1, 9000),               # one column
     (70_000, 300, 2_500_000),      # the large tiles
+    (30_000, 4000, 60_000),        # 15 to a column: looked at first
+    (30_000, 4000, 64_500),        # above 16: the column sort at once
+    (9000, 3_000_000, 9000),       # most columns empty
 ])
 def test_transpose_by_column_sort(ctx, n_rows, n_cols, m):
     first = _inserts(m, n_rows, n_cols, seed=m)
