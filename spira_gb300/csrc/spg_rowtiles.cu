@@ -65,7 +65,7 @@ struct RtArgs {
     bool keep_zeros;
     unsigned long long *ctr;
     unsigned long long *plan_state, *tile_state;
-    uint32_t *tile_start;  // first row of each tile, then n_rows
+    uint64_t *tile_start;  // first row of each tile, then n_rows (2^32 in the transpose of a matrix of 2^32 columns)
     uint32_t *longer;      // rows of RT_CAP+1 .. RT_MID entries from the front, longer ones from the back
     uint64_t n_longer;
     uint32_t *big_cols;    // their ordered entries, at the rows' input positions
@@ -148,9 +148,9 @@ __global__ void __launch_bounds__(RP_T) rt_plan(RtArgs a) {
     }
     __syncthreads();
     if (!s_ok) return;  // (the tile kernel then has no tiles; the status word fails the call)
-    for (uint32_t k = lane; k < n; k += 32) a.tile_start[s_base + before + k] = (uint32_t)(r0 + s_list[p0 + k]);
+    for (uint32_t k = lane; k < n; k += 32) a.tile_start[s_base + before + k] = r0 + s_list[p0 + k];
     if (t == 0 && r0 + RP_ROWS >= a.n_rows) {
-        a.tile_start[s_base + total] = (uint32_t)a.n_rows;
+        a.tile_start[s_base + total] = a.n_rows;
         a.ctr[RC_TILES] = s_base + total;
     }
 }
@@ -669,7 +669,7 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     SPG_TRY(out->vals.alloc(csr_alloc_elems(m) * sizeof(double), s));
     SPG_TRY(state.alloc((RC_N + plan_tiles + t_max) * sizeof(unsigned long long), s));
     SPG_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, (RC_N + plan_tiles + t_max) * sizeof(unsigned long long), s));
-    SPG_TRY(tiles.alloc((t_max + 1) * sizeof(uint32_t), s));
+    SPG_TRY(tiles.alloc((t_max + 1) * sizeof(uint64_t), s));
     SPG_TRY(longer.alloc(n_long * sizeof(uint32_t), s));
     if (may_long) {
         SPG_TRY(big_cols.alloc(m * sizeof(uint32_t), s));
@@ -685,7 +685,7 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     a.ctr = state.as<unsigned long long>();
     a.plan_state = a.ctr + RC_N;
     a.tile_state = a.plan_state + plan_tiles;
-    a.tile_start = tiles.as<uint32_t>();
+    a.tile_start = tiles.as<uint64_t>();
     a.longer = longer.as<uint32_t>();
     a.n_longer = n_long;
     a.big_cols = big_cols.as<uint32_t>();
