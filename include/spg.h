@@ -116,6 +116,11 @@ int spg_ctx_timer_stop(spg_ctx *ctx, double *device_ms);
  * the context stays usable; *gave_up = 1 when the wait gave up as designed.
  * No Spira counterpart. */
 int spg_selftest_wait_timeout(spg_ctx *ctx, long long wait_cycles, int *gave_up);
+/* The same for every kind of wait there is: *kinds = the sum of those that
+ * gave up as designed, with nothing written by the blocks that waited. */
+#define SPG_WAIT_SCAN 1     /* one warp looks back (SpGEMM's tiles, the row tiles' plan) */
+#define SPG_WAIT_ROW_SORT 4 /* a thread per digit looks back (the row sort's passes) */
+int spg_selftest_wait_kinds(spg_ctx *ctx, long long wait_cycles, int *kinds);
 /* Bytes of the context's device memory pool (the device's default
  * stream-ordered pool, from which every device buffer of libspg comes) that
  * live buffers hold, and that the pool holds from the driver (freed buffers

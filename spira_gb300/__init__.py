@@ -101,6 +101,7 @@ _SIGS = [
     ("spg_ctx_sync", _I, [_P]),
     ("spg_ctx_pool_used", _I, [_P, C.POINTER(_U64), C.POINTER(_U64)]),
     ("spg_selftest_wait_timeout", _I, [_P, C.c_longlong, C.POINTER(_I)]),
+    ("spg_selftest_wait_kinds", _I, [_P, C.c_longlong, C.POINTER(_I)]),
     ("spg_ctx_timer_start", _I, [_P]),
     ("spg_ctx_timer_stop", _I, [_P, C.POINTER(C.c_double)]),
     ("spg_csr_create", _I, [_P, _U64, _U64, C.POINTER(_P)]),

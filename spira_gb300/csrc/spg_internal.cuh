@@ -548,6 +548,8 @@ struct StagedSorted {
 };
 int sort_staged_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const double *vals, uint64_t m, int rbits,
                      StagedSorted &out, cudaStream_t s);
+// Part of spg_selftest_wait_kinds: the sort's wait for earlier tiles runs out.
+int rowsort_wait_selftest(Ctx *c, long long wait_cycles, bool *gave_up, cudaStream_t s);
 // off[0..n_rows] from the non-decreasing rows srows[0..u) (spg_lock.cu, stream-ordered).
 int launch_row_offsets(Ctx *c, const uint32_t *srows, uint64_t u, uint64_t n_rows, uint64_t *off, cudaStream_t s);
 // A later lock's delta, small against the matrix, merged into it

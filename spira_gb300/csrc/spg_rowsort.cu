@@ -21,6 +21,7 @@
 // the (row, column) keys took 6, of three launches each and with an index that
 // fetched every value at random afterwards.
 #include <algorithm>
+#include <vector>
 
 #include "spg_internal.cuh"
 
@@ -77,22 +78,26 @@ struct RsSmem {
     uint64_t tile;
 };
 
-template <int T, int I, int PER_SM, int BITS>
+// TEST: waits end after wait_cycles (the limit is a constant otherwise: 1 % of a pass).
+template <int T, int I, int PER_SM, int BITS, bool TEST = false>
 __global__ void __launch_bounds__(T, PER_SM)
 rs_pass(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, const double *__restrict__ vals,
         uint64_t m, int shift, const unsigned long long *__restrict__ hist,
         unsigned long long *__restrict__ ticket, unsigned long long *__restrict__ state,
         uint32_t *__restrict__ out_rows, uint32_t *__restrict__ out_cols, double *__restrict__ out_vals,
-        unsigned int *__restrict__ status, unsigned long long *__restrict__ abort) {
+        unsigned int *__restrict__ status, unsigned long long *__restrict__ abort, long long wait_cycles) {
     constexpr int TILE = T * I, W = T / 32;
     static_assert(T >= RS_RADIX && T % 32 == 0, "a thread per digit");
     extern __shared__ __align__(16) unsigned char rs_raw[];
     auto &S = *reinterpret_cast<RsSmem<T, I> *>(rs_raw);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    if (*abort) return;  // an earlier pass gave up
-    if (t == 0) S.tile = atomicAdd(ticket, 1ull);
+    // An earlier pass, or a block of this one, may have given up. The flag can
+    // change while the block's threads read it: what thread 0 saw counts for
+    // all. (Thread 0 alone reading it cost 3 % of a pass.)
+    const bool stop = *abort;
+    if (t == 0 && !stop) S.tile = atomicAdd(ticket, 1ull);
     for (int i = t; i < W * RS_RADIX / 2; i += T) reinterpret_cast<uint32_t *>(&S.cnt[0][0])[i] = 0;
-    __syncthreads();
+    if (__syncthreads_or(t == 0 && stop)) return;
     const uint64_t tile = S.tile, t0 = tile * TILE;
     const int n = (int)min((uint64_t)TILE, m - t0);
     // the columns and values are wanted once the ranks are known: into the L2 meanwhile
@@ -209,7 +214,7 @@ rs_pass(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, co
                 }
             }
             q -= used;
-            if (wait && clock64() - c0 > LB_WAIT_CYCLES) {
+            if (wait && clock64() - c0 > (TEST ? wait_cycles : LB_WAIT_CYCLES)) {
                 atomicOr(status, RS_STATUS_TIMEOUT);
                 *(volatile unsigned long long *)abort = 1ull;
                 fail = true;
@@ -238,7 +243,7 @@ int rs_launch(const uint32_t *rows, const uint32_t *cols, const double *vals, ui
     SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint64_t tiles = (m + T * I - 1) / (T * I);
     k<<<(unsigned)tiles, T, smem, s>>>(rows, cols, vals, m, shift, hist, ticket, state, orows, ocols, ovals,
-                                       status, abort);
+                                       status, abort, LB_WAIT_CYCLES);
     SPG_LAUNCH_CHECK();
     return SPG_OK;
 }
@@ -296,6 +301,51 @@ int sort_staged_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const d
         ic = oc;
         iv = ov;
     }
+    return SPG_OK;
+}
+
+// A pass whose first tile nobody takes: every tile waits for it, gives up after
+// wait_cycles and stops the rest, of this pass and of the next one, before
+// anything is written. Half of the blocks start when the others have given up.
+int rowsort_wait_selftest(Ctx *c, long long wait_cycles, bool *gave_up, cudaStream_t s) {
+    constexpr int T = 256, I = 4, PER_SM = 6;
+    const uint64_t tiles = 1 + 2 * PER_SM * (uint64_t)c->n_sms, m = tiles * T * I;
+    const uint64_t words = RS_RADIX + 3 + 2 * tiles * RS_RADIX;  // digit counts, two tickets, the flag, two passes' states
+    DevBuf work, rows, vals, orows, ocols, ovals;
+    SPG_TRY(work.alloc(words * sizeof(unsigned long long), s));
+    SPG_TRY(rows.alloc(m * sizeof(uint32_t), s));  // (the columns too)
+    SPG_TRY(vals.alloc(m * sizeof(double), s));
+    SPG_TRY(orows.alloc(m * sizeof(uint32_t), s));
+    SPG_TRY(ocols.alloc(m * sizeof(uint32_t), s));
+    SPG_TRY(ovals.alloc(m * sizeof(double), s));
+    SPG_CUDA_TRY(cudaMemsetAsync(work.ptr, 0, words * sizeof(unsigned long long), s));
+    SPG_CUDA_TRY(cudaMemsetAsync(rows.ptr, 0, m * sizeof(uint32_t), s));
+    SPG_CUDA_TRY(cudaMemsetAsync(vals.ptr, 0, m * sizeof(double), s));
+    SPG_CUDA_TRY(cudaMemsetAsync(orows.ptr, 0xFF, m * sizeof(uint32_t), s));
+    unsigned long long *hist = work.as<unsigned long long>(), *ticket = hist + RS_RADIX, *abort = ticket + 2,
+                       *state = abort + 1;
+    SPG_CUDA_TRY(cudaMemsetAsync(ticket, 1, 1, s));  // the first pass's tickets start at 1
+    auto k = rs_pass<T, I, PER_SM, 8, true>;
+    constexpr size_t smem = sizeof(RsSmem<T, I>);
+    SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (uint64_t p = 0; p < 2; ++p) {
+        k<<<(unsigned)(tiles - 1 + p), T, smem, s>>>(rows.as<uint32_t>(), rows.as<uint32_t>(), vals.as<double>(), m, 0,
+                                                    hist, ticket + p, state + p * tiles * RS_RADIX,
+                                                    orows.as<uint32_t>(), ocols.as<uint32_t>(), ovals.as<double>(),
+                                                    c->d_status, abort, wait_cycles);
+        SPG_LAUNCH_CHECK();
+    }
+    std::vector<unsigned long long> w(words);
+    std::vector<uint32_t> o(m);
+    SPG_CUDA_TRY(cudaMemcpyAsync(w.data(), work.ptr, words * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    SPG_CUDA_TRY(cudaMemcpyAsync(o.data(), orows.ptr, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    SPG_CUDA_TRY(cudaStreamSynchronize(s));
+    const unsigned long long *wt = w.data() + RS_RADIX, *ws = wt + 3;
+    bool ok = (*(volatile unsigned *)c->h_status & RS_STATUS_TIMEOUT) && wt[2] == 1 && wt[1] == 0;
+    for (uint64_t i = 0; i < RS_RADIX; ++i) ok = ok && ws[i] == 0 && ws[RS_RADIX + i] == LB_POISON;  // tiles 0 and 1
+    for (uint64_t i = wt[0] * RS_RADIX; i < 2 * tiles * RS_RADIX; ++i) ok = ok && ws[i] == 0;  // tiles nobody took
+    for (uint32_t x : o) ok = ok && x == 0xFFFFFFFFu;
+    *gave_up = ok;
     return SPG_OK;
 }
 

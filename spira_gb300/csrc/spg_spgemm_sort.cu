@@ -696,3 +696,14 @@ extern "C" int spg_selftest_wait_timeout(spg_ctx *c, long long wait_cycles, int 
     *gave_up = (h[0] == 1 && h[1] == LB_POISON) ? 1 : 0;
     return SPG_OK;  // the timeout itself is reported by the next spg_ctx_sync
 }
+
+extern "C" int spg_selftest_wait_kinds(spg_ctx *c, long long wait_cycles, int *kinds) {
+    if (!kinds) return set_error(SPG_ERR_INVALID_ARGUMENT, "spg_selftest_wait_kinds: null argument");
+    *kinds = 0;
+    int scan = 0;
+    SPG_TRY(spg_selftest_wait_timeout(c, wait_cycles, &scan));
+    bool sort = false;
+    SPG_TRY(rowsort_wait_selftest(c, wait_cycles, &sort, c->stream));
+    *kinds = (scan ? SPG_WAIT_SCAN : 0) | (sort ? SPG_WAIT_ROW_SORT : 0);
+    return SPG_OK;
+}
