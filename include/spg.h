@@ -119,6 +119,7 @@ int spg_selftest_wait_timeout(spg_ctx *ctx, long long wait_cycles, int *gave_up)
 /* The same for every kind of wait there is: *kinds = the sum of those that
  * gave up as designed, with nothing written by the blocks that waited. */
 #define SPG_WAIT_SCAN 1     /* one warp looks back (SpGEMM's tiles, the row tiles' plan) */
+#define SPG_WAIT_BLOCK 2    /* a block looks back (the row tiles, the CSR merge, the hash SpGEMM) */
 #define SPG_WAIT_ROW_SORT 4 /* a thread per digit looks back (the row sort's passes) */
 int spg_selftest_wait_kinds(spg_ctx *ctx, long long wait_cycles, int *kinds);
 /* Bytes of the context's device memory pool (the device's default

@@ -449,7 +449,7 @@ struct BlockLookback {
 template <int T>
 __device__ __forceinline__ bool block_lookback(BlockLookback<T> &S, unsigned long long *tstate, uint64_t id,
                                                uint64_t total, uint64_t &base, unsigned int *status,
-                                               unsigned status_bit) {
+                                               unsigned status_bit, long long wait_cycles = LB_WAIT_CYCLES) {
     constexpr int W = T / 32;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     base = 0;
@@ -472,7 +472,7 @@ __device__ __forceinline__ bool block_lookback(BlockLookback<T> &S, unsigned lon
             S.sum[warp] = add;
             S.state[warp] = (pref ? 1u : 0u) | (waiting ? 2u : 0u) | (poison ? 4u : 0u);
         }
-        const bool late = __syncthreads_or(t == 0 && clock64() - t0 > LB_WAIT_CYCLES);
+        const bool late = __syncthreads_or(t == 0 && clock64() - t0 > wait_cycles);
         bool found = false, wait = false, bad = false;
         uint64_t sum = 0;
 #pragma unroll

@@ -519,6 +519,18 @@ __global__ void sgs_wait_selftest(SgsArgs g, unsigned long long *out) {
     }
 }
 
+// The same for a block's look-back: block b is tile n - 2 + b of n, of which
+// tile 0 never publishes. out[b] = 1 if it gave up.
+template <int T>
+__global__ void __launch_bounds__(T)
+block_wait_selftest(unsigned long long *tstate, uint64_t n, unsigned int *status, long long wait_cycles,
+                    unsigned long long *out) {
+    __shared__ BlockLookback<T> lb;
+    uint64_t base = 0;
+    const bool ok = block_lookback<T>(lb, tstate, n - 2 + blockIdx.x, 1, base, status, SGS_STATUS_TIMEOUT, wait_cycles);
+    if (threadIdx.x == T - 1) out[blockIdx.x] = ok ? 0ull : 1ull;
+}
+
 struct SortConfig {
     uint32_t hb;   // products (and A entries) per warp-sorted row at most
     uint32_t tpb;  // products per tile at most (shared memory)
@@ -697,13 +709,39 @@ extern "C" int spg_selftest_wait_timeout(spg_ctx *c, long long wait_cycles, int 
     return SPG_OK;  // the timeout itself is reported by the next spg_ctx_sync
 }
 
+namespace {
+
+// Windows of T tiles, the last of them with the tile that never publishes.
+template <int T>
+int block_wait_gives_up(Ctx *c, long long wait_cycles, bool *gave_up, cudaStream_t s) {
+    constexpr uint64_t N = 3 * T;
+    std::vector<unsigned long long> h(N + 2, LB_AGG | 1ull);  // tiles, then what the two blocks report
+    h[0] = h[N] = h[N + 1] = 0;
+    DevBuf state;
+    SPG_TRY(state.alloc((N + 2) * sizeof(unsigned long long), s));
+    unsigned long long *d = state.as<unsigned long long>();
+    SPG_CUDA_TRY(cudaMemcpyAsync(d, h.data(), (N + 2) * sizeof(unsigned long long), cudaMemcpyHostToDevice, s));
+    block_wait_selftest<T><<<2, T, 0, s>>>(d, N, c->d_status, wait_cycles, d + N);
+    SPG_LAUNCH_CHECK();
+    SPG_CUDA_TRY(cudaMemcpyAsync(h.data(), d, (N + 2) * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    SPG_CUDA_TRY(cudaStreamSynchronize(s));
+    bool ok = h[0] == 0 && h[N] == 1 && h[N + 1] == 1 && (*(volatile unsigned *)c->h_status & SGS_STATUS_TIMEOUT);
+    for (uint64_t i = 1; i < N; ++i) ok = ok && h[i] == (i < N - 2 ? (LB_AGG | 1ull) : LB_POISON);
+    *gave_up = ok;
+    return SPG_OK;
+}
+
+}  // namespace
+
 extern "C" int spg_selftest_wait_kinds(spg_ctx *c, long long wait_cycles, int *kinds) {
     if (!kinds) return set_error(SPG_ERR_INVALID_ARGUMENT, "spg_selftest_wait_kinds: null argument");
     *kinds = 0;
     int scan = 0;
     SPG_TRY(spg_selftest_wait_timeout(c, wait_cycles, &scan));
-    bool sort = false;
+    bool block = false, narrow = false, sort = false;
+    SPG_TRY(block_wait_gives_up<256>(c, wait_cycles, &block, c->stream));
+    SPG_TRY(block_wait_gives_up<128>(c, wait_cycles, &narrow, c->stream));
     SPG_TRY(rowsort_wait_selftest(c, wait_cycles, &sort, c->stream));
-    *kinds = (scan ? SPG_WAIT_SCAN : 0) | (sort ? SPG_WAIT_ROW_SORT : 0);
+    *kinds = (scan ? SPG_WAIT_SCAN : 0) | (block && narrow ? SPG_WAIT_BLOCK : 0) | (sort ? SPG_WAIT_ROW_SORT : 0);
     return SPG_OK;
 }

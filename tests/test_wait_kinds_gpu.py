@@ -14,7 +14,7 @@ from conftest import assert_csr_equal
 
 pytestmark = pytest.mark.gpu
 
-KINDS = {"scan": 1, "row_sort": 4}
+KINDS = {"scan": 1, "block": 2, "row_sort": 4}
 
 
 @pytest.mark.parametrize("wait_cycles", [1, 200_000, 20_000_000])
