@@ -527,8 +527,10 @@ int radix_sort_pairs_u64(Ctx *c, uint64_t *d_keys, uint32_t *d_vals, uint64_t n,
 // write per column, unless zero, in column order at the row's first input
 // positions (out_cols / out_vals[s_off[r] + k], k < off[r + 1] - off[r]);
 // s_off[r] = first position of row r (n_rows + 1 entries), off the scan of the
-// rows' kept entries, *nnz of them in all (synchronises the stream). *done = false when a row has more than 12 288 entries or columns need more
-// than 26 bits; the outputs are then undefined.
+// rows' kept entries, *nnz of them in all (synchronises the stream). *done =
+// false when a row has more than 12 288 entries or columns need more than
+// ROW_CLASS_CBITS bits; the outputs are then undefined.
+constexpr int ROW_CLASS_CBITS = 26;
 int dedup_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off, uint64_t m,
                        uint64_t n_rows, int cbits, uint32_t *out_cols, double *out_vals, uint64_t *off, uint64_t *nnz,
                        bool *done, cudaStream_t s);

@@ -700,8 +700,10 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
         // 0.54 / 0.43; 2 M of a 5-point stencil 0.27 / 0.23). So: tiles for few
         // inserts, when about 0.7 of the entries have one of their row 32 places
         // on, or when most have their successor a sixteenth of the columns away
-        // or more.
-        const bool tiles = m <= FEW_STAGED || 8 * pre->long_hits > m + m / 32 || pre->clustered < 0;
+        // or more; and for columns wider than the classes take, whose only
+        // other way is the global sort (2 M rows of a 5-point stencil in 2^31
+        // columns 0.26 / 1.33, shuffled 0.67 / 1.72).
+        const bool tiles = m <= FEW_STAGED || cbits > ROW_CLASS_CBITS || 8 * pre->long_hits > m + m / 32 || pre->clustered < 0;
         DevBuf s_off, kept, scols, svals;
         SPG_TRY(staged_offsets(c, pre, rows, m, n, s_off, s));
         bool done = false;

@@ -439,7 +439,6 @@ constexpr int TS1_T = 256, TS1_I = 16;   // rows up to 4096
 constexpr int TS2_T = 768, TS2_I = 16;   // rows up to TS_MAX
 constexpr int TS0 = TS0_T * TS0_I, TS1 = TS1_T * TS1_I, TS_MAX = TS2_T * TS2_I;
 constexpr int RS_DBITS = 6, RS_DIGITS = 1 << RS_DBITS, RS_WORDS = RS_DIGITS / 2;
-constexpr int SEG_MAX_CBITS = 26;
 
 // counters (unsigned) of the plan
 enum : int {
@@ -970,7 +969,7 @@ int launch_tile_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, const 
 int seg_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, uint64_t m, uint64_t n_rows, int cbits,
              const SegOut &o, uint64_t *nnz, bool *done, cudaStream_t s) {
     *done = false;
-    if (cbits > SEG_MAX_CBITS || m > 0xFFFFFFFFull) return SPG_OK;
+    if (cbits > ROW_CLASS_CBITS || m > 0xFFFFFFFFull) return SPG_OK;
     DevBuf ctr_b, lists_b;
     SPG_TRY(ctr_b.alloc(2 * SC_N * sizeof(unsigned), s));  // counters, then the fill cursors
     SPG_TRY(lists_b.alloc(n_rows * sizeof(uint32_t), s));
