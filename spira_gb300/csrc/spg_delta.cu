@@ -58,50 +58,47 @@ __device__ __forceinline__ bool sd_off(const SdArgs &a) { return a.ctr[1] != 0 |
 __global__ void __launch_bounds__(SD_T) sd_probe(SdArgs a) {
     if (a.abort && *a.abort) return;
     const uint64_t i = blockIdx.x * (uint64_t)SD_T + threadIdx.x;
+    // More than SD_RUN inserts of a row ahead or behind, here or in a block
+    // before: the attempt ends. (An epoch in no order shows only now, sorted,
+    // how many inserts its rows get: 900 k in 3000 rows of 1 M, thrown away
+    // after 64 steps of every insert 456 us, at once 371.)
+    const uint32_t r = i < a.m ? a.rows[i] : 0;
+    const bool over = i < a.m && ((i >= (uint64_t)SD_RUN && a.rows[i - SD_RUN] == r) ||
+                                  (i + SD_RUN < a.m && a.rows[i + SD_RUN] == r));
+    if (__syncthreads_or(over || (threadIdx.x == 0 && a.ctr[1]))) {
+        if (threadIdx.x == 0) a.ctr[1] = 1ull;
+        return;
+    }
     bool last = false;
     if (i < a.m) {
-        const uint32_t r = a.rows[i], c = a.cols[i];
+        const uint32_t c = a.cols[i];
         uint64_t p = i;  // sorted position
-        bool over = false;
         last = true;
-        for (int k = 1;; ++k) {  // the row's inserts before this one
+        for (int k = 1; k < SD_RUN; ++k) {  // the row's inserts before this one
             if (i < (uint64_t)k || a.rows[i - k] != r) break;
-            if (k == SD_RUN) {
-                over = true;
-                break;
-            }
             if (a.cols[i - k] > c) --p;
         }
-        for (int k = 1;; ++k) {  // and after it
+        for (int k = 1; k < SD_RUN; ++k) {  // and after it
             if (i + k >= a.m || a.rows[i + k] != r) break;
-            if (k == SD_RUN) {
-                over = true;
-                break;
-            }
             const uint32_t o = a.cols[i + k];
             if (o < c) ++p;
             last = last && o != c;
         }
-        if (over) {
-            a.ctr[1] = 1ull;
-        } else {
-            const double v = a.vals[i];
-            const uint64_t rb = a.A.off[r], re = a.A.off[r + 1];
-            uint64_t lo = rb, hi = re;
-            while (lo < hi) {
-                const uint64_t mid = (lo + hi) >> 1;
-                if (a.A.cols[mid] < c) lo = mid + 1;
-                else hi = mid;
-            }
-            const bool hit = last && lo < re && a.A.cols[lo] == c, zero = is_zero(v);
-            a.place[p] = lo;
-            a.row[p] = r;
-            a.col[p] = c;
-            a.val[p] = v;
-            a.flag[p] = (hit ? SD_HIT : 0u) | (last ? SD_LAST : 0u);
-            a.P[p] = !last ? 0 : hit ? (zero ? -1 : 0) : (zero ? 0 : 1);
+        const double v = a.vals[i];
+        const uint64_t rb = a.A.off[r], re = a.A.off[r + 1];
+        uint64_t lo = rb, hi = re;
+        while (lo < hi) {
+            const uint64_t mid = (lo + hi) >> 1;
+            if (a.A.cols[mid] < c) lo = mid + 1;
+            else hi = mid;
         }
-        last = last && !over;
+        const bool hit = last && lo < re && a.A.cols[lo] == c, zero = is_zero(v);
+        a.place[p] = lo;
+        a.row[p] = r;
+        a.col[p] = c;
+        a.val[p] = v;
+        a.flag[p] = (hit ? SD_HIT : 0u) | (last ? SD_LAST : 0u);
+        a.P[p] = !last ? 0 : hit ? (zero ? -1 : 0) : (zero ? 0 : 1);
     }
     const unsigned n = __popc(__ballot_sync(0xffffffffu, last));
     if ((threadIdx.x & 31) == 0 && n) atomicAdd(a.ctr, (unsigned long long)n);
