@@ -544,12 +544,13 @@ struct CsrView {
 };
 // Staged inserts stably sorted by row (spg_rowsort.cu). *abort != 0 (and the
 // context's status word is set) if a wait gave up: whatever runs on the outputs
-// before the next phase_sync has to look at it first.
+// before the next phase_sync has to look at it first. earlier: the flag of what
+// the inputs come from (nothing is sorted if it is set); may be null.
 struct StagedSorted {
     DevBuf rows, cols, vals, abort;
 };
 int sort_staged_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const double *vals, uint64_t m, int rbits,
-                     StagedSorted &out, cudaStream_t s);
+                     StagedSorted &out, cudaStream_t s, const unsigned long long *earlier = nullptr);
 // Part of spg_selftest_wait_kinds: the sort's wait for earlier tiles runs out.
 int rowsort_wait_selftest(Ctx *c, long long wait_cycles, bool *gave_up, cudaStream_t s);
 // off[0..n_rows] from the non-decreasing rows srows[0..u) (spg_lock.cu, stream-ordered).
@@ -565,8 +566,9 @@ int merge_small_delta(Ctx *c, const CsrView &A, uint64_t n_rows, const uint32_t 
 // Row-grouped entries (row r's are [s_off[r], s_off[r+1]), columns in any
 // order) as CSR: the last write of every key in (row, column) order, zeros
 // dropped unless keep_zeros (spg_rowtiles.cu). The output arrays are sized
-// for m entries; n of them are used. *done = false when a row has more than
-// 12 288 entries; the outputs are then undefined.
+// for m entries; n of them are used. *done = false when there are rows of more
+// than 12 288 entries and no memory to sort those apart; the outputs are then
+// undefined.
 struct GroupedOut {
     DevBuf off, cols, vals;
     uint64_t n = 0;
@@ -574,6 +576,17 @@ struct GroupedOut {
 int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off,
                        uint64_t m, uint64_t n_rows, int cbits, bool keep_zeros, const unsigned long long *abort,
                        GroupedOut *out, bool *done, cudaStream_t s);
+
+// Its rows of more than 12 288 entries, which no block takes: the n of them in
+// huge[], `entries` in all, as (place in huge[], column, value) in order, reduced
+// like the others; row q's are [first[q], first[q + 1]), and count[huge[q]] is
+// their number (spg_lock.cu). abort: as of StagedSorted.
+struct HugeRows {
+    uint64_t n = 0, entries = 0;
+    DevBuf row, cols, vals, first, abort;
+};
+int order_huge_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off, const uint32_t *huge,
+                    int cbits, bool keep_zeros, HugeRows *H, uint64_t *count, cudaStream_t s);
 
 // SpGEMM pieces shared by its variants (spg_spgemm.cu, spg_spgemm_sort.cu).
 // Expand - sort - compress output: kept entries in (row, column) order.

@@ -12,9 +12,10 @@
 //   2. inserts in any row order are sorted stably by row (spg_rowsort.cu);
 //   3. a first lock sorts, dedups and compacts the grouped rows into the CSR, in
 //      one pass over tiles of rows (spg_rowtiles.cu) or by row classes
-//      (spg_prims.cu); rows too long for either go through a global stable
-//      radix sort of the keys (row << cbits | col), in which the last element
-//      of a run of equal keys is the last write;
+//      (spg_prims.cu). Rows of more than 12 288 inserts fit neither: they are
+//      sorted apart for the tiles, or, where they are most of the inserts, all
+//      goes through a global stable radix sort of the keys (row << cbits | col),
+//      in which the last element of a run of equal keys is the last write;
 //   4. a later epoch of few inserts goes insert by insert (spg_delta.cu); any
 //      other becomes a sorted delta (zeros kept) and is merged into the old
 //      CSR tile by tile (spg_merge.cu): an equal column takes the delta's
@@ -518,7 +519,6 @@ first_keep_gather(const uint64_t *__restrict__ keys, const uint32_t *__restrict_
 // Order flags of a staged epoch, from lock_prepare beside the range check.
 struct Prepared {
     unsigned unsorted = 1, ungrouped = 1, not_strict = 1;
-    bool grouped_fits = true;  // false: a row too long for the row-grouped kernels
     uint64_t long_hits = 0;  // sampled inserts that 32 others of their row follow (3 / 16 of the inserts looked at)
     int64_t clustered = 0;   // sampled inserts with a near successor in their row, less those with a far one
     bool ready = false;
@@ -615,6 +615,153 @@ int sort_dedup(Ctx *c, const uint32_t *rows, const uint32_t *cols, const double 
     return SPG_OK;
 }
 
+// ---- rows that fit no block (HugeRows): gathered, sorted by (row, column) with
+// the row sort's passes, their last writes kept by a count, a scan and a gather.
+// Entry p of all the huge rows' entries: its row is the last q with g[q] <= p.
+// A warp takes 256 neighbours and finds the row of the first by a search.
+__global__ void __launch_bounds__(LB) huge_gather(const uint32_t *__restrict__ huge, const uint64_t *__restrict__ g,
+                                                  uint64_t n, const uint64_t *__restrict__ s_off,
+                                                  const uint32_t *__restrict__ cols, const double *__restrict__ vals,
+                                                  int row_shift, uint32_t *__restrict__ col, uint32_t *__restrict__ row,
+                                                  double *__restrict__ val) {
+    const uint64_t w = (blockIdx.x * (uint64_t)LB + threadIdx.x) >> 5, m = g[n];
+    uint64_t p = w * 256 + (threadIdx.x & 31);
+    if (p >= m) return;
+    uint64_t q = 0, hi = n;
+    while (hi - q > 1) {
+        const uint64_t mid = (q + hi) >> 1;
+        if (g[mid] <= p) q = mid;
+        else hi = mid;
+    }
+    for (int k = 0; k < 8 && p < m; ++k, p += 32) {
+        while (g[q + 1] <= p) ++q;
+        const uint64_t e = s_off[huge[q]] + (p - g[q]);
+        col[p] = cols[e] | (uint32_t)(q << row_shift);
+        row[p] = (uint32_t)q;
+        val[p] = vals[e];
+    }
+}
+
+__global__ void huge_lengths(const uint32_t *__restrict__ huge, uint64_t n, const uint64_t *__restrict__ s_off,
+                             uint64_t *__restrict__ g) {
+    for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < n; q += (uint64_t)gridDim.x * blockDim.x)
+        g[q] = s_off[huge[q] + 1ull] - s_off[huge[q]];
+}
+
+__global__ void huge_counts(const uint32_t *__restrict__ huge, uint64_t n, const uint64_t *__restrict__ first,
+                            uint64_t *__restrict__ count) {
+    for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < n; q += (uint64_t)gridDim.x * blockDim.x)
+        count[huge[q]] = first[q + 1] - first[q];
+}
+
+// The sorted entries' last writes, counted per tile of KTILE (out_row null)
+// and, tile_vals being the counts' scan, written to their places.
+__global__ void __launch_bounds__(KT)
+huge_keep(const uint32_t *__restrict__ row, const uint32_t *__restrict__ col, const double *__restrict__ val,
+          uint32_t col_mask, uint64_t m, bool keep_zeros, const unsigned long long *__restrict__ abort, uint64_t *__restrict__ tile_vals,
+          uint64_t n, uint32_t *__restrict__ out_row, uint32_t *__restrict__ out_col, double *__restrict__ out_val,
+          uint64_t *__restrict__ first) {
+    if (*abort) return;  // (the rows are places in `first`)
+    __shared__ unsigned s_w[KI][KT / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t base = blockIdx.x * (uint64_t)KTILE + threadIdx.x;
+    uint32_t r[KI], c[KI], rank[KI];
+    double v[KI];
+    bool f[KI];
+#pragma unroll
+    for (int k = 0; k < KI; ++k) {
+        const uint64_t i = base + (uint64_t)k * KT;
+        r[k] = i < m ? row[i] : 0u;
+        c[k] = i < m ? col[i] : 0u;
+        v[k] = i < m ? val[i] : 0.0;
+        f[k] = i < m && (i + 1 == m || row[i + 1] != r[k] || col[i + 1] != c[k]) && (keep_zeros || !is_zero(v[k]));
+    }
+#pragma unroll
+    for (int k = 0; k < KI; ++k) {
+        const unsigned b = __ballot_sync(0xffffffffu, f[k]);
+        rank[k] = __popc(b & lane_lt_mask());
+        if (lane == 0) s_w[k][warp] = __popc(b);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned run = 0;
+        for (int k = 0; k < KI; ++k)
+            for (int w = 0; w < KT / 32; ++w) {
+                const unsigned x = s_w[k][w];
+                s_w[k][w] = run;
+                run += x;
+            }
+        if (!out_row) tile_vals[blockIdx.x] = run;
+    }
+    if (!out_row) return;
+    __syncthreads();
+    const uint64_t at = tile_vals[blockIdx.x];
+#pragma unroll
+    for (int k = 0; k < KI; ++k) {
+        const uint64_t i = base + (uint64_t)k * KT, j = at + s_w[k][warp] + rank[k];
+        if (i < m && (i == 0 || row[i - 1] != r[k])) first[r[k]] = j;
+        if (i + 1 == m) first[n] = j + (f[k] ? 1 : 0);
+        if (f[k]) {
+            out_row[j] = r[k];
+            out_col[j] = c[k] & col_mask;
+            out_val[j] = v[k];
+        }
+    }
+}
+
+}  // namespace
+
+int order_huge_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off, const uint32_t *huge,
+                    int cbits, bool keep_zeros, HugeRows *H, uint64_t *count, cudaStream_t s) {
+    const uint64_t n = H->n, m = H->entries, tiles = (m + KTILE - 1) / KTILE;
+    const unsigned gn = grid_for(n, LB, (unsigned)c->n_sms * 8);
+    // stably by (row, column): by both at once where they fit 32 bits
+    const bool both = bits_for(n) + cbits <= 32;
+    const int row_shift = both && n > 1 ? cbits : 63;  // (63: the column alone)
+    StagedSorted by_col, by_row;
+    {
+        DevBuf g, col, row, val;
+        SPG_TRY(g.alloc((n + 1) * sizeof(uint64_t), s));
+        SPG_TRY(col.alloc(m * sizeof(uint32_t), s));
+        SPG_TRY(row.alloc(m * sizeof(uint32_t), s));
+        SPG_TRY(val.alloc(m * sizeof(double), s));
+        huge_lengths<<<gn, LB, 0, s>>>(huge, n, s_off, g.as<uint64_t>());
+        SPG_LAUNCH_CHECK();
+        SPG_TRY(exclusive_scan_u64(c, g.as<uint64_t>(), n, g.as<uint64_t>() + n, s));
+        huge_gather<<<grid_for(m, LB * 8), LB, 0, s>>>(huge, g.as<uint64_t>(), n, s_off, cols, vals,
+                                                     row_shift, col.as<uint32_t>(), row.as<uint32_t>(), val.as<double>());
+        SPG_LAUNCH_CHECK();
+        SPG_TRY(sort_staged_rows(c, col.as<uint32_t>(), row.as<uint32_t>(), val.as<double>(), m,
+                                 both ? bits_for(n) + cbits : cbits, by_col, s));
+    }
+    const DevBuf *row = &by_col.cols, *col = &by_col.rows, *val = &by_col.vals;
+    if (!both) {
+        SPG_TRY(sort_staged_rows(c, row->as<uint32_t>(), col->as<uint32_t>(), val->as<double>(), m, bits_for(n), by_row, s,
+                                 by_col.abort.as<unsigned long long>()));
+        row = &by_row.rows, col = &by_row.cols, val = &by_row.vals;
+    }
+    H->abort = std::move(both ? by_col.abort : by_row.abort);
+    DevBuf tile_vals;
+    SPG_TRY(tile_vals.alloc(tiles * sizeof(uint64_t), s));
+    SPG_TRY(H->first.alloc((n + 1) * sizeof(uint64_t), s));
+    SPG_TRY(H->row.alloc(m * sizeof(uint32_t), s));
+    SPG_TRY(H->cols.alloc(m * sizeof(uint32_t), s));
+    SPG_TRY(H->vals.alloc(m * sizeof(double), s));
+    for (int pass = 0; pass < 2; ++pass) {
+        huge_keep<<<(unsigned)tiles, KT, 0, s>>>(row->as<uint32_t>(), col->as<uint32_t>(), val->as<double>(),
+                                                 both ? (uint32_t)((1ull << cbits) - 1) : 0xFFFFFFFFu, m, keep_zeros, H->abort.as<unsigned long long>(), tile_vals.as<uint64_t>(), n,
+                                                 pass ? H->row.as<uint32_t>() : nullptr, H->cols.as<uint32_t>(),
+                                                 H->vals.as<double>(), H->first.as<uint64_t>());
+        SPG_LAUNCH_CHECK();
+        if (pass == 0) SPG_TRY(exclusive_scan_u64(c, tile_vals.as<uint64_t>(), tiles, nullptr, s));
+    }
+    huge_counts<<<gn, LB, 0, s>>>(huge, n, H->first.as<uint64_t>(), count);
+    SPG_LAUNCH_CHECK();
+    return SPG_OK;
+}
+
+namespace {
+
 // Installs a first lock's CSR built in arrays sized for m entries; when more
 // than an eighth of them stayed unused the entries move to arrays of their
 // own size (build_csr: exact capacity).
@@ -682,8 +829,8 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
     if (m && pre && pre->ready && pre->unsorted && !pre->ungrouped) {
         // Row-grouped inserts (rows non-decreasing, columns in any order, as
         // row-by-row assembly stages them). Two ways to the same CSR:
-        //   tiles    (spg_rowtiles.cu) sort, reduce and write the CSR in one pass,
-        //            whatever the rows' lengths;
+        //   tiles    (spg_rowtiles.cu) sort, reduce and write the CSR in one pass;
+        //            rows above 12 288 entries are sorted apart;
         //   classes  every row is sorted, its last write per column kept unless
         //            zero, and compacted by its length class's kernel, in place
         //            at the row's input positions; a scan of the kept counts
@@ -707,13 +854,7 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
         DevBuf s_off, kept, scols, svals;
         SPG_TRY(staged_offsets(c, pre, rows, m, n, s_off, s));
         bool done = false;
-        if (tiles) {
-            GroupedOut o;
-            SPG_TRY(build_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, cbits, false, abort, &o, &done, s));
-            if (done) return first_install(c, A, std::move(o), m, s);
-            pre->grouped_fits = false;  // a row too long for both ways
-        }
-        if (pre->grouped_fits) {
+        if (!tiles) {
             SPG_TRY(kept.alloc(csr_off_elems(n) * sizeof(uint64_t), s));
             SPG_TRY(scols.alloc(csr_alloc_elems(m) * sizeof(uint32_t), s));
             SPG_TRY(svals.alloc(csr_alloc_elems(m) * sizeof(double), s));
@@ -742,7 +883,13 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
                 SPG_TRY(c->phase_sync(s));
                 return SPG_OK;
             }
+            kept.release();  // (a row too long for the classes)
+            scols.release();
+            svals.release();
         }
+        GroupedOut o;
+        SPG_TRY(build_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, cbits, false, abort, &o, &done, s));
+        if (done) return first_install(c, A, std::move(o), m, s);
     }
     if (m) {
         const unsigned g = grid_for(m, LB, (unsigned)c->n_sms * 16);
@@ -832,7 +979,7 @@ int merge_epoch(Ctx *c, const Csr *A, const uint32_t *rows, const uint32_t *cols
     GroupedOut D;
     bool done = false;
     SPG_TRY(build_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, bits_for(A->n_cols), true, abort, &D, &done, s));
-    if (!done) {  // a row too long for the tiles
+    if (!done) {  // (no memory to sort rows too long for the tiles apart)
         Delta d;
         SPG_TRY(sort_dedup(c, rows, cols, vals, m, n, A->n_cols, d, s));
         SPG_TRY(launch_row_offsets(c, d.row.as<uint32_t>(), d.u, n, D.off.as<uint64_t>(), s));

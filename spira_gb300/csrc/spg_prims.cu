@@ -493,6 +493,7 @@ __global__ void __launch_bounds__(256) seg_place(const uint32_t *__restrict__ co
                                                  uint64_t n_rows, int cbits, const unsigned *__restrict__ ctr,
                                                  unsigned *__restrict__ cur, uint32_t *__restrict__ lists, SegOut o) {
     __shared__ unsigned sc[10], sbase[10], base[10];
+    if (ctr[SC_OVERFLOW]) return;  // (set by the launch before: the rest of the plan would be thrown away)
     if (threadIdx.x == 0) {
         base[6] = 0;
         for (int c = 7; c <= 9; ++c) base[c] = base[c - 1] + ctr[SC_LIST + c - 1];
@@ -601,7 +602,9 @@ __device__ __forceinline__ void sort_short_class(const uint32_t *__restrict__ co
 // us; two 104, eight 125 for the registers). Finding a class's g-th row in its
 // ballot with __fns and one row per segment at a time took 130.
 __global__ void __launch_bounds__(256) seg_short_sort(const uint32_t *__restrict__ cols,
-                                                      const uint64_t *__restrict__ s_off, uint64_t n_rows, SegOut o) {
+                                                      const uint64_t *__restrict__ s_off, uint64_t n_rows,
+                                                      const unsigned *__restrict__ ctr, SegOut o) {
+    if (ctr[SC_OVERFLOW]) n_rows = 0;  // (leaving here instead: 5 % of the kernel)
     __shared__ uint8_t s_ord[256 / 32][32];  // the warp's lanes by class
     const int lane = threadIdx.x & 31;
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
@@ -726,7 +729,7 @@ __global__ void __launch_bounds__(256, sizeof(K) == 8 ? 2 : 4) seg_medium_sort(c
                                                        const uint64_t *__restrict__ s_off,
                                                        const uint32_t *__restrict__ lists,
                                                        const unsigned *__restrict__ ctr, int cbits, SegOut o) {
-    const unsigned n = ctr[SC_LIST + 6];  // class 6 heads the lists
+    const unsigned n = ctr[SC_OVERFLOW] ? 0 : ctr[SC_LIST + 6];  // class 6 heads the lists
     const int lane = threadIdx.x & 31;
     const unsigned warps = gridDim.x * (blockDim.x >> 5);
     for (unsigned k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < n; k += warps) {
@@ -981,7 +984,7 @@ int seg_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, uint64_t m, ui
     SPG_LAUNCH_CHECK();
     seg_place<<<gr, 256, 0, s>>>(cols, s_off, n_rows, cbits, ctr, cur, lists, o);
     SPG_LAUNCH_CHECK();
-    seg_short_sort<<<grid_for((n_rows + 31) / 32, 8, (unsigned)c->n_sms * 16), 256, 0, s>>>(cols, s_off, n_rows, o);
+    seg_short_sort<<<grid_for((n_rows + 31) / 32, 8, (unsigned)c->n_sms * 16), 256, 0, s>>>(cols, s_off, n_rows, ctr, o);
     SPG_LAUNCH_CHECK();
     // (8 blocks per SM: twice what fits at once, which balanced rows of
     // unequal length better than one wave)

@@ -263,7 +263,7 @@ RsLaunch rs_launch_of(int bits) {
 }  // namespace
 
 int sort_staged_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const double *vals, uint64_t m, int rbits,
-                     StagedSorted &out, cudaStream_t s) {
+                     StagedSorted &out, cudaStream_t s, const unsigned long long *earlier) {
     const int passes = std::max(1, (rbits + 7) / 8), bits = std::max(5, (rbits + passes - 1) / passes);
     // tiles of RS_LT x RS_LI entries; of 1024 while the larger ones are fewer than
     // two for three SMs (first lock in random order into 1 M rows, large / small:
@@ -277,7 +277,8 @@ int sort_staged_rows(Ctx *c, const uint32_t *rows, const uint32_t *cols, const d
     unsigned long long *hist = work.as<unsigned long long>(), *ticket = hist + passes * RS_RADIX,
                        *state = ticket + passes;
     SPG_TRY(out.abort.alloc(sizeof(unsigned long long), s));
-    SPG_CUDA_TRY(cudaMemsetAsync(out.abort.ptr, 0, sizeof(unsigned long long), s));
+    if (earlier) SPG_CUDA_TRY(cudaMemcpyAsync(out.abort.ptr, earlier, sizeof(*earlier), cudaMemcpyDeviceToDevice, s));
+    else SPG_CUDA_TRY(cudaMemsetAsync(out.abort.ptr, 0, sizeof(unsigned long long), s));
     SPG_TRY(out.rows.alloc(m * sizeof(uint32_t), s));
     SPG_TRY(out.cols.alloc(csr_alloc_elems(m) * sizeof(uint32_t), s));  // (a CSR's arrays, for the transpose)
     SPG_TRY(out.vals.alloc(csr_alloc_elems(m) * sizeof(double), s));

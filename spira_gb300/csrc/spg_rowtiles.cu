@@ -22,7 +22,12 @@
 //      the CSR, consecutive threads on consecutive entries.
 // Rows of more than RT_CAP entries are ordered beforehand by larger blocks
 // (the same steps, two sizes) into scratch at their input positions; their
-// tiles copy.
+// tiles copy. Rows of more than RT_BIG entries fit no block: when the plan
+// meets some, the kernels stop, those rows' entries alone are sorted by column
+// (order_huge_rows), and a second run gives each its place, where a pass over
+// all of them puts their entries (10 M shuffled inserts, five to a row, with one
+// row of 20 000: 0.79 ms, 0.70 without it; all of them sorted by (row, column)
+// 1.24, and 1.59 when the row sort and the tiles had been tried before that).
 //
 // Floor: 24 bytes per entry of HBM traffic (12 in, 12 out). Bound: latency
 // between the fifteen barriers of a tile, at 60 % of the issue slots: on the
@@ -54,7 +59,7 @@ constexpr int RT_LIM = 32;              // longest bucket ordered by counting
 constexpr unsigned RT_STATUS_TIMEOUT = 0x20u;
 
 // Counters at the head of the scratch words.
-enum : int { RC_PLAN_TICKET = 0, RC_TICKET = 1, RC_TILES = 2, RC_BIG = 3, RC_OVERFLOW = 4, RC_MID = 5, RC_MID_TICKET = 6, RC_BIG_TICKET = 7, RC_N = 8 };
+enum : int { RC_PLAN_TICKET = 0, RC_TICKET = 1, RC_TILES = 2, RC_BIG = 3, RC_OVERFLOW = 4, RC_MID = 5, RC_MID_TICKET = 6, RC_BIG_TICKET = 7, RC_HUGE = 8, RC_HUGE_ENTRIES = 9, RC_N = 10 };
 
 struct RtArgs {
     const uint32_t *cols;
@@ -68,6 +73,8 @@ struct RtArgs {
     uint64_t *tile_start;  // first row of each tile, then n_rows (2^32 in the transpose of a matrix of 2^32 columns)
     uint32_t *longer;      // rows of RT_CAP+1 .. RT_MID entries from the front, longer ones from the back
     uint64_t n_longer;
+    uint32_t *huge;        // rows of more than RT_BIG entries
+    bool huge_ready;       // they are ordered: off[r] holds such a row's kept count
     uint32_t *big_cols;    // their ordered entries, at the rows' input positions
     double *big_vals;
     uint64_t *off;         // out; off[r] holds a big row's kept count until its tile is written
@@ -75,7 +82,7 @@ struct RtArgs {
     double *out_vals;
     const unsigned long long *abort;  // may be null: the inputs are not to be read if set
     unsigned int *status;
-    unsigned long long *words;  // [0] 1: a row is too long, nothing is built; [1] entries kept
+    unsigned long long *words;  // [0] 1: rows too long are listed, nothing is built; [1] entries kept, or such rows; [2] their entries
 };
 
 // ---------------------------------------------------------------- tile plan
@@ -122,9 +129,16 @@ __global__ void __launch_bounds__(RP_T) rt_plan(RtArgs a) {
         if (e == r) {  // longer than a tile
             const uint64_t L = s_off[r + 1] - s_off[r];
             if (lane == 0) {
-                if (L > (uint64_t)RT_BIG) a.ctr[RC_OVERFLOW] = 1ull;
-                else if (L > (uint64_t)RT_MID) a.longer[a.n_longer - 1 - atomicAdd(a.ctr + RC_BIG, 1ull)] = (uint32_t)(r0 + r);
-                else a.longer[atomicAdd(a.ctr + RC_MID, 1ull)] = (uint32_t)(r0 + r);
+                if (L > (uint64_t)RT_BIG) {
+                    if (!a.huge_ready) {
+                        a.ctr[RC_OVERFLOW] = 1ull;
+                        a.huge[atomicAdd(a.ctr + RC_HUGE, 1ull)] = (uint32_t)(r0 + r);
+                        atomicAdd(a.ctr + RC_HUGE_ENTRIES, (unsigned long long)L);
+                    }
+                } else if (L > (uint64_t)RT_MID) a.longer[a.n_longer - 1 - atomicAdd(a.ctr + RC_BIG, 1ull)] = (uint32_t)(r0 + r);
+                else {
+                    a.longer[atomicAdd(a.ctr + RC_MID, 1ull)] = (uint32_t)(r0 + r);
+                }
             }
             ++e;
         }
@@ -192,6 +206,7 @@ struct RtSmem : RtArrays<CAP, APART> {
     struct Tile {
         uint64_t id, r0, r1, s0, s1;  // its rows and their entries
         uint32_t total;               // kept entries
+        uint32_t copied;              // of a longer row: those that its tile copies
     } tile[3];  // this one, the one before (sorted, not yet written) and the next
 };
 
@@ -547,7 +562,11 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
     auto &S = *reinterpret_cast<RtSmem<T, CAP, true> *>(rt_raw);
     const int t = threadIdx.x;
     if (a.ctr[RC_OVERFLOW]) {
-        if (blockIdx.x == 0 && t == 0) store_word(a.words, 0, 1ull);
+        if (blockIdx.x == 0 && t == 0) {
+            store_word(a.words, 0, 1ull);
+            store_word(a.words, 1, a.ctr[RC_HUGE]);
+            store_word(a.words, 2, a.ctr[RC_HUGE_ENTRIES]);
+        }
         return;
     }
     const uint64_t n_tiles = a.ctr[RC_TILES];
@@ -578,6 +597,7 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
                 total = rt_order<T, CAP, true>(S, c, a.vals + s0, E, a.cbits, a.keep_zeros, o, v);
             } else {
                 total = (uint32_t)a.off[r0];
+                if (t == 0) cur.copied = cur.s1 - cur.s0 <= (uint64_t)RT_BIG ? total : 0;  // (the others by rt_huge_rows)
             }
             if (t == 0) {
                 cur.total = total;
@@ -600,19 +620,20 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
                 }
             } else {  // one row, eight loads of a thread in flight (one pair at a time: 55 us more on the Zipf matrix)
                 constexpr int U = 4;
-                for (uint32_t k0 = t; k0 < n; k0 += U * T) {
+                const uint32_t copied = prev.copied;
+                for (uint32_t k0 = t; k0 < copied; k0 += U * T) {
                     uint32_t cc[U];
                     double vv[U];
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         const uint32_t k = k0 + u * T;
-                        cc[u] = k < n ? a.big_cols[prev.s0 + k] : 0u;
-                        vv[u] = k < n ? a.big_vals[prev.s0 + k] : 0.0;
+                        cc[u] = k < copied ? a.big_cols[prev.s0 + k] : 0u;
+                        vv[u] = k < copied ? a.big_vals[prev.s0 + k] : 0.0;
                     }
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         const uint32_t k = k0 + u * T;
-                        if (k < n) {
+                        if (k < copied) {
                             a.out_cols[base + k] = cc[u];
                             a.out_vals[base + k] = vv[u];
                         }
@@ -649,6 +670,51 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
     }
 }
 
+// The kept entries of the rows that fit no block, to their rows' places.
+__global__ void __launch_bounds__(256)
+rt_huge_rows(const uint32_t *__restrict__ huge, const uint32_t *__restrict__ row, const uint32_t *__restrict__ cols,
+             const double *__restrict__ vals, const uint64_t *__restrict__ first, uint64_t n_huge,
+             const unsigned int *status, const uint64_t *__restrict__ off, uint32_t *__restrict__ out_cols,
+             double *__restrict__ out_vals) {
+    __shared__ unsigned int gave_up;
+    if (threadIdx.x == 0) gave_up = *(const volatile unsigned int *)status;
+    __syncthreads();
+    if (gave_up) return;  // a wait of the tiles: not every place is known
+    const uint64_t n = first[n_huge];
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t q = row[i];
+        const uint64_t o = off[huge[q]] + (i - first[q]);
+        out_cols[o] = cols[i];
+        out_vals[o] = vals[i];
+    }
+}
+
+// Plan, longer rows, tiles.
+int rt_run(Ctx *c, const RtArgs &a, uint64_t plan_tiles, uint64_t t_max, uint64_t m, cudaStream_t s) {
+    rt_plan<<<(unsigned)plan_tiles, RP_T, 0, s>>>(a);
+    SPG_LAUNCH_CHECK();
+    if (m > (uint64_t)RT_CAP) {
+        auto k = rt_long_rows<RT_MID_T, RT_MID, RT_MID_PER_SM, RC_MID, RC_MID_TICKET>;
+        constexpr size_t smem = sizeof(RtSmem<RT_MID_T, RT_MID, false>);
+        SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k<<<(unsigned)std::min<uint64_t>(a.n_longer, (uint64_t)c->n_sms * RT_MID_PER_SM), RT_MID_T, smem, s>>>(a);
+        SPG_LAUNCH_CHECK();
+    }
+    if (m > (uint64_t)RT_MID) {
+        auto k = rt_long_rows<RT_BIG_T, RT_BIG, 1, RC_BIG, RC_BIG_TICKET>;
+        constexpr size_t smem = sizeof(RtSmem<RT_BIG_T, RT_BIG, false>);
+        SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k<<<(unsigned)std::min<uint64_t>(m / (RT_MID + 1), (uint64_t)c->n_sms), RT_BIG_T, smem, s>>>(a);
+        SPG_LAUNCH_CHECK();
+    }
+    constexpr size_t smem = sizeof(RtSmem<RT_T, RT_CAP, true>);
+    SPG_CUDA_TRY(cudaFuncSetAttribute(rt_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned blocks = (unsigned)std::min<uint64_t>(t_max, (uint64_t)c->n_sms * RT_PER_SM);
+    rt_tiles<<<blocks, RT_T, smem, s>>>(a);
+    SPG_LAUNCH_CHECK();
+    return SPG_OK;
+}
+
 }  // namespace
 
 int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off,
@@ -659,7 +725,7 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     // two neighbouring tiles of one part hold more than RT_CAP entries together
     const uint64_t t_max = 2 * (m / RT_CAP) + 2 * (plan_tiles + m / RP_PART) + 4;
     const bool may_long = m > (uint64_t)RT_CAP;
-    const uint64_t n_long = m / (RT_CAP + 1) + 1;
+    const uint64_t n_long = m / (RT_CAP + 1) + 1, n_huge = m / (RT_BIG + 1);
     DevBuf state, tiles, longer, big_cols, big_vals;
     // (the outputs first: the scratch below is a little smaller, and took the
     // freed outputs of an earlier lock when it came first, so that the pool
@@ -667,10 +733,11 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     SPG_TRY(out->off.alloc(csr_off_elems(n_rows) * sizeof(uint64_t), s));
     SPG_TRY(out->cols.alloc(csr_alloc_elems(m) * sizeof(uint32_t), s));
     SPG_TRY(out->vals.alloc(csr_alloc_elems(m) * sizeof(double), s));
-    SPG_TRY(state.alloc((RC_N + plan_tiles + t_max) * sizeof(unsigned long long), s));
-    SPG_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, (RC_N + plan_tiles + t_max) * sizeof(unsigned long long), s));
+    const size_t state_bytes = (RC_N + plan_tiles + t_max) * sizeof(unsigned long long);
+    SPG_TRY(state.alloc(state_bytes, s));
+    SPG_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, state_bytes, s));
     SPG_TRY(tiles.alloc((t_max + 1) * sizeof(uint64_t), s));
-    SPG_TRY(longer.alloc(n_long * sizeof(uint32_t), s));
+    SPG_TRY(longer.alloc((n_long + n_huge) * sizeof(uint32_t), s));
     if (may_long) {
         SPG_TRY(big_cols.alloc(m * sizeof(uint32_t), s));
         SPG_TRY(big_vals.alloc(m * sizeof(double), s));
@@ -688,6 +755,7 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     a.tile_start = tiles.as<uint64_t>();
     a.longer = longer.as<uint32_t>();
     a.n_longer = n_long;
+    a.huge = a.longer + n_long;
     a.big_cols = big_cols.as<uint32_t>();
     a.big_vals = big_vals.as<double>();
     a.off = out->off.as<uint64_t>();
@@ -696,30 +764,31 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     a.abort = abort;
     a.status = c->d_status;
     a.words = c->d_words;
-    rt_plan<<<(unsigned)plan_tiles, RP_T, 0, s>>>(a);
-    SPG_LAUNCH_CHECK();
-    if (may_long) {
-        auto k = rt_long_rows<RT_MID_T, RT_MID, RT_MID_PER_SM, RC_MID, RC_MID_TICKET>;
-        constexpr size_t smem = sizeof(RtSmem<RT_MID_T, RT_MID, false>);
-        SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<(unsigned)std::min<uint64_t>(n_long, (uint64_t)c->n_sms * RT_MID_PER_SM), RT_MID_T, smem, s>>>(a);
+    HugeRows H;
+    while (true) {
+        SPG_TRY(rt_run(c, a, plan_tiles, t_max, m, s));
+        if (a.huge_ready)
+            rt_huge_rows<<<grid_for(H.entries, 256, (unsigned)c->n_sms * 8), 256, 0, s>>>(
+                a.huge, H.row.as<uint32_t>(), H.cols.as<uint32_t>(), H.vals.as<double>(), H.first.as<uint64_t>(), H.n,
+                a.status, a.off, a.out_cols, a.out_vals);
         SPG_LAUNCH_CHECK();
+        SPG_TRY(c->phase_sync(s));
+        if (c->word(0) == 0) break;
+        H.n = c->word(1);
+        H.entries = c->word(2);
+        // mostly such rows, and grouped as they came: the global sort (300 rows of
+        // 13 000 in 5 M columns 0.45 ms, apart 0.58); rows sorted before are no
+        // use to it (one such row in 100 k of ten, shuffled: 0.39 / 0.30)
+        if (!abort && 2 * H.entries > m) return SPG_OK;
+        const int rc = order_huge_rows(c, cols, vals, s_off, a.huge, cbits, keep_zeros, &H, a.off, s);
+        if (rc == SPG_ERR_NO_MEMORY) return SPG_OK;  // (the global sort needs less)
+        SPG_TRY(rc);
+        SPG_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, state_bytes, s));
+        a.huge_ready = true;
+        a.abort = H.abort.as<unsigned long long>();  // (the staged rows' own is clear, or the wait above had failed)
     }
-    if (m > (uint64_t)RT_MID) {
-        auto k = rt_long_rows<RT_BIG_T, RT_BIG, 1, RC_BIG, RC_BIG_TICKET>;
-        constexpr size_t smem = sizeof(RtSmem<RT_BIG_T, RT_BIG, false>);
-        SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<(unsigned)std::min<uint64_t>(m / (RT_MID + 1), (uint64_t)c->n_sms), RT_BIG_T, smem, s>>>(a);
-        SPG_LAUNCH_CHECK();
-    }
-    constexpr size_t smem = sizeof(RtSmem<RT_T, RT_CAP, true>);
-    SPG_CUDA_TRY(cudaFuncSetAttribute(rt_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned blocks = (unsigned)std::min<uint64_t>(t_max, (uint64_t)c->n_sms * RT_PER_SM);
-    rt_tiles<<<blocks, RT_T, smem, s>>>(a);
-    SPG_LAUNCH_CHECK();
-    SPG_TRY(c->phase_sync(s));
-    *done = c->word(0) == 0;
-    out->n = *done ? c->word(1) : 0;
+    *done = true;
+    out->n = c->word(1);
     return SPG_OK;
 }
 

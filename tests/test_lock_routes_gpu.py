@@ -28,3 +28,57 @@ def test_lock_many_clustered_rows_of_wide_columns(ctx):
         A = sg.Csr(ctx, n, n_cols)
         A.lock(*e)
         assert_csr_equal(A.download(), oracle.lock_epochs(n, n_cols, [e]))
+
+
+def _hub_inserts(n_rows, n_cols, hubs, seed, per_row=3):
+    """per_row inserts into every row and, at `hubs`' rows, so many more."""
+    L = np.full(n_rows, per_row, np.int64)
+    for r, k in hubs:
+        L[r] += k
+    rows = np.repeat(np.arange(n_rows, dtype=np.uint32), L)
+    ctr = np.arange(len(rows), dtype=np.uint64)
+    vals = gen.sym_unit(gen.hash3(seed, 2, ctr))
+    vals[::7] = 0.0
+    vals[::101] = np.nan
+    return rows, gen.below(gen.hash3(seed, 1, ctr), n_cols), vals
+
+
+@pytest.mark.parametrize("order", ["grouped", "any"])
+@pytest.mark.parametrize("n_rows,n_cols,hubs", [
+    (900, 5000, [(0, 12_285)]),                              # 12 288 entries: still a block's
+    (900, 5000, [(0, 12_286)]),                              # one more, on few columns
+    (900, (1 << 32) - 5, [(899, 20_000)]),                   # the widest columns, the last row
+    (900, 1, [(450, 30_000)]),                               # one column: one entry is left
+    (3000, 400_000, [(0, 15_000), (1, 13_000), (2500, 40_961), (2999, 12_286)]),
+    (40, 70_000, [(r, 13_000 + r) for r in range(40)]),      # nothing but such rows
+])
+def test_lock_rows_longer_than_a_block(ctx, n_rows, n_cols, hubs, order):
+    """Rows above 12 288 entries are sorted apart and put between the others,
+    in a first lock and in a later one (whose zeros delete)."""
+    epochs = []
+    for seed in (1, 2):
+        e = _hub_inserts(n_rows, n_cols, hubs, seed)
+        if order == "any":
+            p = np.argsort(gen.hash3(seed, 3, np.arange(len(e[0]), dtype=np.uint64)), kind="stable")
+            e = tuple(x[p] for x in e)
+        epochs.append(e)
+    A = sg.Csr(ctx, n_rows, n_cols)
+    for k in (1, 2):
+        A.lock(*epochs[k - 1])
+        assert_csr_equal(A.download(), oracle.lock_epochs(n_rows, n_cols, epochs[:k]))
+
+
+def test_lock_hub_row_among_clustered_rows(ctx):
+    """More than the few-inserts rule, short rows of near columns (the row
+    classes' case) and one row that they cannot take."""
+    n = 1_100_000
+    rows = np.repeat(np.arange(n, dtype=np.uint32), 4)
+    ctr = np.arange(len(rows), dtype=np.uint64)
+    cols = ((rows + gen.hash3(8, 1, ctr) % np.uint64(6)) % np.uint64(n)).astype(np.uint32)
+    hub = np.full(13_000, 77, np.uint32)
+    k = np.arange(len(hub), dtype=np.uint64)
+    e = (np.insert(rows, 77 * 4, hub), np.insert(cols, 77 * 4, gen.below(gen.hash3(8, 2, k), n)),
+         gen.sym_unit(gen.hash3(8, 3, np.arange(len(rows) + len(hub), dtype=np.uint64))))
+    A = sg.Csr(ctx, n, n)
+    A.lock(*e)
+    assert_csr_equal(A.download(), oracle.lock_epochs(n, n, [e]))
