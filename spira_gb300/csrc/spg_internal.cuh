@@ -565,7 +565,8 @@ int merge_small_delta(Ctx *c, const CsrView &A, uint64_t n_rows, const uint32_t 
                       uint32_t *cols_out, double *vals_out, uint64_t *nnz, uint64_t *u, bool *done, cudaStream_t s);
 // Row-grouped entries (row r's are [s_off[r], s_off[r+1]), columns in any
 // order) as CSR: the last write of every key in (row, column) order, zeros
-// dropped unless keep_zeros (spg_rowtiles.cu). The output arrays are sized
+// dropped unless keep_zeros (spg_rowtiles.cu). near: most entries' columns lie
+// near their row's others (a choice of kernels). The output arrays are sized
 // for m entries; n of them are used. *done = false when there are rows of more
 // than 12 288 entries and no memory to sort those apart; the outputs are then
 // undefined.
@@ -574,8 +575,8 @@ struct GroupedOut {
     uint64_t n = 0;
 };
 int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off,
-                       uint64_t m, uint64_t n_rows, int cbits, bool keep_zeros, const unsigned long long *abort,
-                       GroupedOut *out, bool *done, cudaStream_t s);
+                       uint64_t m, uint64_t n_rows, int cbits, bool near, bool keep_zeros,
+                       const unsigned long long *abort, GroupedOut *out, bool *done, cudaStream_t s);
 
 // Its rows of more than 12 288 entries, which no block takes: the n of them in
 // huge[], `entries` in all, as (place in huge[], column, value) in order, reduced

@@ -888,7 +888,8 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
             svals.release();
         }
         GroupedOut o;
-        SPG_TRY(build_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, cbits, false, abort, &o, &done, s));
+        SPG_TRY(build_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, cbits, pre->clustered > 0, false, abort, &o, &done,
+                                   s));
         if (done) return first_install(c, A, std::move(o), m, s);
     }
     if (m) {
@@ -978,7 +979,8 @@ int merge_epoch(Ctx *c, const Csr *A, const uint32_t *rows, const uint32_t *cols
     // the epoch's last writes, zeros kept (they delete), in (row, column) order
     GroupedOut D;
     bool done = false;
-    SPG_TRY(build_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, bits_for(A->n_cols), true, abort, &D, &done, s));
+    SPG_TRY(build_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, bits_for(A->n_cols), pre->clustered > 0, true, abort,
+                               &D, &done, s));
     if (!done) {  // (no memory to sort rows too long for the tiles apart)
         Delta d;
         SPG_TRY(sort_dedup(c, rows, cols, vals, m, n, A->n_cols, d, s));

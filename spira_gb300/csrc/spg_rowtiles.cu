@@ -12,7 +12,9 @@
 //      shared-memory counter per bucket ranks the arrivals, one scan turns
 //      the counters into slots. Buckets of more than RT_LIM entries (columns
 //      clustered in a long row, or many duplicates) are split again over
-//      their own column range until none is left;
+//      their own column range until none is left. A long row with more entries
+//      than columns in its range needs none of this: a cell per column takes
+//      the last position;
 //   3. an entry's sorted place is its bucket's first slot plus the bucket's
 //      entries before it by (column, input position): a few compares, for
 //      four entries at a time;
@@ -56,6 +58,7 @@ constexpr int RT_BIG = 12288, RT_BIG_T = 1024;                   // ... and for 
 // on 200 columns 265 us, 222 at 32; rows of 40 uniform columns 387 / 425).
 constexpr int RT_LONG = 32;
 constexpr int RT_LIM = 32;              // longest bucket ordered by counting
+constexpr int RT_FEW_CBITS = 14;
 constexpr unsigned RT_STATUS_TIMEOUT = 0x20u;
 
 // Counters at the head of the scratch words.
@@ -267,7 +270,7 @@ __device__ __forceinline__ void rt_minmax(Smem &S, uint32_t lo, bool on, uint32_
 // value is zero, and returns the number kept (in every thread). S.keep / kpre
 // have the keep bits by sorted place; o[i] is the kept entry's index among the
 // kept ones, or ~0 for a dropped one; v[i] its value.
-template <int T, int CAP, bool APART>
+template <bool REPEATS, int T, int CAP, bool APART>
 __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uint32_t (&c)[CAP / T],
                                              const double *__restrict__ vals, int E, int cbits, bool keep_zeros,
                                              uint32_t (&pk)[CAP / T], double (&v)[CAP / T]) {
@@ -289,27 +292,45 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
             hi = above ? 32 * w + __ffs((int)above) - 1 : 32 * w + 32 >= E ? E : S.wend[w];
         }
         pk[i] = lo << 16 | hi;
-        rt_minmax(S, lo, hi - lo > (uint32_t)RT_LONG, c[i], lane);
+        const bool long_row = hi - lo > (uint32_t)RT_LONG;
+        if (REPEATS && long_row && e >= (int)lo + 2) S.scol[e] = 0;
+        rt_minmax(S, lo, long_row, c[i], lane);
     }
     __syncthreads();
+    // bit i: entry i has a later write (found below); bit 16 + i (REPEATS only):
+    // its row has more entries than columns in its range, and a cell of S.scol
+    // for each of them (from the third on), which takes the greatest position:
+    // nothing else of such a row is kept, and its place is its column
+    uint32_t flags = 0;
+    auto exact = [&](int i) { return REPEATS && ((flags >> (16 + i)) & 1u); };
+    static_assert(I <= 16, "two bits per entry");
 #pragma unroll
     for (int i = 0; i < I; ++i) {
-        if (t + i * T < E) {
+        const int e = t + i * T;
+        if (e < E) {
             const uint32_t lo = pk[i] >> 16, L = (pk[i] & 0xFFFFu) - lo;
             uint32_t x = c[i] << shift;
             if (L > (uint32_t)RT_LONG) {
-                const uint32_t mn = S.scol[lo];
-                x = (c[i] - mn) << min(31, __clz((int)(S.scol[lo + 1] - mn)));
+                const uint32_t mn = S.scol[lo], range = S.scol[lo + 1] - mn;
+                if (REPEATS && range < L - 2) {
+                    const uint32_t f = lo + (c[i] - mn);
+                    atomicMax(&S.scol[f + 2], (uint32_t)e + 1);
+                    pk[i] = f << 16 | f;
+                    flags |= 0x10000u << i;
+                    continue;
+                }
+                x = (c[i] - mn) << min(31, __clz((int)range));
             }
             pk[i] = lo + __umulhi(x, L);
         }
     }
-    uint32_t dropped = 0;  // bit i: entry i has a later write (found below)
     // pk: bucket; after counting, bucket << 16 | rank of arrival
     while (true) {
 #pragma unroll
         for (int i = 0; i < I; ++i) {
-            if (t + i * T < E) {
+            if (exact(i)) {  // (so that the other rows' slots start at their first entries)
+                atomicAdd(&S.cnt[(t + i * T) >> 1], 1u << (((t + i * T) & 1) * 16));
+            } else if (t + i * T < E) {
                 const uint32_t sh = (pk[i] & 1u) * 16u;
                 const uint32_t v = atomicAdd(&S.cnt[pk[i] >> 1], 1u << sh);
                 pk[i] = pk[i] << 16 | ((v >> sh) & 0xFFFFu);
@@ -350,7 +371,7 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
         // last position and that entry's arrival rank.
 #pragma unroll
         for (int i = 0; i < I; ++i) {
-            if (t + i * T < E && (pk[i] & 0xFFFFu) == 0) {
+            if (t + i * T < E && !exact(i) && (pk[i] & 0xFFFFu) == 0) {
                 const uint32_t lo = cnt16[pk[i] >> 16], len = cnt16[(pk[i] >> 16) + 1] - lo;
                 if (len > (uint32_t)RT_LIM) {
                     S.scol[lo] = 0xFFFFFFFFu;
@@ -363,7 +384,7 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
 #pragma unroll
         for (int i = 0; i < I; ++i) {
             uint32_t lo = 0, len = 0;
-            if (t + i * T < E) {
+            if (t + i * T < E && !exact(i)) {
                 lo = cnt16[pk[i] >> 16];
                 len = cnt16[(pk[i] >> 16) + 1] - lo;
             }
@@ -376,7 +397,7 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < I; ++i) {
-            if (t + i * T < E) {
+            if (t + i * T < E && !exact(i)) {
                 const uint32_t lo = cnt16[pk[i] >> 16], len = cnt16[(pk[i] >> 16) + 1] - lo;
                 if (len > (uint32_t)RT_LIM && S.scol[lo + 2] == (uint32_t)(t + i * T)) S.scol[lo + 3] = pk[i] & 0xFFFFu;
             }
@@ -384,7 +405,7 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < I; ++i) {
-            if (t + i * T < E) {
+            if (t + i * T < E && !exact(i)) {
                 const uint32_t lo = cnt16[pk[i] >> 16], len = cnt16[(pk[i] >> 16) + 1] - lo;
                 uint32_t b = lo;  // a short bucket keeps its slots: they are its own
                 if (len > (uint32_t)RT_LIM) {
@@ -394,7 +415,7 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
                     } else {
                         const uint32_t r = pk[i] & 0xFFFFu, last = S.scol[lo + 3];
                         b = lo + (r == last ? len - 1 : r > last ? r - 1 : r);
-                        if (r != last) dropped |= 1u << i;
+                        if (r != last) flags |= 1u << i;
                     }
                 }
                 pk[i] = b;
@@ -408,7 +429,9 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
 #pragma unroll
     for (int i = 0; i < I; ++i) {
         const int e = t + i * T;
-        if (e < E) {
+        if (exact(i)) {
+            if (S.scol[(pk[i] & 0xFFFFu) + 2] != (uint32_t)e + 1) flags |= 1u << i;
+        } else if (e < E) {
             const uint32_t b = pk[i] >> 16, lo = cnt16[b], hi = cnt16[b + 1];
             S.scol[lo + (pk[i] & 0xFFFFu)] = c[i];
             S.spos[lo + (pk[i] & 0xFFFFu)] = (uint16_t)e;
@@ -461,7 +484,7 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
             if (e < E) {
                 const uint32_t lo = pk[i] >> 16, hi = pk[i] & 0xFFFFu;
                 uint32_t f = lo + (acc[g] & 0xFFFFu);
-                bool kept = !((dropped >> i) & 1u) && (keep_zeros || !is_zero(v[i]));
+                bool kept = !((flags >> i) & 1u) && (keep_zeros || !is_zero(v[i]));
                 if (acc[g] >= 0x20000u) {
                     for (uint32_t j = lo; j < hi; ++j) {
                         if (S.scol[j] == c[i]) {
@@ -506,7 +529,7 @@ __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uin
 
 // Rows longer than a tile, a block each (taken from the list one by one):
 // ordered and compacted into scratch at the row's input positions.
-template <int T, int CAP, int PER_SM, int COUNT, int TICKET>
+template <int T, int CAP, int PER_SM, int COUNT, int TICKET, bool REPEATS>
 __global__ void __launch_bounds__(T, PER_SM) rt_long_rows(RtArgs a) {
     constexpr int I = CAP / T;
     __shared__ uint64_t s_next;
@@ -532,7 +555,7 @@ __global__ void __launch_bounds__(T, PER_SM) rt_long_rows(RtArgs a) {
         }
         if (t < 2) S.scol[t] = t == 0 ? 0xFFFFFFFFu : 0u;  // the row's cells
         for (int w = t; w < E / 2 + 1; w += T) S.cnt[w] = 0;
-        const uint32_t total = rt_order<T, CAP, false>(S, c, a.vals + s0, E, a.cbits, a.keep_zeros, o, v);
+        const uint32_t total = rt_order<REPEATS, T, CAP, false>(S, c, a.vals + s0, E, a.cbits, a.keep_zeros, o, v);
 #pragma unroll
         for (int i = 0; i < I; ++i) {
             if (t + i * T < E && o[i] != ~0u) {
@@ -556,6 +579,7 @@ __global__ void __launch_bounds__(T, PER_SM) rt_long_rows(RtArgs a) {
 // rest). So a block publishes a sorted tile's count, keeps its entries in
 // shared memory and sorts the next tile before it writes this one, whose
 // place is known by then.
+template <bool REPEATS>
 __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
     constexpr int T = RT_T, CAP = RT_CAP, I = CAP / T;
     extern __shared__ __align__(16) unsigned char rt_raw[];
@@ -594,7 +618,7 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
                     const uint64_t b = a.s_off[r], e = a.s_off[r + 1];
                     if (b != e) rt_mark_row(S, (int)(b - s0), (int)(e - s0));
                 }
-                total = rt_order<T, CAP, true>(S, c, a.vals + s0, E, a.cbits, a.keep_zeros, o, v);
+                total = rt_order<REPEATS, T, CAP, true>(S, c, a.vals + s0, E, a.cbits, a.keep_zeros, o, v);
             } else {
                 total = (uint32_t)a.off[r0];
                 if (t == 0) cur.copied = cur.s1 - cur.s0 <= (uint64_t)RT_BIG ? total : 0;  // (the others by rt_huge_rows)
@@ -690,27 +714,28 @@ rt_huge_rows(const uint32_t *__restrict__ huge, const uint32_t *__restrict__ row
 }
 
 // Plan, longer rows, tiles.
+template <bool REPEATS>
 int rt_run(Ctx *c, const RtArgs &a, uint64_t plan_tiles, uint64_t t_max, uint64_t m, cudaStream_t s) {
     rt_plan<<<(unsigned)plan_tiles, RP_T, 0, s>>>(a);
     SPG_LAUNCH_CHECK();
     if (m > (uint64_t)RT_CAP) {
-        auto k = rt_long_rows<RT_MID_T, RT_MID, RT_MID_PER_SM, RC_MID, RC_MID_TICKET>;
+        auto k = rt_long_rows<RT_MID_T, RT_MID, RT_MID_PER_SM, RC_MID, RC_MID_TICKET, REPEATS>;
         constexpr size_t smem = sizeof(RtSmem<RT_MID_T, RT_MID, false>);
         SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k<<<(unsigned)std::min<uint64_t>(a.n_longer, (uint64_t)c->n_sms * RT_MID_PER_SM), RT_MID_T, smem, s>>>(a);
         SPG_LAUNCH_CHECK();
     }
     if (m > (uint64_t)RT_MID) {
-        auto k = rt_long_rows<RT_BIG_T, RT_BIG, 1, RC_BIG, RC_BIG_TICKET>;
+        auto k = rt_long_rows<RT_BIG_T, RT_BIG, 1, RC_BIG, RC_BIG_TICKET, REPEATS>;
         constexpr size_t smem = sizeof(RtSmem<RT_BIG_T, RT_BIG, false>);
         SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k<<<(unsigned)std::min<uint64_t>(m / (RT_MID + 1), (uint64_t)c->n_sms), RT_BIG_T, smem, s>>>(a);
         SPG_LAUNCH_CHECK();
     }
     constexpr size_t smem = sizeof(RtSmem<RT_T, RT_CAP, true>);
-    SPG_CUDA_TRY(cudaFuncSetAttribute(rt_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SPG_CUDA_TRY(cudaFuncSetAttribute(rt_tiles<REPEATS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned blocks = (unsigned)std::min<uint64_t>(t_max, (uint64_t)c->n_sms * RT_PER_SM);
-    rt_tiles<<<blocks, RT_T, smem, s>>>(a);
+    rt_tiles<REPEATS><<<blocks, RT_T, smem, s>>>(a);
     SPG_LAUNCH_CHECK();
     return SPG_OK;
 }
@@ -718,8 +743,8 @@ int rt_run(Ctx *c, const RtArgs &a, uint64_t plan_tiles, uint64_t t_max, uint64_
 }  // namespace
 
 int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off,
-                       uint64_t m, uint64_t n_rows, int cbits, bool keep_zeros, const unsigned long long *abort,
-                       GroupedOut *out, bool *done, cudaStream_t s) {
+                       uint64_t m, uint64_t n_rows, int cbits, bool near, bool keep_zeros,
+                       const unsigned long long *abort, GroupedOut *out, bool *done, cudaStream_t s) {
     *done = false;
     const uint64_t plan_tiles = (n_rows + RP_ROWS - 1) / RP_ROWS;
     // two neighbouring tiles of one part hold more than RT_CAP entries together
@@ -764,9 +789,14 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
     a.abort = abort;
     a.status = c->d_status;
     a.words = c->d_words;
+    // Long rows may have more inserts than columns where the matrix has few
+    // columns or the rows' columns lie near each other. (The kernels for that:
+    // 2000 inserts a row on 64 columns 573 -> 284 us, 20 k rows of 1000 on 300
+    // neighbouring ones 570 -> 396; but 3 % of the 4M-row Zipf matrix's lock.)
+    const bool repeats = near || cbits <= RT_FEW_CBITS;
     HugeRows H;
     while (true) {
-        SPG_TRY(rt_run(c, a, plan_tiles, t_max, m, s));
+        SPG_TRY(repeats ? rt_run<true>(c, a, plan_tiles, t_max, m, s) : rt_run<false>(c, a, plan_tiles, t_max, m, s));
         if (a.huge_ready)
             rt_huge_rows<<<grid_for(H.entries, 256, (unsigned)c->n_sms * 8), 256, 0, s>>>(
                 a.huge, H.row.as<uint32_t>(), H.cols.as<uint32_t>(), H.vals.as<double>(), H.first.as<uint64_t>(), H.n,

@@ -82,3 +82,34 @@ def test_lock_hub_row_among_clustered_rows(ctx):
     A = sg.Csr(ctx, n, n)
     A.lock(*e)
     assert_csr_equal(A.download(), oracle.lock_epochs(n, n, [e]))
+
+
+@pytest.mark.parametrize("L", [33, 40, 2048, 2049, 4097, 12_288])
+@pytest.mark.parametrize("wide", [False, True])
+def test_lock_rows_of_more_inserts_than_columns(ctx, L, wide):
+    """Rows around the point where each column of the row's range has a place
+    of its own (range below length - 2), beside rows that are short or spread;
+    the last write of a column wins, and a last zero leaves nothing."""
+    n_cols = (1 << 31) + 7 if wide else 40_000
+    lens, lo, rng = [], [], []
+    for k in (L - 1, L - 2, L - 3, L // 2, 1, 0, 7):  # columns in the range
+        for length in (L, 5, 0, 33):
+            lens.append(length)
+            lo.append(3 + 11 * len(lens))
+            rng.append(max(1, min(k if length == L else n_cols - 1000, n_cols - 1000)))
+    lens, lo, rng = (np.asarray(x, np.int64) for x in (lens, lo, rng))
+    rows = np.repeat(np.arange(len(lens), dtype=np.uint32), lens)
+    ctr = np.arange(len(rows), dtype=np.uint64)
+    cols = (lo[rows] + (gen.hash3(L, 1, ctr) % rng[rows].astype(np.uint64)).astype(np.int64)).astype(np.uint32)
+    first = np.r_[True, rows[1:] != rows[:-1]]  # the ends of every range occur
+    last = np.r_[rows[1:] != rows[:-1], True]
+    cols[first] = lo[rows[first]]
+    cols[last] = lo[rows[last]] + rng[rows[last]] - 1
+    vals = gen.sym_unit(gen.hash3(L, 2, ctr))
+    vals[::5] = 0.0
+    e = (rows, cols, vals)
+    A = sg.Csr(ctx, len(lens), n_cols)
+    A.lock(*e)
+    assert_csr_equal(A.download(), oracle.lock_epochs(len(lens), n_cols, [e]))
+    A.lock(*(x[::-1].copy() for x in e))
+    assert_csr_equal(A.download(), oracle.lock_epochs(len(lens), n_cols, [e, tuple(x[::-1].copy() for x in e)]))
