@@ -850,7 +850,15 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
         // or more; and for columns wider than the classes take, whose only
         // other way is the global sort (2 M rows of a 5-point stencil in 2^31
         // columns 0.26 / 1.33, shuffled 0.67 / 1.72).
-        const bool tiles = m <= FEW_STAGED || cbits > ROW_CLASS_CBITS || 8 * pre->long_hits > m + m / 32 || pre->clustered < 0;
+        // Rows of 2 400 to 4 096 inserts on average go to the classes' radix blocks
+        // (2 500 rows of 4000 in 1 M columns: 436 tiles / 385 us), and so do rows
+        // of 1 536 and more in up to 2^14 columns, which those sort in two or three
+        // passes (3 333 rows of 3000 on 4096: 520 / 350; 1 250 of 8000 on 16 384:
+        // 498 / 443; 5 000 of 2000 on 4096: 387 / 333).
+        const uint64_t mean = m / n;
+        const bool radix = (mean >= 2400 && mean <= 4096) || (mean >= 1536 && cbits <= 14);
+        const bool tiles = (m <= FEW_STAGED && !radix) || cbits > ROW_CLASS_CBITS || 
+                           (!radix && (8 * pre->long_hits > m + m / 32 || pre->clustered < 0));
         DevBuf s_off, kept, scols, svals;
         SPG_TRY(staged_offsets(c, pre, rows, m, n, s_off, s));
         bool done = false;

@@ -113,3 +113,22 @@ def test_lock_rows_of_more_inserts_than_columns(ctx, L, wide):
     assert_csr_equal(A.download(), oracle.lock_epochs(len(lens), n_cols, [e]))
     A.lock(*(x[::-1].copy() for x in e))
     assert_csr_equal(A.download(), oracle.lock_epochs(len(lens), n_cols, [e, tuple(x[::-1].copy() for x in e)]))
+
+
+@pytest.mark.parametrize("mean", [1535, 1536, 2399, 2400, 4096, 4097])
+@pytest.mark.parametrize("n_cols", [1 << 14, (1 << 14) + 1])
+def test_lock_mean_row_length_rule(ctx, mean, n_cols):
+    """Means of inserts per row at the ends of the ranges that go to the row
+    classes, with rows of other lengths among them."""
+    n = 40
+    lens = np.full(n, mean, np.int64)
+    lens[::4] += 900  # (the mean stays)
+    lens[1::4] -= 900
+    rows = np.repeat(np.arange(n, dtype=np.uint32), lens)
+    ctr = np.arange(len(rows), dtype=np.uint64)
+    cols = gen.below(gen.hash3(mean, 1, ctr), n_cols)
+    vals = gen.sym_unit(gen.hash3(mean, 2, ctr))
+    vals[::9] = 0.0
+    A = sg.Csr(ctx, n, n_cols)
+    A.lock(rows, cols, vals)
+    assert_csr_equal(A.download(), oracle.lock_epochs(n, n_cols, [(rows, cols, vals)]))
