@@ -11,10 +11,10 @@
 // variants compute the same C (the autotuner and the learned selector choose
 // among them, spg_tune.cu):
 //
-//   SPG_SPGEMM_ROWMERGE: when no row has more than 64 products, eight lanes
-//   add up each row in a hash table and write C in one pass
-//   (spg_spgemm_hash.cu; 3D 7-point Laplacian squared 0.93 -> 0.63 ms).
-//   Otherwise every row owns a scratch region of its product count. Light rows (at most MG_RMAX entries in A's row and MG_PMAX
+//   SPG_SPGEMM_ROWMERGE: when no row has more than 64 products (and there are
+//   not many rows of few, merges_rows), eight lanes add up each row in a hash
+//   table and write C in one pass (spg_spgemm_hash.cu; 3D 7-point Laplacian
+//   squared 0.93 -> 0.63 ms). Otherwise every row owns a scratch region of its product count. Light rows (at most MG_RMAX entries in A's row and MG_PMAX
 //   products): one thread merges the row's B rows (each sorted by column) as
 //   a k-way merge on the column, taking equal columns in ascending A-entry
 //   order, so every C(i, j) is summed in Spira's order. Heavy rows go through
@@ -45,19 +45,27 @@ namespace {
 constexpr int GB = 256;
 
 // Products per row of A (thread per row); entry m is 0. ctr[0] += all of them,
-// ctr[1] += the rows of more than SPGEMM_HASH_MAX; the host gets both in
-// words[0 .. 1].
+// ctr[1] += the rows of more than SPGEMM_HASH_MAX, ctr[2] += the rows whose
+// first two columns are nearer than `near`, less those whose are not; the host
+// gets all three in words[0 .. 2].
 __global__ void __launch_bounds__(GB)
 sg_row_products(const uint64_t *__restrict__ aoff, const uint32_t *__restrict__ acols,
-                const uint64_t *__restrict__ boff, uint64_t m, uint64_t *__restrict__ cnt,
+                const uint64_t *__restrict__ boff, uint64_t m, uint32_t near, uint64_t *__restrict__ cnt,
                 unsigned long long *__restrict__ ctr, unsigned long long *__restrict__ words) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     unsigned long long s = 0;
-    if (i < m)
-        for (uint64_t ka = aoff[i]; ka < aoff[i + 1]; ++ka) {
+    int score = 0;
+    if (i < m) {
+        const uint64_t a0 = aoff[i], a1 = aoff[i + 1];
+        uint32_t first = 0;
+        for (uint64_t ka = a0; ka < a1; ++ka) {
             const uint32_t k = acols[ka];
             s += boff[k + 1] - boff[k];
+            if (ka == a0) first = k;
+            else if (ka == a0 + 1) score = k - first < near ? 1 : -1;
         }
+    }
+    score = __reduce_add_sync(0xffffffffu, score);
     if (i <= m) cnt[i] = s;
     unsigned long long sum = s, over = s > (unsigned long long)SPGEMM_HASH_MAX ? 1 : 0;
 #pragma unroll
@@ -66,21 +74,24 @@ sg_row_products(const uint64_t *__restrict__ aoff, const uint32_t *__restrict__ 
         over += __shfl_xor_sync(0xffffffffu, over, o);
     }
     __shared__ unsigned long long s_s[GB / 32], s_o[GB / 32];
+    __shared__ int s_near[GB / 32];
     if ((threadIdx.x & 31) == 0) {
         s_s[threadIdx.x >> 5] = sum;
         s_o[threadIdx.x >> 5] = over;
+        s_near[threadIdx.x >> 5] = score;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 1; w < GB / 32; ++w) {
             sum += s_s[w];
             over += s_o[w];
+            score += s_near[w];
         }
         if (sum) atomicAdd(ctr, sum);
         if (over) atomicAdd(ctr + 1, over);
-        if (last_block(ctr + 2)) {
-            store_word(words, 0, *(volatile unsigned long long *)ctr);
-            store_word(words, 1, *(volatile unsigned long long *)(ctr + 1));
+        if (score) atomicAdd(ctr + 2, (unsigned long long)(long long)score);
+        if (last_block(ctr + 3)) {
+            for (int k = 0; k < 3; ++k) store_word(words, k, *(volatile unsigned long long *)(ctr + k));
         }
     }
 }
@@ -445,21 +456,24 @@ void spgemm_install(Csr *Cm, uint64_t m, uint64_t n, DevBuf &&off, DevBuf &&cols
     Cm->may_have_zeros = false;
 }
 
-// Products per row of A (pofs[i], not yet scanned; pofs[m] = 0), their number P
-// and how many rows have more than SPGEMM_HASH_MAX.
+// Products per row of A (pofs[i], not yet scanned; pofs[m] = 0), their number P,
+// how many rows have more than SPGEMM_HASH_MAX, and whether A's rows start with
+// columns near each other.
 int spgemm_products(Ctx *c, const Csr *A, const Csr *B, DevBuf *pofs, uint64_t *P, uint64_t *long_rows,
-                    cudaStream_t s) {
+                    bool *near, cudaStream_t s) {
     const uint64_t m = A->n_rows;
     DevBuf ctr;
-    SPG_TRY(ctr.alloc(3 * sizeof(unsigned long long), s));
-    SPG_CUDA_TRY(cudaMemsetAsync(ctr.ptr, 0, 3 * sizeof(unsigned long long), s));
+    SPG_TRY(ctr.alloc(4 * sizeof(unsigned long long), s));
+    SPG_CUDA_TRY(cudaMemsetAsync(ctr.ptr, 0, 4 * sizeof(unsigned long long), s));
     SPG_TRY(pofs->alloc((m + 1) * sizeof(uint64_t), s));
-    sg_row_products<<<grid_for(m + 1, GB), GB, 0, s>>>(A->d_off(), A->d_cols(), B->d_off(), m, pofs->as<uint64_t>(),
+    sg_row_products<<<grid_for(m + 1, GB), GB, 0, s>>>(A->d_off(), A->d_cols(), B->d_off(), m,
+                                                       (uint32_t)(A->n_cols / 16), pofs->as<uint64_t>(),
                                                        ctr.as<unsigned long long>(), c->d_words);
     SPG_LAUNCH_CHECK();
     SPG_TRY(c->phase_sync(s));
     *P = c->word(0);
     *long_rows = c->word(1);
+    *near = (long long)c->word(2) > 0;
     if (*P >= (1ull << 32))
         return set_error(SPG_ERR_UNSUPPORTED, "spgemm: %llu products exceed 2^32-1", (unsigned long long)*P);
     return SPG_OK;
@@ -472,7 +486,8 @@ int spgemm_esc_all(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, cudaStream_t s) 
     const int cbits = bits_for(n), rbits = bits_for(m);
     DevBuf pofs;
     uint64_t P = 0, long_rows = 0;
-    SPG_TRY(spgemm_products(c, A, B, &pofs, &P, &long_rows, s));
+    bool near = false;
+    SPG_TRY(spgemm_products(c, A, B, &pofs, &P, &long_rows, &near, s));
     SPG_TRY(exclusive_scan_u64(c, pofs.as<uint64_t>(), m + 1, nullptr, s));
     EscOut eo;
     SPG_TRY(spgemm_esc(c, A, B, pofs.as<uint64_t>(), P, rbits, cbits, &eo, s));
@@ -494,6 +509,21 @@ int spgemm_esc_all(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, cudaStream_t s) 
     return SPG_OK;
 }
 
+// Rows of few products: a thread's merge takes less than a hash tile's share
+// (its table is cleared, compacted and sorted whatever the row holds), but the
+// scans, the compaction and a second wait cost about 85 us more per call. What
+// the merge saves per row falls with the products; where the rows' columns are
+// near each other it stays above zero up to about 40. Merge / hash, us:
+//   1 M rows, scattered: 1 product 188 / 364, 4 253 / 399, 9 372 / 456, 16 549 / 543, 25 831 / 696
+//   1 M rows, near:      9 (tridiagonal) 276 / 419, 16 338 / 452, 25 (5-point stencil) 528 / 494, 36 530 / 518
+//   4 M rows, near:      9 739 / 1555, 16 963 / 1668, 25 1682 / 1866, 36 1688 / 1915, 64 2251 / 2110
+//   100 k rows:          1 139 / 83, 16 181 / 105, near 9 146 / 90
+bool spgemm_merges_rows(uint64_t m, uint64_t P, bool near) {
+    const double mean = (double)P / (double)m;
+    const double saved_ns = std::max(0.25 - (near ? 0.007 : 0.01) * mean, near && mean <= 40.0 ? 0.075 : 0.0);
+    return (double)m * saved_ns > 85e3;
+}
+
 // SPG_SPGEMM_ROWMERGE.
 int spgemm_rowmerge(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, cudaStream_t s) {
     const uint64_t m = A->n_rows, n = B->n_cols;
@@ -501,9 +531,10 @@ int spgemm_rowmerge(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, cudaStream_t s)
     int rc = SPG_OK;
     DevBuf pofs;
     uint64_t P = 0, long_rows = 0;
-    SPG_TRY(spgemm_products(c, A, B, &pofs, &P, &long_rows, s));
+    bool near = false;
+    SPG_TRY(spgemm_products(c, A, B, &pofs, &P, &long_rows, &near, s));
     // every row's products fit a hash table: eight lanes per row, C in one pass
-    if (P && long_rows == 0 && n <= 0xFFFFFFFFull) {
+    if (P && long_rows == 0 && n <= 0xFFFFFFFFull && !spgemm_merges_rows(m, P, near)) {
         pofs.release();
         return spgemm_hash_rows(c, A, B, Cm, P, s);
     }
