@@ -426,7 +426,8 @@ int spg_spgemm_selector_predict(spg_ctx *ctx, const float *d_features, uint32_t 
  * the autotuner), SPG_POLICY_AUTOTUNE, SPG_POLICY_FIXED (SPG_SPGEMM_WARPSORT_128
  * without measuring). The selector never picks a WARPSORT variant that a
  * smaller one does the same work for: when every row of A * B has at most 64
- * products and A entries, _128 and _256 are skipped; up to 128, _256. The
+ * products and A entries, _128, _256 and ESC are skipped; up to 128, _256.
+ * Many rows of few products (about 350 000 of one, 1 M of 16) go to ROWMERGE. The
  * choice is cached per (A, B) until either changes. */
 int spg_set_spgemm_policy(spg_ctx *ctx, int policy);
 

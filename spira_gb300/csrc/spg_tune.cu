@@ -499,7 +499,7 @@ int selector_load_default(Ctx *c) {
 // ---------------------------------------------------------------- SpGEMM choice
 // max_products / max_a (may be null): the most products and A entries of any row.
 int spgemm_features(Ctx *c, const Csr *A, const Csr *B, float *f, double *max_products = nullptr,
-                    double *max_a = nullptr) {
+                    double *max_a = nullptr, double *sum_p = nullptr) {
     cudaStream_t s = c->stream;
     DevBuf acc;
     SPG_TRY(acc.alloc(38 * sizeof(double), s));
@@ -514,6 +514,7 @@ int spgemm_features(Ctx *c, const Csr *A, const Csr *B, float *f, double *max_pr
     SPG_CUDA_TRY(cudaStreamSynchronize(s));
     if (max_products) *max_products = h[34];
     if (max_a) *max_a = h[37];
+    if (sum_p) *sum_p = h[32];
     const double m = (double)(A->n_rows ? A->n_rows : 1);
     for (int i = 0; i < 32; ++i) f[i] = (float)(h[i] / m);
     const double mean = h[32] / m;
@@ -567,8 +568,8 @@ int spgemm_resolve_auto(Ctx *c, const Csr *A, const Csr *B, int *variant) {
     int v = SPG_SPGEMM_WARPSORT_128;
     if (c->spgemm_policy == SPG_POLICY_SELECTOR && c->gemm_model_k == SPG_SPGEMM_N_VARIANTS) {
         float f[F];
-        double maxp = 0.0, maxa = 0.0;
-        SPG_TRY(spgemm_features(c, A, B, f, &maxp, &maxa));
+        double maxp = 0.0, maxa = 0.0, sum_p = 0.0;
+        SPG_TRY(spgemm_features(c, A, B, f, &maxp, &maxa, &sum_p));
         cudaStream_t s = c->stream;
         DevBuf df, dout;
         SPG_TRY(df.alloc(F * sizeof(float), s));
@@ -583,6 +584,12 @@ int spgemm_resolve_auto(Ctx *c, const Csr *A, const Csr *B, int *variant) {
         // shared memory per tile (fewer tiles resident); likewise 256 against 128 up to 128.
         if (maxp <= 64.0 && maxa <= 64.0) sc[SPG_SPGEMM_WARPSORT_128] = sc[SPG_SPGEMM_WARPSORT_256] = INFINITY;
         else if (maxp <= 128.0 && maxa <= 128.0) sc[SPG_SPGEMM_WARPSORT_256] = INFINITY;
+        // ESC sorts every product by (row, column) in global memory: with rows that short it took 2 to 10
+        // times the warps' sort in every measurement (1 M rows of 2: 949 / 584 us, 100 k 325 / 103).
+        if (maxp <= 64.0 && maxa <= 64.0) sc[SPG_SPGEMM_ESC] = INFINITY;
+        // ROWMERGE merges many rows of few products in a thread each: 1 M rows of 3 372 / 585 us.
+        const uint64_t P = (uint64_t)sum_p;
+        if (maxp <= 64.0 && A->n_rows && P && spgemm_merges_rows(A->n_rows, P, false)) sc[SPG_SPGEMM_ROWMERGE] = -INFINITY;
         v = 0;
         for (int k = 1; k < SPG_SPGEMM_N_VARIANTS; ++k)
             if (sc[k] < sc[v]) v = k;

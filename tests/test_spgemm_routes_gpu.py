@@ -1,5 +1,5 @@
-"""ROWMERGE's choice between a thread's merge per row and the hash rows.
-Every way gives the same bits."""
+"""ROWMERGE's choice between a thread's merge per row and the hash rows, and
+AUTO's for rows of few products. Every way gives the same bits."""
 from __future__ import annotations
 
 import numpy as np
@@ -36,3 +36,12 @@ def test_rowmerge_of_many_short_rows(ctx, n, per_row, near):
     want = oracle.spgemm(H, H)
     for v in (sg.SPGEMM_VARIANTS["rowmerge"], sg.SPGEMM_VARIANTS["warpsort_64"], -1):
         assert_csr_equal(A.spgemm(A, v).download(), want)
+
+
+@pytest.mark.parametrize("n,per_row", [(10_000, 2), (100_000, 2), (1_000_000, 2), (1_000_000, 1)])
+def test_auto_leaves_esc_to_long_rows(ctx, n, per_row):
+    A, _ = _matrix(ctx, n, per_row, False)
+    picked = A.spgemm_selected(A)
+    assert picked in (sg.SPGEMM_VARIANTS["rowmerge"], sg.SPGEMM_VARIANTS["warpsort_64"])
+    if n == 1_000_000:
+        assert picked == sg.SPGEMM_VARIANTS["rowmerge"]
