@@ -23,7 +23,8 @@ namespace spg {
 namespace {
 
 constexpr int TB = 256;
-constexpr uint64_t LOOK_LARGE = 10u << 20;
+constexpr unsigned LOOK_SAMPLES = 1024;  // a block
+constexpr uint64_t LOOK_FEW = 1u << 20;
 
 // rowid[k] = source row of entry k (eight lanes per row).
 __global__ void tr_expand(const uint64_t *__restrict__ off, uint64_t n_rows, uint32_t *__restrict__ rowid) {
@@ -36,6 +37,26 @@ __global__ void tr_expand(const uint64_t *__restrict__ off, uint64_t n_rows, uin
 __global__ void tr_count(const uint32_t *__restrict__ cols, uint64_t nnz, unsigned long long *__restrict__ cnt) {
     for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < nnz; k += (uint64_t)gridDim.x * blockDim.x)
         atomicAdd(cnt + cols[k], 1ull);
+}
+
+// Whether the source rows repeat each other's pattern: of a row's entry and the
+// one in the same place of the next row, in LOOK_SAMPLES rows, words[0] = how
+// often the column is the same or one more, words[1] = the samples taken.
+__global__ void __launch_bounds__(LOOK_SAMPLES)
+tr_sample(const uint64_t *__restrict__ off, const uint32_t *__restrict__ cols, uint64_t m,
+          unsigned long long *__restrict__ words) {
+    const uint64_t k = threadIdx.x, r = k * (m - 1) / LOOK_SAMPLES;
+    const uint64_t b = off[r], e = off[r + 1], f = off[r + 2];
+    bool same = false;
+    if (e > b) {
+        const uint64_t j = k % (e - b);
+        same = j < f - e && cols[e + j] - cols[b + j] <= 1u;
+    }
+    const int hits = __syncthreads_count(same), taken = __syncthreads_count(e > b);
+    if (threadIdx.x == 0) {
+        store_word(words, 0, (unsigned long long)hits);
+        store_word(words, 1, (unsigned long long)taken);
+    }
 }
 
 // Thread per source row: entry (w, c) goes to toff[c] + (a cursor of column
@@ -229,12 +250,26 @@ int transpose_impl(Ctx *c, const Csr *A, Csr *T, cudaStream_t s) {
     SPG_TRY(out_off.alloc(csr_off_elems(n) * sizeof(uint64_t), s));
     unsigned long long longest = NET_MAX + 1;
     // Whether the networks may do: source rows below their padding key, and not
-    // above 16 entries a column on average (32 from 10 M entries on), where
-    // finding out costs more than they gain. Looked at first / column sort at
-    // once: 500k x 200k with 20 to a column 267 / 219 us, 500k x 500k with 24 568 /
-    // 502 (columns above 32 both); 25 and 27 to a column, all alike: 300 k columns
-    // 344 / 363, 500 k 514 / 538, 1 M 961 / 1020; 13: 225 / 331.
-    const bool look = nnz && m < 0xFFFFFFFFull && nnz <= (nnz > LOOK_LARGE ? NET_MAX : 16) * n;
+    // above 32 entries a column on average. From 16 on it depends on whether the
+    // columns are alike: 27 to every column are the networks' case (looked at
+    // first / column sort at once: 300 k columns 344 / 363 us, 500 k 514 / 538, 1 M
+    // 961 / 1020), random ones have some column above 32, and the look is lost
+    // (500k x 200k with 20 to a column 267 / 219, 500k x 500k with 24 568 / 502).
+    // A sample of the rows tells, for 10 us: rows that repeat their predecessor's
+    // columns, in place or moved by one, as stencils, bands and blocks do. Such
+    // matrices are square, so others are not sampled, nor are those of up to 1 M
+    // entries, where the column sort is as fast for both (20 k columns of 28: 77 us
+    // a band, 79 random ones; looked at 85).
+    bool look = nnz && m < 0xFFFFFFFFull && nnz <= NET_MAX * n;
+    if (look && nnz > 16 * n) {
+        look = false;
+        if (m == n && nnz > LOOK_FEW) {
+            tr_sample<<<1, LOOK_SAMPLES, 0, s>>>(A->d_off(), A->d_cols(), m, c->d_words);
+            SPG_LAUNCH_CHECK();
+            SPG_TRY(c->phase_sync(s));
+            look = 4 * c->word(0) >= 3 * c->word(1);
+        }
+    }
     if (look || nnz == 0) SPG_CUDA_TRY(cudaMemsetAsync(out_off.ptr, 0, csr_off_elems(n) * sizeof(uint64_t), s));
     if (look) {
         tr_count<<<grid_for(nnz, TB, gmax), TB, 0, s>>>(A->d_cols(), nnz,
