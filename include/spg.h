@@ -313,7 +313,8 @@ int spg_batch_destroy(spg_batch *batch);
  * columns give a + b (one IEEE add) and are kept unless the sum is +-0, other
  * entries are copied, stored zeros are dropped; C is reshaped to A's shape
  * with tight capacity (serial/matrix_addition.hpp:34-110,
- * parallel/algorithms/matrix_addition.hpp:24-99). A and B of different shapes
+ * parallel/algorithms/matrix_addition.hpp:24-99); its arrays hold about C's
+ * size, or room for A's and B's entries where those are at most 4 Mi. A and B of different shapes
  * give SPG_ERR_INVALID_ARGUMENT, an unlocked A or B SPG_ERR_LOGIC; C must not
  * be A or B. */
 int spg_csr_add(spg_ctx *ctx, const spg_csr *A, const spg_csr *B, spg_csr *C);

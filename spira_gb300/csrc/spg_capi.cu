@@ -37,6 +37,16 @@ int Ctx::phase_sync(cudaStream_t s) {
     return take_status();  // a wait that gave up: nothing after it may be used
 }
 
+int Ctx::wait_word(int k, cudaStream_t s) {
+    for (unsigned spin = 1; !word(k); ++spin) {
+        if (spin % 1024) continue;
+        const cudaError_t e = cudaStreamQuery(s);
+        if (e == cudaSuccess) break;
+        if (e != cudaErrorNotReady) SPG_CUDA_TRY(e);
+    }
+    return SPG_OK;
+}
+
 int Ctx::ensure_pinned(size_t bytes) {
     if (pinned_bytes >= bytes) return SPG_OK;
     if (pinned) cudaFreeHost(pinned);

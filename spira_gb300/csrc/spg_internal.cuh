@@ -123,6 +123,9 @@ struct Ctx {
     unsigned long long *h_words = nullptr;
     unsigned long long *d_words = nullptr;
     uint64_t word(int k) const { return *(volatile unsigned long long *)(h_words + k); }
+    // Waits for a word that was set to 0 before the launch and that a running
+    // kernel stores (store_word_now), or for the stream if that is sooner.
+    int wait_word(int k, cudaStream_t s);
     // Returns SPG_ERR_DEVICE_TIMEOUT (and clears the word) if a kernel flagged
     // one since the last check; call after a stream synchronisation.
     int take_status() {
@@ -350,6 +353,14 @@ __device__ __forceinline__ bool last_block(Count *done) {
 
 __device__ __forceinline__ void store_word(unsigned long long *words, int k, unsigned long long v) {
     *(volatile unsigned long long *)(words + k) = v;
+}
+
+// The same for a host that reads the word while the kernel runs (Ctx::wait_word),
+// after what the thread stored before.
+__device__ __forceinline__ void store_word_now(unsigned long long *words, int k, unsigned long long v) {
+    __threadfence_system();
+    store_word(words, k, v);
+    __threadfence_system();
 }
 
 // Lanes of the (full) warp whose NB-bit value d (a radix digit, or 256 for
@@ -617,6 +628,16 @@ int spgemm_resolve_auto(Ctx *c, const Csr *A, const Csr *B, int *variant);
 enum class MergeMode { Sum, Replace };
 int merge_csr(Ctx *c, const CsrView &A, const CsrView &B, uint64_t n_rows, MergeMode mode, uint64_t *off_out,
               uint32_t *cols_out, double *vals_out, uint64_t *nnz, cudaStream_t s);
+// C = A + B with C's arrays allocated here: for all entries of both sides when
+// they are few, by a sample of the equal pairs otherwise.
+int sum_csr(Ctx *c, const CsrView &A, const CsrView &B, uint64_t n_rows, uint64_t *off_out, DevBuf &cols, DevBuf &vals,
+            uint64_t *nnz, cudaStream_t s);
+// Results up to this size keep arrays of their upper bound; larger ones get
+// arrays of about their own size (12 bytes an entry).
+constexpr uint64_t RESULT_BOUND = 4u << 20;
+// Moves n entries out of arrays for `room` of them when more than an eighth is
+// unused (waits for the copy).
+int fit_arrays(Ctx *c, uint64_t n, uint64_t room, DevBuf &cols, DevBuf &vals, cudaStream_t s);
 
 // CSR helpers used by several ops (spg_lock.cu).
 int csr_alloc(Csr *A, uint64_t capacity, cudaStream_t s);

@@ -711,6 +711,18 @@ huge_keep(const uint32_t *__restrict__ row, const uint32_t *__restrict__ col, co
 
 }  // namespace
 
+int fit_arrays(Ctx *c, uint64_t n, uint64_t room, DevBuf &cols, DevBuf &vals, cudaStream_t s) {
+    if (n >= room - room / 8) return SPG_OK;
+    DevBuf own_cols, own_vals;
+    SPG_TRY(own_cols.alloc(csr_alloc_elems(n) * sizeof(uint32_t), s));
+    SPG_TRY(own_vals.alloc(csr_alloc_elems(n) * sizeof(double), s));
+    SPG_CUDA_TRY(cudaMemcpyAsync(own_cols.ptr, cols.ptr, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+    SPG_CUDA_TRY(cudaMemcpyAsync(own_vals.ptr, vals.ptr, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    cols = std::move(own_cols);
+    vals = std::move(own_vals);
+    return c->phase_sync(s);
+}
+
 int order_huge_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint64_t *s_off, const uint32_t *huge,
                     int cbits, bool keep_zeros, HugeRows *H, uint64_t *count, cudaStream_t s) {
     const uint64_t n = H->n, m = H->entries, tiles = (m + KTILE - 1) / KTILE;
@@ -762,21 +774,11 @@ int order_huge_rows(Ctx *c, const uint32_t *cols, const double *vals, const uint
 
 namespace {
 
-// Installs a first lock's CSR built in arrays sized for m entries; when more
-// than an eighth of them stayed unused the entries move to arrays of their
-// own size (build_csr: exact capacity).
+// Installs a first lock's CSR built in arrays sized for m entries (build_csr:
+// exact capacity).
 int first_install(Ctx *c, Csr *A, GroupedOut &&o, uint64_t m, cudaStream_t s) {
     const uint64_t nnz = o.n;
-    if (nnz < m - m / 8) {
-        DevBuf cols, vals;
-        SPG_TRY(cols.alloc(csr_alloc_elems(nnz) * sizeof(uint32_t), s));
-        SPG_TRY(vals.alloc(csr_alloc_elems(nnz) * sizeof(double), s));
-        SPG_CUDA_TRY(cudaMemcpyAsync(cols.ptr, o.cols.ptr, nnz * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-        SPG_CUDA_TRY(cudaMemcpyAsync(vals.ptr, o.vals.ptr, nnz * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        o.cols = std::move(cols);
-        o.vals = std::move(vals);
-        SPG_TRY(c->phase_sync(s));
-    }
+    SPG_TRY(fit_arrays(c, nnz, m, o.cols, o.vals, s));
     A->invalidate_derived();
     A->off = std::move(o.off);
     A->cols = std::move(o.cols);

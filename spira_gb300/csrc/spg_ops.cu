@@ -301,17 +301,13 @@ void install(Csr *C, uint64_t n_rows, uint64_t n_cols, DevBuf &off, DevBuf &cols
     C->may_have_zeros = false;
 }
 
-// C's arrays have room for every entry of both sides; nnz(C) of it is used, at
-// least half (an equal pair becomes one entry) but for cancellations.
 int add_impl(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, cudaStream_t s) {
     const uint64_t n = A->n_rows;
     DevBuf off, cols, vals;
     SPG_TRY(off.alloc(csr_off_elems(n) * sizeof(uint64_t), s));
-    SPG_TRY(cols.alloc(csr_alloc_elems(A->nnz + B->nnz) * sizeof(uint32_t), s));
-    SPG_TRY(vals.alloc(csr_alloc_elems(A->nnz + B->nnz) * sizeof(double), s));
     uint64_t nnz = 0;
-    SPG_TRY(merge_csr(c, {A->d_off(), A->d_cols(), A->d_vals(), A->nnz}, {B->d_off(), B->d_cols(), B->d_vals(), B->nnz},
-                      n, MergeMode::Sum, off.as<uint64_t>(), cols.as<uint32_t>(), vals.as<double>(), &nnz, s));
+    SPG_TRY(sum_csr(c, {A->d_off(), A->d_cols(), A->d_vals(), A->nnz}, {B->d_off(), B->d_cols(), B->d_vals(), B->nnz},
+                    n, off.as<uint64_t>(), cols, vals, &nnz, s));
     install(Cm, n, A->n_cols, off, cols, vals, nnz);
     return SPG_OK;
 }
