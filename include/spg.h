@@ -385,7 +385,8 @@ int spg_spgemm(spg_ctx *ctx, const spg_csr *A, const spg_csr *B, spg_csr *C);
 enum spg_spgemm_variant {
     SPG_SPGEMM_AUTO = -1,        /* the context's policy, as for SpMV */
     SPG_SPGEMM_ROWMERGE = 0,     /* rows of <= 64 products: eight lanes per row and a hash
-                                    table, C in one pass; if some row has more: a thread
+                                    table, C in one pass (from 4 Mi products on in arrays of
+                                    about C's size, below of the products'); if some row has more: a thread
                                     per row merges the row's B rows (k-way, by column); rows with > 32 A entries or > 4096 products
                                     go through expand-sort-compress; a compaction pass */
     SPG_SPGEMM_ESC = 1,          /* expand every product, one global radix sort by

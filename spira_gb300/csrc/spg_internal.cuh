@@ -614,7 +614,7 @@ uint64_t read_u64(Ctx *c, const uint64_t *d, cudaStream_t s, int *rc);
 // (spg_spgemm_hash.cu).
 constexpr int SPGEMM_HASH_MAX = 64;
 bool spgemm_merges_rows(uint64_t m, uint64_t P, bool near);  // whether a thread's merge per row is the faster way all the same
-int spgemm_hash_rows(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, uint64_t P, cudaStream_t s);
+int spgemm_hash_rows(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, uint64_t P, uint64_t room, cudaStream_t s);
 int spgemm_warpsort(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, int variant, cudaStream_t s);
 int spgemm_run(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, int variant, cudaStream_t s);
 // SPG_SPGEMM_AUTO resolved by the context's policy (spg_tune.cu).

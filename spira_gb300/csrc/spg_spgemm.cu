@@ -44,15 +44,72 @@ namespace {
 
 constexpr int GB = 256;
 
+// The distinct columns of SG_SAMPLES rows of C (or of all), of those of 1 to
+// SPGEMM_HASH_MAX products: ctr[0] += the rows' products, ctr[1] += their
+// columns. Eight lanes and a table per row, a lane per entry of A.
+constexpr uint32_t SG_SAMPLES = 2048;
+constexpr int SG_SAMPLE_G = 8, SG_SAMPLE_BLOCKS = SG_SAMPLES * SG_SAMPLE_G / GB;
+
+__device__ void sg_sample_rows(const uint64_t *__restrict__ aoff, const uint32_t *__restrict__ acols,
+                               const uint64_t *__restrict__ boff, const uint32_t *__restrict__ bcols, uint64_t m,
+                               unsigned long long *__restrict__ ctr) {
+    constexpr uint32_t EMPTY = 0xFFFFFFFFu, SLOTS = SPGEMM_HASH_MAX;
+    __shared__ uint32_t s_key[GB / SG_SAMPLE_G][SLOTS];
+    const int t = threadIdx.x, l = t % SG_SAMPLE_G;
+    uint32_t *key = s_key[t / SG_SAMPLE_G];
+    for (uint32_t h = l; h < SLOTS; h += SG_SAMPLE_G) key[h] = EMPTY;
+    __syncwarp();
+    const uint64_t rows = min(m, (uint64_t)SG_SAMPLES), k = ((uint64_t)blockIdx.x * GB + t) / SG_SAMPLE_G;
+    uint64_t a0 = 0, a1 = 0, p = 0;
+    if (k < rows) {  // one row of each of as many parts, at a place of its own
+        const uint64_t part = m / rows, row = k * part + (k * 0x9E3779B1ull >> 8) % part;
+        a0 = aoff[row];
+        a1 = aoff[row + 1];
+        for (uint64_t i = a0 + l; i < a1; i += SG_SAMPLE_G) p += boff[acols[i] + 1ull] - boff[acols[i]];
+    }
+#pragma unroll
+    for (int o = 1; o < SG_SAMPLE_G; o <<= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+    uint32_t distinct = 0;
+    if (p > 0 && p <= (uint64_t)SLOTS) {
+        for (uint64_t i = a0 + l; i < a1; i += SG_SAMPLE_G) {
+            const uint64_t e = boff[acols[i] + 1ull];
+            for (uint64_t q = boff[acols[i]]; q < e; ++q) {
+                const uint32_t c = bcols[q];
+                uint32_t h = (c * 0x9E3779B1u) >> 26;
+                while (true) {  // (at most SLOTS columns: it ends)
+                    const uint32_t was = atomicCAS(&key[h], EMPTY, c);
+                    if (was == EMPTY) ++distinct;
+                    if (was == EMPTY || was == c) break;
+                    h = (h + 1) % SLOTS;
+                }
+            }
+        }
+    } else {
+        p = 0;
+    }
+    const uint32_t products = __reduce_add_sync(0xffffffffu, l == 0 ? (uint32_t)p : 0u);
+    distinct = __reduce_add_sync(0xffffffffu, distinct);
+    if ((t & 31) == 0 && products) {
+        atomicAdd(ctr, (unsigned long long)products);
+        atomicAdd(ctr + 1, (unsigned long long)distinct);
+        __threadfence();
+    }
+}
+
 // Products per row of A (thread per row); entry m is 0. ctr[0] += all of them,
 // ctr[1] += the rows of more than SPGEMM_HASH_MAX, ctr[2] += the rows whose
 // first two columns are nearer than `near`, less those whose are not; the host
-// gets all three in words[0 .. 2].
+// gets all three in words[0 .. 2]. With a sample wanted, the first blocks take
+// it (ctr[3], ctr[4], words[3 .. 4]) beside the others.
+template <bool SAMPLE>
 __global__ void __launch_bounds__(GB)
 sg_row_products(const uint64_t *__restrict__ aoff, const uint32_t *__restrict__ acols,
-                const uint64_t *__restrict__ boff, uint64_t m, uint32_t near, uint64_t *__restrict__ cnt,
-                unsigned long long *__restrict__ ctr, unsigned long long *__restrict__ words) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+                const uint64_t *__restrict__ boff, const uint32_t *__restrict__ bcols, uint64_t m, uint32_t near,
+                uint64_t *__restrict__ cnt, unsigned long long *__restrict__ ctr,
+                unsigned long long *__restrict__ words) {
+    const bool sampling = SAMPLE && blockIdx.x < SG_SAMPLE_BLOCKS;
+    if (SAMPLE && sampling) sg_sample_rows(aoff, acols, boff, bcols, m, ctr + 3);
+    const uint64_t i = sampling ? ~0ull : (blockIdx.x - (SAMPLE ? SG_SAMPLE_BLOCKS : 0u)) * (uint64_t)blockDim.x + threadIdx.x;
     unsigned long long s = 0;
     int score = 0;
     if (i < m) {
@@ -90,8 +147,8 @@ sg_row_products(const uint64_t *__restrict__ aoff, const uint32_t *__restrict__ 
         if (sum) atomicAdd(ctr, sum);
         if (over) atomicAdd(ctr + 1, over);
         if (score) atomicAdd(ctr + 2, (unsigned long long)(long long)score);
-        if (last_block(ctr + 3)) {
-            for (int k = 0; k < 3; ++k) store_word(words, k, *(volatile unsigned long long *)(ctr + k));
+        if (last_block(ctr + 5)) {
+            for (int k = 0; k < 5; ++k) store_word(words, k, *(volatile unsigned long long *)(ctr + k));
         }
     }
 }
@@ -458,22 +515,30 @@ void spgemm_install(Csr *Cm, uint64_t m, uint64_t n, DevBuf &&off, DevBuf &&cols
 
 // Products per row of A (pofs[i], not yet scanned; pofs[m] = 0), their number P,
 // how many rows have more than SPGEMM_HASH_MAX, and whether A's rows start with
-// columns near each other.
+// columns near each other. expected (may be null): about how many entries C has,
+// P at most (by a sample of its rows where there may be many products).
 int spgemm_products(Ctx *c, const Csr *A, const Csr *B, DevBuf *pofs, uint64_t *P, uint64_t *long_rows,
-                    bool *near, cudaStream_t s) {
+                    bool *near, uint64_t *expected, cudaStream_t s) {
     const uint64_t m = A->n_rows;
     DevBuf ctr;
-    SPG_TRY(ctr.alloc(4 * sizeof(unsigned long long), s));
-    SPG_CUDA_TRY(cudaMemsetAsync(ctr.ptr, 0, 4 * sizeof(unsigned long long), s));
+    SPG_TRY(ctr.alloc(6 * sizeof(unsigned long long), s));
+    SPG_CUDA_TRY(cudaMemsetAsync(ctr.ptr, 0, 6 * sizeof(unsigned long long), s));
     SPG_TRY(pofs->alloc((m + 1) * sizeof(uint64_t), s));
-    sg_row_products<<<grid_for(m + 1, GB), GB, 0, s>>>(A->d_off(), A->d_cols(), B->d_off(), m,
-                                                       (uint32_t)(A->n_cols / 16), pofs->as<uint64_t>(),
-                                                       ctr.as<unsigned long long>(), c->d_words);
+    const bool sample = expected && (double)A->nnz * (double)B->nnz > (double)RESULT_BOUND * (double)B->n_rows;
+    auto k = sample ? sg_row_products<true> : sg_row_products<false>;
+    k<<<grid_for(m + 1, GB) + (sample ? SG_SAMPLE_BLOCKS : 0), GB, 0, s>>>(
+        A->d_off(), A->d_cols(), B->d_off(), B->d_cols(), m, (uint32_t)(A->n_cols / 16), pofs->as<uint64_t>(),
+        ctr.as<unsigned long long>(), c->d_words);
     SPG_LAUNCH_CHECK();
     SPG_TRY(c->phase_sync(s));
     *P = c->word(0);
     *long_rows = c->word(1);
     *near = (long long)c->word(2) > 0;
+    if (expected) {
+        *expected = *P;
+        if (sample && c->word(3) && *P > RESULT_BOUND)
+            *expected = std::min(*P, (uint64_t)((double)*P * (double)c->word(4) / (double)c->word(3)) + *P / 32);
+    }
     if (*P >= (1ull << 32))
         return set_error(SPG_ERR_UNSUPPORTED, "spgemm: %llu products exceed 2^32-1", (unsigned long long)*P);
     return SPG_OK;
@@ -487,7 +552,7 @@ int spgemm_esc_all(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, cudaStream_t s) 
     DevBuf pofs;
     uint64_t P = 0, long_rows = 0;
     bool near = false;
-    SPG_TRY(spgemm_products(c, A, B, &pofs, &P, &long_rows, &near, s));
+    SPG_TRY(spgemm_products(c, A, B, &pofs, &P, &long_rows, &near, nullptr, s));
     SPG_TRY(exclusive_scan_u64(c, pofs.as<uint64_t>(), m + 1, nullptr, s));
     EscOut eo;
     SPG_TRY(spgemm_esc(c, A, B, pofs.as<uint64_t>(), P, rbits, cbits, &eo, s));
@@ -532,11 +597,12 @@ int spgemm_rowmerge(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, cudaStream_t s)
     DevBuf pofs;
     uint64_t P = 0, long_rows = 0;
     bool near = false;
-    SPG_TRY(spgemm_products(c, A, B, &pofs, &P, &long_rows, &near, s));
+    uint64_t expected = 0;
+    SPG_TRY(spgemm_products(c, A, B, &pofs, &P, &long_rows, &near, &expected, s));
     // every row's products fit a hash table: eight lanes per row, C in one pass
     if (P && long_rows == 0 && n <= 0xFFFFFFFFull && !spgemm_merges_rows(m, P, near)) {
         pofs.release();
-        return spgemm_hash_rows(c, A, B, Cm, P, s);
+        return spgemm_hash_rows(c, A, B, Cm, P, expected, s);
     }
     SPG_TRY(exclusive_scan_u64(c, pofs.as<uint64_t>(), m + 1, nullptr, s));
     // out_off holds the per-row kept counts, then (scanned) C's offsets

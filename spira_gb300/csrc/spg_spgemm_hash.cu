@@ -43,6 +43,7 @@ struct ShArgs {
     uint64_t *coff;
     uint32_t *ccols;
     double *cvals;
+    uint64_t room;  // entries that ccols and cvals have room for: those beyond are counted, not written
     unsigned int *status;
     unsigned long long *words;  // [0] entries of C
 };
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(SH_T, 8) sh_tiles(ShArgs a) {
         a.coff[a.m] = base + total;
         store_word(a.words, 0, base + total);
     }
-    for (int j = warp; j < SH_ROWS; j += SH_T / 32) {
+    for (int j = base + total <= a.room ? warp : SH_ROWS; j < SH_ROWS; j += SH_T / 32) {
         const uint32_t n = __shfl_sync(0xffffffffu, cnt, j), o = __shfl_sync(0xffffffffu, before, j);
         for (uint32_t q = lane; q < n; q += 32) {
             a.ccols[base + o + q] = S.key[j][q];
@@ -270,29 +271,40 @@ __global__ void __launch_bounds__(SH_T, 8) sh_tiles(ShArgs a) {
 }  // namespace
 
 // Every row has at most SPGEMM_HASH_MAX products, P of them in all (0 < P <
-// 2^32); B has fewer than 2^32 columns (SH_EMPTY is none of them).
-int spgemm_hash_rows(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, uint64_t P, cudaStream_t s) {
+// 2^32); B has fewer than 2^32 columns (SH_EMPTY is none of them). C has about
+// `room` entries (P at most).
+int spgemm_hash_rows(Ctx *c, const Csr *A, const Csr *B, Csr *Cm, uint64_t P, uint64_t room, cudaStream_t s) {
     const uint64_t m = A->n_rows, n = B->n_cols, tiles = (m + SH_ROWS - 1) / SH_ROWS;
     static_assert(SPGEMM_HASH_MAX == SH_H, "a slot per product");
-    // C at the products' upper bound (kept entries <= products), as WARPSORT's
     DevBuf state, off, cols, vals;
     SPG_TRY(off.alloc(csr_off_elems(m) * sizeof(uint64_t), s));
-    SPG_TRY(cols.alloc(csr_alloc_elems(P) * sizeof(uint32_t), s));
-    SPG_TRY(vals.alloc(csr_alloc_elems(P) * sizeof(double), s));
     SPG_TRY(state.alloc((1 + tiles) * sizeof(unsigned long long), s));
-    SPG_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, (1 + tiles) * sizeof(unsigned long long), s));
     unsigned long long *ticket = state.as<unsigned long long>();
     ShArgs a{A->d_off(), A->d_cols(), A->d_vals(), B->d_off(), B->d_cols(), B->d_vals(), m, tiles, ticket, ticket + 1,
-             off.as<uint64_t>(), cols.as<uint32_t>(), vals.as<double>(), c->d_status, c->d_words};
+             off.as<uint64_t>(), nullptr, nullptr, 0, c->d_status, c->d_words};
     // 32-bit indices and sort keys (column, six slot bits) where they fit
     const bool i32 = B->nnz <= 0xFFFFFFFFull, k32 = n <= (1ull << 26);
     auto k = i32 ? (k32 ? sh_tiles<uint32_t, uint32_t> : sh_tiles<uint32_t, unsigned long long>)
                  : (k32 ? sh_tiles<unsigned long long, uint32_t> : sh_tiles<unsigned long long, unsigned long long>);
     SPG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ShSmem)));
-    k<<<(unsigned)tiles, SH_T, sizeof(ShSmem), s>>>(a);
-    SPG_LAUNCH_CHECK();
-    SPG_TRY(c->phase_sync(s));
-    const uint64_t nnz = c->word(0);
+    uint64_t nnz = 0;
+    while (true) {
+        // (the larger one first: the smaller one first took a part of the place that
+        // a freed result had left for it, and the pool mapped memory at every call)
+        SPG_TRY(vals.alloc(csr_alloc_elems(room) * sizeof(double), s));
+        SPG_TRY(cols.alloc(csr_alloc_elems(room) * sizeof(uint32_t), s));
+        SPG_CUDA_TRY(cudaMemsetAsync(state.ptr, 0, (1 + tiles) * sizeof(unsigned long long), s));
+        a.ccols = cols.as<uint32_t>();
+        a.cvals = vals.as<double>();
+        a.room = room;
+        k<<<(unsigned)tiles, SH_T, sizeof(ShSmem), s>>>(a);
+        SPG_LAUNCH_CHECK();
+        SPG_TRY(c->phase_sync(s));
+        nnz = c->word(0);
+        if (nnz <= room) break;
+        room = nnz;  // more entries than expected: again
+    }
+    if (P > RESULT_BOUND) SPG_TRY(fit_arrays(c, nnz, room, cols, vals, s));
     spgemm_install(Cm, m, n, std::move(off), std::move(cols), std::move(vals), nnz);
     return SPG_OK;
 }

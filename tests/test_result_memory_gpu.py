@@ -1,4 +1,5 @@
-"""Results of A + B hold about their own size, also where the sample that sizes their arrays is wrong. Bit-exact against the
+"""Results of A + B and of ROWMERGE's hash rows hold about their own size, also
+where the sample that sizes their arrays is wrong. Bit-exact against the
 oracle."""
 from __future__ import annotations
 
@@ -11,7 +12,7 @@ from spira_gb300 import gen
 from conftest import assert_csr_equal
 
 pytestmark = pytest.mark.gpu
-SAMPLES = 1024
+SAMPLES, ROW_SAMPLES = 1024, 2048
 
 
 def _held(ctx, make):
@@ -70,3 +71,29 @@ def test_add_holds_its_own_size(ctx, case):
     assert_csr_equal(C.download(), oracle.add(H, HB))
     if case != "few":
         assert held <= 1.15 * _own_size(C) + (1 << 20)
+
+
+@pytest.mark.parametrize("case", ["collapsing", "distinct", "misleading"])
+def test_hash_rows_hold_their_own_size(ctx, case):
+    """100 k rows of 8 times 8 products."""
+    m, groups, width = 100_000, 4096, 500_000
+    k = np.arange(ROW_SAMPLES, dtype=np.uint64)
+    part = np.uint64(m // ROW_SAMPLES)
+    sampled = (k * part + (k * np.uint64(0x9E3779B1) >> np.uint64(8)) % part).astype(np.int64)
+    collapse = np.zeros(m, bool)
+    collapse[:] = case == "collapsing"
+    if case == "misleading":
+        collapse[sampled] = True
+    r = np.repeat(np.arange(m, dtype=np.uint32), 8)
+    j = np.tile(np.arange(8, dtype=np.uint32), m)
+    # B's rows: 0..7 have the same eight columns, the others columns of their own
+    ac = np.where(collapse[r], j, 8 + (r * 7 + j * 131) % (groups - 8)).astype(np.uint32)
+    HA = oracle.lock_epochs(m, groups, [(r, ac, gen.sym_unit(gen.hash3(1, 1, np.arange(len(r), dtype=np.uint64))))])
+    br = np.repeat(np.arange(groups, dtype=np.uint32), 8)
+    bj = np.tile(np.arange(8, dtype=np.uint32), groups)
+    bc = np.where(br < 8, bj * 1000, (br * 97 + bj * 60_013) % width).astype(np.uint32)
+    HB = oracle.lock_epochs(groups, width, [(br, bc, gen.sym_unit(gen.hash3(1, 2, np.arange(len(br), dtype=np.uint64))))])
+    A, B = _load(ctx, HA), _load(ctx, HB)
+    C, held = _held(ctx, lambda: A.spgemm(B, sg.SPGEMM_VARIANTS["rowmerge"]))
+    assert_csr_equal(C.download(), oracle.spgemm(HA, HB))
+    assert held <= 1.15 * _own_size(C) + (1 << 20)
