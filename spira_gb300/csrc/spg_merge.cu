@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(MT_T, MT_PER_SM) mt_tiles(MtArgs a) {
             }
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
-            // rows of the thread's eight entries: a scan over the marks
+            // rows of the thread's MT_E entries: a scan over the marks
             uint32_t mw[MT_E / 2], sum = 0;
 #pragma unroll
             for (int j = 0; j < MT_E / 2; ++j) mw[j] = reinterpret_cast<const uint32_t *>(S.mark)[t * (MT_E / 2) + j];
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(MT_T, MT_PER_SM) mt_tiles(MtArgs a) {
                 }
             }
             __syncthreads();
-            // kept entries before each word: every warp for itself, three words a lane
+            // kept entries before each word: every warp for itself, MT_KW / 32 words a lane
             uint32_t n3 = 0;
 #pragma unroll
             for (int k = 0; k < MT_KW / 32; ++k) n3 += __popc(S.keep[lane * (MT_KW / 32) + k]);

@@ -426,8 +426,7 @@ int radix_sort_pairs_u64(Ctx *c, uint64_t *d_keys, uint32_t *d_vals, uint64_t n,
 //     rows (128 x 16, 256 x 16 and 768 x 16 entries) keep few threads idle.
 // In every network the key carries the entry's position in its row, so the
 // sorted order is the stable order. Columns of more than 26 bits, or a row
-// longer than TS_MAX, make the sort report failure; callers then sort
-// globally. Work lists are filled with atomics, in no particular order: every
+// longer than TS_MAX, make the sort report failure (the row tiles take over). Work lists are filled with atomics, in no particular order: every
 // row's output places are fixed by s_off, so the result does not depend on
 // that order.
 // ---------------------------------------------------------------------------
@@ -490,7 +489,7 @@ __global__ void __launch_bounds__(256) seg_count(const uint64_t *__restrict__ s_
 // lists[base_c + k] for class c (base_c = the rows of the listed classes
 // below it; classes 7..9 are the tile kernels' lists). cur[c]: fill cursors.
 __global__ void __launch_bounds__(256) seg_place(const uint32_t *__restrict__ cols, const uint64_t *__restrict__ s_off,
-                                                 uint64_t n_rows, int cbits, const unsigned *__restrict__ ctr,
+                                                 uint64_t n_rows, const unsigned *__restrict__ ctr,
                                                  unsigned *__restrict__ cur, uint32_t *__restrict__ lists, SegOut o) {
     __shared__ unsigned sc[10], sbase[10], base[10];
     if (ctr[SC_OVERFLOW]) return;  // (set by the launch before: the rest of the plan would be thrown away)
@@ -687,7 +686,7 @@ __device__ __forceinline__ void warp_bitonic_looped(K (&key)[E], int lane) {
 // twice the registers.)
 template <int E, class K>
 __device__ __forceinline__ void sort_medium_row(const uint32_t *__restrict__ cols, uint64_t b, uint32_t L, uint64_t r,
-                                                int cbits, const SegOut &o, int lane) {
+                                                const SegOut &o, int lane) {
     K key[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
@@ -728,7 +727,7 @@ template <class K>
 __global__ void __launch_bounds__(256, sizeof(K) == 8 ? 2 : 4) seg_medium_sort(const uint32_t *__restrict__ cols,
                                                        const uint64_t *__restrict__ s_off,
                                                        const uint32_t *__restrict__ lists,
-                                                       const unsigned *__restrict__ ctr, int cbits, SegOut o) {
+                                                       const unsigned *__restrict__ ctr, SegOut o) {
     const unsigned n = ctr[SC_OVERFLOW] ? 0 : ctr[SC_LIST + 6];  // class 6 heads the lists
     const int lane = threadIdx.x & 31;
     const unsigned warps = gridDim.x * (blockDim.x >> 5);
@@ -736,10 +735,10 @@ __global__ void __launch_bounds__(256, sizeof(K) == 8 ? 2 : 4) seg_medium_sort(c
         const uint64_t r = lists[k];
         const uint64_t b = s_off[r];
         const uint32_t L = (uint32_t)(s_off[r + 1] - b);
-        if (L <= 64) sort_medium_row<2, K>(cols, b, L, r, cbits, o, lane);
-        else if (L <= 128) sort_medium_row<4, K>(cols, b, L, r, cbits, o, lane);
-        else if (L <= 256) sort_medium_row<8, K>(cols, b, L, r, cbits, o, lane);
-        else sort_medium_row<16, K>(cols, b, L, r, cbits, o, lane);
+        if (L <= 64) sort_medium_row<2, K>(cols, b, L, r, o, lane);
+        else if (L <= 128) sort_medium_row<4, K>(cols, b, L, r, o, lane);
+        else if (L <= 256) sort_medium_row<8, K>(cols, b, L, r, o, lane);
+        else sort_medium_row<16, K>(cols, b, L, r, o, lane);
     }
 }
 
@@ -982,14 +981,14 @@ int seg_sort(Ctx *c, const uint32_t *cols, const uint64_t *s_off, uint64_t m, ui
     const unsigned gr = grid_for(n_rows, 256, (unsigned)c->n_sms * 8);
     seg_count<<<gr, 256, 0, s>>>(s_off, n_rows, ctr);
     SPG_LAUNCH_CHECK();
-    seg_place<<<gr, 256, 0, s>>>(cols, s_off, n_rows, cbits, ctr, cur, lists, o);
+    seg_place<<<gr, 256, 0, s>>>(cols, s_off, n_rows, ctr, cur, lists, o);
     SPG_LAUNCH_CHECK();
     seg_short_sort<<<grid_for((n_rows + 31) / 32, 8, (unsigned)c->n_sms * 16), 256, 0, s>>>(cols, s_off, n_rows, ctr, o);
     SPG_LAUNCH_CHECK();
     // (8 blocks per SM: twice what fits at once, which balanced rows of
     // unequal length better than one wave)
-    if (cbits <= 22) seg_medium_sort<uint32_t><<<(unsigned)c->n_sms * 8, 256, 0, s>>>(cols, s_off, lists, ctr, cbits, o);
-    else seg_medium_sort<uint64_t><<<(unsigned)c->n_sms * 8, 256, 0, s>>>(cols, s_off, lists, ctr, cbits, o);
+    if (cbits <= 22) seg_medium_sort<uint32_t><<<(unsigned)c->n_sms * 8, 256, 0, s>>>(cols, s_off, lists, ctr, o);
+    else seg_medium_sort<uint64_t><<<(unsigned)c->n_sms * 8, 256, 0, s>>>(cols, s_off, lists, ctr, o);
     SPG_LAUNCH_CHECK();
     SPG_TRY((launch_tile_sort<TS0_T, TS0_I>(c, cols, s_off, lists, ctr, 0, m / (SEG_MEDIUM + 1) + 1, cbits,
                                                    o, ovf, s)));

@@ -268,8 +268,9 @@ __device__ __forceinline__ void rt_minmax(Smem &S, uint32_t lo, bool on, uint32_
 // S (not yet synchronised; S.cnt is zero up to counter E) by (row, column,
 // position), keeps the last of every run of equal columns of a row unless its
 // value is zero, and returns the number kept (in every thread). S.keep / kpre
-// have the keep bits by sorted place; o[i] is the kept entry's index among the
-// kept ones, or ~0 for a dropped one; v[i] its value.
+// have the keep bits by sorted place; pk[i] is the kept entry's index among the
+// kept ones, or ~0 for a dropped one; v[i] its value. REPEATS: for matrices
+// whose long rows may have more entries than columns.
 template <bool REPEATS, int T, int CAP, bool APART>
 __device__ __forceinline__ uint32_t rt_order(RtSmem<T, CAP, APART> &S, const uint32_t (&c)[CAP / T],
                                              const double *__restrict__ vals, int E, int cbits, bool keep_zeros,
