@@ -593,11 +593,11 @@ int sort_keys(Ctx *c, const uint32_t *rows, const uint32_t *cols, uint64_t m, ui
 }
 
 int sort_dedup(Ctx *c, const uint32_t *rows, const uint32_t *cols, const double *vals, uint64_t m,
-               uint64_t n_rows, uint64_t n_cols, Delta &D, cudaStream_t s) {
+               uint64_t n_rows, uint64_t n_cols, bool sorted, Delta &D, cudaStream_t s) {
     const int cbits = bits_for(n_cols);
     const unsigned g = grid_for(m, LB, (unsigned)c->n_sms * 16);
     DevBuf keys, idx, pos;
-    SPG_TRY(sort_keys(c, rows, cols, m, n_rows, n_cols, keys, idx, false, s));
+    SPG_TRY(sort_keys(c, rows, cols, m, n_rows, n_cols, keys, idx, sorted, s));
     SPG_TRY(pos.alloc((m + 1) * sizeof(uint64_t), s));
     lock_last_flags<<<g, LB, 0, s>>>(keys.as<uint64_t>(), m, pos.as<uint64_t>());
     SPG_LAUNCH_CHECK();
@@ -991,9 +991,9 @@ int merge_epoch(Ctx *c, const Csr *A, const uint32_t *rows, const uint32_t *cols
     bool done = false;
     SPG_TRY(build_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, bits_for(A->n_cols), pre->clustered > 0, true, abort,
                                &D, &done, s));
-    if (!done) {  // (no memory to sort rows too long for the tiles apart)
+    if (!done) {  // (mostly rows too long for the tiles, or no memory to sort those apart)
         Delta d;
-        SPG_TRY(sort_dedup(c, rows, cols, vals, m, n, A->n_cols, d, s));
+        SPG_TRY(sort_dedup(c, rows, cols, vals, m, n, A->n_cols, !pre->unsorted && !again.rows.ptr, d, s));
         SPG_TRY(launch_row_offsets(c, d.row.as<uint32_t>(), d.u, n, D.off.as<uint64_t>(), s));
         D.cols = std::move(d.col);
         D.vals = std::move(d.val);

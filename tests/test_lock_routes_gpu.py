@@ -132,3 +132,31 @@ def test_lock_mean_row_length_rule(ctx, mean, n_cols):
     A = sg.Csr(ctx, n, n_cols)
     A.lock(rows, cols, vals)
     assert_csr_equal(A.download(), oracle.lock_epochs(n, n_cols, [(rows, cols, vals)]))
+
+
+@pytest.mark.parametrize("repeats", [False, True])
+@pytest.mark.parametrize("zeros", [False, True])
+def test_later_epoch_in_order_of_long_rows(ctx, repeats, zeros):
+    """An epoch already in (row, column) order, of rows above 12 288 inserts,
+    into a matrix with and without stored zeros (whose deletes join it)."""
+    n, n_cols, per = 6, 300_000, 20_000
+    first = _hub_inserts(n, n_cols, [(r, 5000) for r in range(n)], 3)
+    H = oracle.lock_epochs(n, n_cols, [first])
+    A = sg.Csr(ctx, n, n_cols)
+    if zeros:
+        v = H.vals.copy()
+        v[::5] = 0.0
+        A.load(H.off, H.cols, v)
+        rows_of = np.repeat(np.arange(n, dtype=np.uint32), np.diff(H.off.astype(np.int64)))
+        first = (rows_of[v != 0.0], H.cols[v != 0.0], v[v != 0.0])  # (zeros of dirty rows go away)
+    else:
+        A.lock(*first)
+    r = np.repeat(np.arange(n, dtype=np.uint32), per)
+    c = np.sort(gen.below(gen.hash3(4, 1, np.arange(len(r), dtype=np.uint64)), n_cols).reshape(n, per), axis=1)
+    if not repeats:
+        c = (np.arange(per, dtype=np.uint32) * 14 + np.arange(n, dtype=np.uint32)[:, None]).astype(np.uint32)
+    v = gen.sym_unit(gen.hash3(4, 2, np.arange(len(r), dtype=np.uint64)))
+    v[::9] = 0.0
+    e = (r, c.reshape(-1).astype(np.uint32), v)
+    A.lock(*e)
+    assert_csr_equal(A.download(), oracle.lock_epochs(n, n_cols, [first, e]), check_capacity=not zeros)
