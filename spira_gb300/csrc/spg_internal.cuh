@@ -119,7 +119,7 @@ struct Ctx {
     // per synchronisation (14.3 against 9.4 us for launch, word and wait). A
     // context runs one operation at a time, and its kernels store all the words
     // that it reads.
-    static constexpr int N_WORDS = 8;
+    static constexpr int N_WORDS = 16;
     unsigned long long *h_words = nullptr;
     unsigned long long *d_words = nullptr;
     uint64_t word(int k) const { return *(volatile unsigned long long *)(h_words + k); }

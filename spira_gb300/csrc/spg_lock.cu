@@ -85,13 +85,20 @@ __device__ __forceinline__ uint32_t column_gap(uint32_t a, uint32_t b) { return 
 // stats[5] += a sample of the inserts that 32 others of their row follow: every
 // fourth insert, by 24 lanes of each warp's 32 (3 / 16 of all). stats[7] += a
 // sample of the inserts whose successor in the row is nearer than `near`
-// columns, less those whose successor is not: every fourth insert.
-template <bool VEC>
+// columns, less those whose successor is not: every fourth insert. stats[8] += a
+// sample of the inserts that are of one row with the 32nd and the 64th after
+// them (an eighth of all), stats[9] += a sample of those whose successor is of an
+// earlier row (every fourth): what they say of inserts in no order, hub_rows below.
+// Both with HUBS only, for up to FEW_STAGED inserts: the registers that they take
+// cost 18 us of 132 for 64 M inserts, and nothing while the blocks are few.
+constexpr int N_STATS = 10;
+
+template <bool VEC, bool HUBS>
 __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *__restrict__ cols, uint64_t m,
                              int cbits, uint64_t n_rows, uint32_t near, uint64_t *__restrict__ off,
                              unsigned *__restrict__ stats,
                              unsigned long long *__restrict__ words) {
-    unsigned mr = 0, mc = 0, hits = 0;
+    unsigned mr = 0, mc = 0, hits = 0, triples = 0, falls = 0;
     int score = 0;
     bool d = false, g = false, e = false, gap = false;
     if (off && blockIdx.x == 0 && threadIdx.x == 0) {  // the rows up to the first insert's and after the last one's
@@ -112,6 +119,11 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
             }
             const uint32_t r32 = __shfl_down_sync(0xffffffffu, r4.x, 8);
             if (4 * q + 32 < 4 * n4 && (threadIdx.x & 31) < 24) hits += r32 == r4.x ? 1u : 0u;
+            if constexpr (HUBS) {
+                const uint32_t r64 = __shfl_down_sync(0xffffffffu, r4.x, 16);
+                if (4 * q + 64 < 4 * n4 && (threadIdx.x & 31) < 16) triples += r32 == r4.x && r64 == r4.x ? 1u : 0u;
+                falls += r4.x > r4.y ? 1u : 0u;
+            }
             uint32_t rn = __shfl_down_sync(0xffffffffu, r4.x, 1), cn = __shfl_down_sync(0xffffffffu, c4.x, 1);
             const bool have_next = ok && 4 * q + 4 < m;
             if (have_next && ((threadIdx.x & 31) == 31 || q + 1 >= n4)) {
@@ -143,10 +155,14 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
         const uint32_t r = rows[i], c = cols[i];
         mr = max(mr, r);
         mc = max(mc, c);
-        if (!VEC && (i & 3) == 0 && ((i >> 2) & 31) < 24 && i + 32 < m) hits += rows[i + 32] == r ? 1u : 0u;
+        if (!VEC && (i & 3) == 0 && ((i >> 2) & 31) < 24 && i + 32 < m && rows[i + 32] == r) {
+            ++hits;
+            if (HUBS && ((i >> 2) & 31) < 16 && i + 64 < m) triples += rows[i + 64] == r ? 1u : 0u;
+        }
         if (i + 1 < m) {
             const uint32_t r2 = rows[i + 1], c2 = cols[i + 1];
             const uint64_t k = ((uint64_t)r << cbits) | c, k2 = ((uint64_t)r2 << cbits) | c2;
+            if (HUBS && !VEC && (i & 3) == 0 && r > r2) ++falls;
             if (!VEC && (i & 3) == 0 && r == r2) score += column_gap(c, c2) < near ? 1 : -1;
             d |= k > k2;
             e |= k >= k2;
@@ -160,12 +176,16 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
         mc = max(mc, __shfl_xor_sync(0xffffffffu, mc, o));
     }
     hits = __reduce_add_sync(0xffffffffu, hits);
+    if constexpr (HUBS) {
+        triples = __reduce_add_sync(0xffffffffu, triples);
+        falls = __reduce_add_sync(0xffffffffu, falls);
+    }
     score = __reduce_add_sync(0xffffffffu, score);
     const unsigned flags = (__any_sync(0xffffffffu, d) ? 1u : 0u) | (__any_sync(0xffffffffu, g) ? 2u : 0u) |
                            (__any_sync(0xffffffffu, e) ? 4u : 0u) | (__any_sync(0xffffffffu, gap) ? 8u : 0u);
     // one set of atomics per block: per-warp atomics on the same two words
     // serialise at L2 and cost more than the pass itself
-    __shared__ unsigned s_mr[LB / 32], s_mc[LB / 32], s_fl[LB / 32], s_hits[LB / 32];
+    __shared__ unsigned s_mr[LB / 32], s_mc[LB / 32], s_fl[LB / 32], s_hits[LB / 32], s_triples[LB / 32], s_falls[LB / 32];
     __shared__ int s_score[LB / 32];
     const int w = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) {
@@ -174,10 +194,14 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
         s_fl[w] = flags;
         s_hits[w] = hits;
         s_score[w] = score;
+        if constexpr (HUBS) {
+            s_triples[w] = triples;
+            s_falls[w] = falls;
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned bm = 0, bc = 0, bf = 0, bh = 0;
+        unsigned bm = 0, bc = 0, bf = 0, bh = 0, bt = 0, bd = 0;
         int bs = 0;
         for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
             bm = max(bm, s_mr[i]);
@@ -185,6 +209,10 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
             bf |= s_fl[i];
             bh += s_hits[i];
             bs += s_score[i];
+            if constexpr (HUBS) {
+                bt += s_triples[i];
+                bd += s_falls[i];
+            }
         }
         atomicMax(stats, bm);
         atomicMax(stats + 1, bc);
@@ -194,8 +222,10 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
         if (bf & 2u) stats[3] = 1u;
         if (bf & 4u) stats[4] = 1u;
         if (bf & 8u) stats[6] = 1u;
-        if (last_block(stats + 8)) {
-            for (int i = 0; i < 8; ++i) store_word(words, i, *(volatile unsigned *)(stats + i));
+        if (bt) atomicAdd(stats + 8, bt);
+        if (bd) atomicAdd(stats + 9, bd);
+        if (last_block(stats + N_STATS)) {
+            for (int i = 0; i < N_STATS; ++i) store_word(words, i, *(volatile unsigned *)(stats + i));
         }
     }
 }
@@ -521,10 +551,30 @@ struct Prepared {
     unsigned unsorted = 1, ungrouped = 1, not_strict = 1;
     uint64_t long_hits = 0;  // sampled inserts that 32 others of their row follow (3 / 16 of the inserts looked at)
     int64_t clustered = 0;   // sampled inserts with a near successor in their row, less those with a far one
+    double pairs = 0.0, triples = 0.0;  // the chance that two, three inserts are of one row (of inserts in no order)
     bool ready = false;
     DevBuf off;             // a first lock: the staged rows' offsets ...
     bool have_off = false;  // ... when the rows are grouped and no step between them was long
 };
+
+// Whether inserts in no order go to the global sort, as rows that no block
+// takes hold much of them. With K such rows of equal length, a share f of the
+// inserts, and short ones besides, two inserts are of one row with chance f^2 /
+// K and three with f^3 / K^2: their square and ratio give f and the rows' length.
+// From half of the inserts on, sorting those rows apart is slower than sorting
+// all (row sort, attempt and tiles / global, later epochs: 2.5 M in 10 rows 499 /
+// 392 us, 3 M in 200 rows 701 / 507), in small epochs from a tenth on (5 rows of
+// 13 000 430 / 351, and 100 k others 468 / 393), where launches are what is paid;
+// below, it is faster (12 M with one row of 2 M: 979 / 1461). Above 4 M inserts
+// nothing is sampled, and the plan of the tiles finds out (10 M in 10 rows 1073 /
+// 831).
+constexpr uint64_t HUB_FEW = 1u << 19;
+
+bool hub_rows(const Prepared &pre, uint64_t m) {
+    if (pre.triples == 0.0) return false;
+    const double length = (double)m * pre.triples / pre.pairs, share = pre.pairs * pre.pairs / pre.triples;
+    return length > 12288.0 && share > (m <= HUB_FEW ? 0.1 : 0.5);
+}
 
 // The staged (grouped) rows' offsets.
 int staged_offsets(Ctx *c, Prepared *pre, const uint32_t *rows, uint64_t m, uint64_t n_rows, DevBuf &off,
@@ -938,14 +988,15 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
     return SPG_OK;
 }
 
-// The general merge of an epoch (rows non-decreasing) into the old CSR.
+// The general merge of an epoch into the old CSR (rows in any order only without
+// stored zeros in it).
 template <class AllocOut>
 int merge_epoch(Ctx *c, const Csr *A, const uint32_t *rows, const uint32_t *cols, const double *vals, uint64_t m,
                 const unsigned long long *abort, AllocOut alloc_out, Prepared *pre, DevBuf &new_off, DevBuf &out_cols,
                 DevBuf &out_vals, uint64_t *new_nnz, uint64_t *u, cudaStream_t s) {
     const uint64_t n = A->n_rows;
     DevBuf s_off;
-    SPG_TRY(staged_offsets(c, pre, rows, m, n, s_off, s));
+    if (!pre->ungrouped) SPG_TRY(staged_offsets(c, pre, rows, m, n, s_off, s));
     StagedSorted again;
     if (A->may_have_zeros && A->nnz) {
         // Explicit old zeros of dirty rows become deletes staged before the epoch.
@@ -989,9 +1040,11 @@ int merge_epoch(Ctx *c, const Csr *A, const uint32_t *rows, const uint32_t *cols
     // the epoch's last writes, zeros kept (they delete), in (row, column) order
     GroupedOut D;
     bool done = false;
-    SPG_TRY(build_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, bits_for(A->n_cols), pre->clustered > 0, true, abort,
-                               &D, &done, s));
-    if (!done) {  // (mostly rows too long for the tiles, or no memory to sort those apart)
+    if (!pre->ungrouped)
+        SPG_TRY(build_grouped_rows(c, cols, vals, s_off.as<uint64_t>(), m, n, bits_for(A->n_cols), pre->clustered > 0, true,
+                                   abort, &D, &done, s));
+    if (!done) {  // mostly rows too long for the tiles (or no memory to sort those apart)
+        if (!D.off.ptr) SPG_TRY(D.off.alloc(csr_off_elems(n) * sizeof(uint64_t), s));
         Delta d;
         SPG_TRY(sort_dedup(c, rows, cols, vals, m, n, A->n_cols, !pre->unsorted && !again.rows.ptr, d, s));
         SPG_TRY(launch_row_offsets(c, d.row.as<uint32_t>(), d.u, n, D.off.as<uint64_t>(), s));
@@ -1019,21 +1072,19 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
     Prepared pre;
     if (m) {
         DevBuf stats;
-        SPG_TRY(stats.alloc(9 * sizeof(unsigned), s));
-        SPG_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, 9 * sizeof(unsigned), s));
+        SPG_TRY(stats.alloc((N_STATS + 1) * sizeof(unsigned), s));
+        SPG_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, (N_STATS + 1) * sizeof(unsigned), s));
         if (!A->built) SPG_TRY(pre.off.alloc(csr_off_elems(A->n_rows) * sizeof(uint64_t), s));
-        if (((uintptr_t)rows | (uintptr_t)cols) % 16 == 0)
-            lock_prepare<true><<<grid_for((m + 3) / 4, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
-                rows, cols, m, bits_for(A->n_cols), A->n_rows, near_columns(A->n_cols), pre.off.as<uint64_t>(), stats.as<unsigned>(),
-                c->d_words);
-        else
-            lock_prepare<false><<<grid_for(m, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
-                rows, cols, m, bits_for(A->n_cols), A->n_rows, near_columns(A->n_cols), pre.off.as<uint64_t>(), stats.as<unsigned>(),
-                c->d_words);
+        const bool vec = ((uintptr_t)rows | (uintptr_t)cols) % 16 == 0, hubs = m <= FEW_STAGED;
+        auto k = vec ? (hubs ? lock_prepare<true, true> : lock_prepare<true, false>)
+                     : (hubs ? lock_prepare<false, true> : lock_prepare<false, false>);
+        k<<<grid_for(vec ? (m + 3) / 4 : m, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
+            rows, cols, m, bits_for(A->n_cols), A->n_rows, near_columns(A->n_cols), pre.off.as<uint64_t>(),
+            stats.as<unsigned>(), c->d_words);
         SPG_LAUNCH_CHECK();
         SPG_TRY(c->phase_sync(s));
-        unsigned h[8];
-        for (int i = 0; i < 8; ++i) h[i] = (unsigned)c->word(i);
+        unsigned h[N_STATS];
+        for (int i = 0; i < N_STATS; ++i) h[i] = (unsigned)c->word(i);
         if ((uint64_t)h[0] >= A->n_rows)
             return set_error(SPG_ERR_OUT_OF_RANGE, "spira::matrix: row_index out of range (%u >= %llu)", h[0],
                              (unsigned long long)A->n_rows);
@@ -1045,6 +1096,12 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
         pre.not_strict = h[4];
         pre.long_hits = h[5];
         pre.clustered = (int)h[7];
+        // (fewer than 32 say nothing; in no order every other insert or so is followed
+        // by an earlier row's)
+        if (h[8] >= 32 && (double)h[9] * 4.0 > 0.25 * (double)m * (1.0 - std::min(1.0, (double)h[5] * 16.0 / 3.0 / (double)m))) {
+            pre.pairs = (double)h[5] * 16.0 / 3.0 / (double)m;
+            pre.triples = (double)h[8] * 8.0 / (double)m;
+        }
         pre.have_off = pre.off.ptr && !h[3] && !h[6];
         pre.ready = true;
     }
@@ -1052,10 +1109,11 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
     const bool has_old = A->built;
     if (has_old && m == 0) return SPG_OK;  // no dirty row: Spira's merge leaves the CSR as it is
     StagedSorted sorted;
-    // Rows in any order are sorted by row, and row-grouped from here on; not
-    // for a first lock of rows that the row kernels cannot all take (12 288
-    // entries): it goes to the global sort.
-    if (m && pre.ungrouped && (has_old || m <= 12288 * n)) {
+    // Rows in any order are sorted by row, and row-grouped from here on; but they
+    // go to the global sort where the row kernels cannot take most of them (12 288
+    // inserts a row), and no stored zeros ask for the rows' offsets.
+    const bool global = pre.ungrouped && (has_old ? !A->may_have_zeros && hub_rows(pre, m) : m > 12288 * n || hub_rows(pre, m));
+    if (m && pre.ungrouped && !global) {
         SPG_TRY(sort_staged_rows(c, rows, cols, vals, m, bits_for(n), sorted, s));
         rows = sorted.rows.as<uint32_t>();
         cols = sorted.cols.as<uint32_t>();
@@ -1083,7 +1141,7 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
     // more than it takes (1 M rows of 10, insert by insert / general merge: 100 k
     // inserts 274 / 385 us, 1.25 M 430 / 507, 2.5 M 551 / 560; 30 k rows of 1000:
     // 300 k 466 / 663; 3 M, 100 to a row, 1216 with the attempt / 862).
-    if (!A->may_have_zeros && m <= A->nnz / 5 && m <= 32 * n && 16 * pre.long_hits <= m) {
+    if (!global && !A->may_have_zeros && m <= A->nnz / 5 && m <= 32 * n && 16 * pre.long_hits <= m) {
         SPG_TRY(alloc_out(m));
         SPG_TRY(merge_small_delta(c, {A->d_off(), A->d_cols(), A->d_vals(), A->nnz}, n, rows, cols, vals, m, abort,
                                   new_off.as<uint64_t>(), out_cols.as<uint32_t>(), out_vals.as<double>(), &new_nnz, &u,

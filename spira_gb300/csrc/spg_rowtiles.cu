@@ -62,7 +62,8 @@ constexpr int RT_FEW_CBITS = 14;
 constexpr unsigned RT_STATUS_TIMEOUT = 0x20u;
 
 // Counters at the head of the scratch words.
-enum : int { RC_PLAN_TICKET = 0, RC_TICKET = 1, RC_TILES = 2, RC_BIG = 3, RC_OVERFLOW = 4, RC_MID = 5, RC_MID_TICKET = 6, RC_BIG_TICKET = 7, RC_HUGE = 8, RC_HUGE_ENTRIES = 9, RC_N = 10 };
+enum : int { RC_PLAN_TICKET = 0, RC_TICKET = 1, RC_TILES = 2, RC_BIG = 3, RC_OVERFLOW = 4, RC_MID = 5, RC_MID_TICKET = 6, RC_BIG_TICKET = 7, RC_HUGE = 8, RC_N = 9 };
+constexpr int RC_HUGE_BITS = 24;  // RC_HUGE: rows in the low bits (2^32 / 12 289 at most), their entries above
 
 struct RtArgs {
     const uint32_t *cols;
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(RP_T) rt_plan(RtArgs a) {
     const int parts = (int)min((uint64_t)RP_SUB, (s_off[nr] - s_off[0]) / RP_PART + 1);
     const int per = (nr + parts - 1) / parts;
     const int p0 = min(nr, warp * per), p1 = warp < parts ? min(nr, p0 + per) : p0;
-    uint32_t n = 0;
+    uint32_t n = 0, huge = 0;
     for (int r = p0; r < p1;) {
         if (lane == 0) s_list[p0 + n] = (uint16_t)r;
         ++n;
@@ -132,22 +133,27 @@ __global__ void __launch_bounds__(RP_T) rt_plan(RtArgs a) {
         if (e == r) {  // longer than a tile
             const uint64_t L = s_off[r + 1] - s_off[r];
             if (lane == 0) {
-                if (L > (uint64_t)RT_BIG) {
-                    if (!a.huge_ready) {
-                        a.ctr[RC_OVERFLOW] = 1ull;
-                        a.huge[atomicAdd(a.ctr + RC_HUGE, 1ull)] = (uint32_t)(r0 + r);
-                        atomicAdd(a.ctr + RC_HUGE_ENTRIES, (unsigned long long)L);
-                    }
-                } else if (L > (uint64_t)RT_MID) a.longer[a.n_longer - 1 - atomicAdd(a.ctr + RC_BIG, 1ull)] = (uint32_t)(r0 + r);
-                else {
-                    a.longer[atomicAdd(a.ctr + RC_MID, 1ull)] = (uint32_t)(r0 + r);
-                }
+                if (L > (uint64_t)RT_BIG) ++huge;
+                else if (L > (uint64_t)RT_MID) a.longer[a.n_longer - 1 - atomicAdd(a.ctr + RC_BIG, 1ull)] = (uint32_t)(r0 + r);
+                else a.longer[atomicAdd(a.ctr + RC_MID, 1ull)] = (uint32_t)(r0 + r);
             }
             ++e;
         }
         r = e;
     }
     if (lane == 0) s_n[warp] = n;
+    __syncwarp();
+    if (!a.huge_ready && __shfl_sync(0xffffffffu, huge, 0)) {  // (listed here, 32 tiles at a time: an atomic each in the loop waits)
+        if (lane == 0) a.ctr[RC_OVERFLOW] = 1ull;
+        for (uint32_t k0 = 0; k0 < n; k0 += 32) {
+            const int r = k0 + lane < n ? s_list[p0 + k0 + lane] : p0;
+            const uint64_t L = k0 + lane < n ? s_off[r + 1] - s_off[r] : 0;
+            if (L > (uint64_t)RT_BIG) {
+                const unsigned long long at = atomicAdd(a.ctr + RC_HUGE, (unsigned long long)L << RC_HUGE_BITS | 1ull);
+                a.huge[at & ((1ull << RC_HUGE_BITS) - 1)] = (uint32_t)(r0 + r);
+            }
+        }
+    }
     __syncthreads();
     uint32_t before = 0, total = 0;
 #pragma unroll
@@ -589,8 +595,8 @@ __global__ void __launch_bounds__(RT_T, RT_PER_SM) rt_tiles(RtArgs a) {
     if (a.ctr[RC_OVERFLOW]) {
         if (blockIdx.x == 0 && t == 0) {
             store_word(a.words, 0, 1ull);
-            store_word(a.words, 1, a.ctr[RC_HUGE]);
-            store_word(a.words, 2, a.ctr[RC_HUGE_ENTRIES]);
+            store_word(a.words, 1, a.ctr[RC_HUGE] & ((1ull << RC_HUGE_BITS) - 1));
+            store_word(a.words, 2, a.ctr[RC_HUGE] >> RC_HUGE_BITS);
         }
         return;
     }
@@ -807,10 +813,9 @@ int build_grouped_rows(Ctx *c, const uint32_t *cols, const double *vals, const u
         if (c->word(0) == 0) break;
         H.n = c->word(1);
         H.entries = c->word(2);
-        // mostly such rows, and grouped as they came: the global sort (300 rows of
-        // 13 000 in 5 M columns 0.45 ms, apart 0.58); rows sorted before are no
-        // use to it (one such row in 100 k of ten, shuffled: 0.39 / 0.30)
-        if (!abort && 2 * H.entries > m) return SPG_OK;
+        // mostly such rows: the global sort (300 rows of 13 000 in 5 M columns 0.45
+        // ms, apart 0.58)
+        if (2 * H.entries > m) return SPG_OK;
         const int rc = order_huge_rows(c, cols, vals, s_off, a.huge, cbits, keep_zeros, &H, a.off, s);
         if (rc == SPG_ERR_NO_MEMORY) return SPG_OK;  // (the global sort needs less)
         SPG_TRY(rc);

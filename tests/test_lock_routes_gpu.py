@@ -160,3 +160,29 @@ def test_later_epoch_in_order_of_long_rows(ctx, repeats, zeros):
     e = (r, c.reshape(-1).astype(np.uint32), v)
     A.lock(*e)
     assert_csr_equal(A.download(), oracle.lock_epochs(n, n_cols, [first, e]), check_capacity=not zeros)
+
+
+@pytest.mark.parametrize("order", ["any", "streams"])
+@pytest.mark.parametrize("n_rows,hubs,others", [
+    (3000, 5, 0), (3000, 5, 20_000), (3000, 1, 90_000), (3000, 1, 300_000), (8, 8, 0), (40, 40, 2000),
+])
+def test_lock_unordered_with_hub_rows(ctx, n_rows, hubs, others, order):
+    """Unordered inserts with some to all of them in rows of more than a block
+    takes, in a first and a later lock: what the sample says changes the way, not
+    the result. Streams: three ordered ones, one after another."""
+    n_cols, epochs = 50_000, []
+    for seed in (5, 6):
+        m = hubs * 13_000 + others
+        ctr = np.arange(m, dtype=np.uint64)
+        r = np.where(ctr < hubs * 13_000, (ctr % np.uint64(hubs)) * np.uint64(max(1, n_rows // hubs)),
+                     gen.hash3(seed, 1, ctr) % np.uint64(n_rows)).astype(np.uint32)
+        p = np.argsort(gen.hash3(seed, 2, ctr), kind="stable")
+        if order == "streams":
+            p = np.concatenate([q[np.argsort(r[q], kind="stable")] for q in np.array_split(p, 3)])
+        v = gen.sym_unit(gen.hash3(seed, 4, ctr))
+        v[::8] = 0.0
+        epochs.append((r[p], gen.below(gen.hash3(seed, 3, ctr), n_cols)[p], v[p]))
+    A = sg.Csr(ctx, n_rows, n_cols)
+    for k in (1, 2):
+        A.lock(*epochs[k - 1])
+        assert_csr_equal(A.download(), oracle.lock_epochs(n_rows, n_cols, epochs[:k]))
