@@ -908,7 +908,7 @@ int first_lock(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t *cols, const
         // passes (3 333 rows of 3000 on 4096: 520 / 350; 1 250 of 8000 on 16 384:
         // 498 / 443; 5 000 of 2000 on 4096: 387 / 333).
         const uint64_t mean = m / n;
-        const bool radix = (mean >= 2400 && mean <= 4096) || (mean >= 1536 && cbits <= 14);
+        const bool radix = (mean >= 2400 && mean <= 4096) || (mean >= 1536 && mean <= 12288 && cbits <= 14);
         const bool tiles = (m <= FEW_STAGED && !radix) || cbits > ROW_CLASS_CBITS || 
                            (!radix && (8 * pre->long_hits > m + m / 32 || pre->clustered < 0));
         DevBuf s_off, kept, scols, svals;
