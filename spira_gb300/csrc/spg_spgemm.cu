@@ -53,7 +53,8 @@ constexpr int SG_SAMPLE_G = 8, SG_SAMPLE_BLOCKS = SG_SAMPLES * SG_SAMPLE_G / GB;
 __device__ void sg_sample_rows(const uint64_t *__restrict__ aoff, const uint32_t *__restrict__ acols,
                                const uint64_t *__restrict__ boff, const uint32_t *__restrict__ bcols, uint64_t m,
                                unsigned long long *__restrict__ ctr) {
-    constexpr uint32_t EMPTY = 0xFFFFFFFFu, SLOTS = SPGEMM_HASH_MAX;
+    constexpr uint32_t EMPTY = 0xFFFFFFFFu, SLOTS = 2 * SPGEMM_HASH_MAX;  // (half full at most: full tables took 30 us more)
+    static_assert(SLOTS == 128, "seven hash bits");
     __shared__ uint32_t s_key[GB / SG_SAMPLE_G][SLOTS];
     const int t = threadIdx.x, l = t % SG_SAMPLE_G;
     uint32_t *key = s_key[t / SG_SAMPLE_G];
@@ -70,13 +71,13 @@ __device__ void sg_sample_rows(const uint64_t *__restrict__ aoff, const uint32_t
 #pragma unroll
     for (int o = 1; o < SG_SAMPLE_G; o <<= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
     uint32_t distinct = 0;
-    if (p > 0 && p <= (uint64_t)SLOTS) {
+    if (p > 0 && p <= (uint64_t)SPGEMM_HASH_MAX) {
         for (uint64_t i = a0 + l; i < a1; i += SG_SAMPLE_G) {
             const uint64_t e = boff[acols[i] + 1ull];
             for (uint64_t q = boff[acols[i]]; q < e; ++q) {
                 const uint32_t c = bcols[q];
-                uint32_t h = (c * 0x9E3779B1u) >> 26;
-                while (true) {  // (at most SLOTS columns: it ends)
+                uint32_t h = (c * 0x9E3779B1u) >> 25;
+                while (true) {  // (at most SPGEMM_HASH_MAX columns: it ends)
                     const uint32_t was = atomicCAS(&key[h], EMPTY, c);
                     if (was == EMPTY) ++distinct;
                     if (was == EMPTY || was == c) break;
@@ -114,23 +115,20 @@ sg_row_products(const uint64_t *__restrict__ aoff, const uint32_t *__restrict__ 
     int score = 0;
     if (i < m) {
         const uint64_t a0 = aoff[i], a1 = aoff[i + 1];
-        uint32_t first = 0;
         for (uint64_t ka = a0; ka < a1; ++ka) {
             const uint32_t k = acols[ka];
             s += boff[k + 1] - boff[k];
-            if (ka == a0) first = k;
-            else if (ka == a0 + 1) score = k - first < near ? 1 : -1;
         }
+        if (a1 - a0 > 1) score = acols[a0 + 1] - acols[a0] < near ? 1 : -1;
     }
-    score = __reduce_add_sync(0xffffffffu, score);
     if (i <= m) cnt[i] = s;
-    unsigned long long sum = s, over = s > (unsigned long long)SPGEMM_HASH_MAX ? 1 : 0;
+    score = __reduce_add_sync(0xffffffffu, score);
+    unsigned over = __popc(__ballot_sync(0xffffffffu, s > (unsigned long long)SPGEMM_HASH_MAX));
+    unsigned long long sum = s;
 #pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        over += __shfl_xor_sync(0xffffffffu, over, o);
-    }
-    __shared__ unsigned long long s_s[GB / 32], s_o[GB / 32];
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    __shared__ unsigned long long s_s[GB / 32];
+    __shared__ unsigned s_o[GB / 32];
     __shared__ int s_near[GB / 32];
     if ((threadIdx.x & 31) == 0) {
         s_s[threadIdx.x >> 5] = sum;
@@ -145,7 +143,7 @@ sg_row_products(const uint64_t *__restrict__ aoff, const uint32_t *__restrict__ 
             score += s_near[w];
         }
         if (sum) atomicAdd(ctr, sum);
-        if (over) atomicAdd(ctr + 1, over);
+        if (over) atomicAdd(ctr + 1, (unsigned long long)over);
         if (score) atomicAdd(ctr + 2, (unsigned long long)(long long)score);
         if (last_block(ctr + 5)) {
             for (int k = 0; k < 5; ++k) store_word(words, k, *(volatile unsigned long long *)(ctr + k));
@@ -537,7 +535,7 @@ int spgemm_products(Ctx *c, const Csr *A, const Csr *B, DevBuf *pofs, uint64_t *
     if (expected) {
         *expected = *P;
         if (sample && c->word(3) && *P > RESULT_BOUND)
-            *expected = std::min(*P, (uint64_t)((double)*P * (double)c->word(4) / (double)c->word(3)) + *P / 32);
+            *expected = std::min(*P, (uint64_t)((double)*P * (double)c->word(4) / (double)c->word(3) * (13.0 / 12.0)));  // (under fit_arrays' eighth)
     }
     if (*P >= (1ull << 32))
         return set_error(SPG_ERR_UNSUPPORTED, "spgemm: %llu products exceed 2^32-1", (unsigned long long)*P);
