@@ -355,7 +355,18 @@ __device__ __forceinline__ void store_word(unsigned long long *words, int k, uns
     *(volatile unsigned long long *)(words + k) = v;
 }
 
-// The same for a host that reads the word while the kernel runs (Ctx::wait_word),
+// words[0 .. N) from N counters that other blocks added to: all are read before
+// the first is stored (one after another, each store waits for its read).
+template <int N, class T>
+__device__ __forceinline__ void store_counters(unsigned long long *words, const T *ctr) {
+    T v[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = *(const volatile T *)(ctr + k);
+#pragma unroll
+    for (int k = 0; k < N; ++k) store_word(words, k, v[k]);
+}
+
+// store_word for a host that reads the word while the kernel runs (Ctx::wait_word),
 // after what the thread stored before.
 __device__ __forceinline__ void store_word_now(unsigned long long *words, int k, unsigned long long v) {
     __threadfence_system();

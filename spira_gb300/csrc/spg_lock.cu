@@ -224,9 +224,7 @@ __global__ void lock_prepare(const uint32_t *__restrict__ rows, const uint32_t *
         if (bf & 8u) stats[6] = 1u;
         if (bt) atomicAdd(stats + 8, bt);
         if (bd) atomicAdd(stats + 9, bd);
-        if (last_block(stats + N_STATS)) {
-            for (int i = 0; i < N_STATS; ++i) store_word(words, i, *(volatile unsigned *)(stats + i));
-        }
+        if (last_block(stats + N_STATS)) store_counters<N_STATS>(words, stats);
     }
 }
 

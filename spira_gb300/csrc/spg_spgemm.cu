@@ -145,9 +145,7 @@ sg_row_products(const uint64_t *__restrict__ aoff, const uint32_t *__restrict__ 
         if (sum) atomicAdd(ctr, sum);
         if (over) atomicAdd(ctr + 1, (unsigned long long)over);
         if (score) atomicAdd(ctr + 2, (unsigned long long)(long long)score);
-        if (last_block(ctr + 5)) {
-            for (int k = 0; k < 5; ++k) store_word(words, k, *(volatile unsigned long long *)(ctr + k));
-        }
+        if (last_block(ctr + 5)) store_counters<SAMPLE ? 5 : 3>(words, ctr);
     }
 }
 
