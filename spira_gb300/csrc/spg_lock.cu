@@ -89,8 +89,9 @@ __device__ __forceinline__ uint32_t column_gap(uint32_t a, uint32_t b) { return 
 // sample of the inserts that are of one row with the 32nd and the 64th after
 // them (an eighth of all), stats[9] += a sample of those whose successor is of an
 // earlier row (every fourth): what they say of inserts in no order, hub_rows below.
-// Both with HUBS only, for up to FEW_STAGED inserts: the registers that they take
-// cost 18 us of 132 for 64 M inserts, and nothing while the blocks are few.
+// Both with HUBS only, for up to FEW_STAGED inserts and for later epochs: the
+// registers that they take cost 18 us of 132 for 64 M inserts, and nothing while
+// the blocks are few.
 constexpr int N_STATS = 10;
 
 template <bool VEC, bool HUBS>
@@ -563,9 +564,8 @@ struct Prepared {
 // all (row sort, attempt and tiles / global, later epochs: 2.5 M in 10 rows 499 /
 // 392 us, 3 M in 200 rows 701 / 507), in small epochs from a tenth on (5 rows of
 // 13 000 430 / 351, and 100 k others 468 / 393), where launches are what is paid;
-// below, it is faster (12 M with one row of 2 M: 979 / 1461). Above 4 M inserts
-// nothing is sampled, and the plan of the tiles finds out (10 M in 10 rows 1073 /
-// 831).
+// below, it is faster (12 M with one row of 2 M: 979 / 1461). First locks of more
+// than 4 M inserts are not sampled: the plan of the tiles finds out.
 constexpr uint64_t HUB_FEW = 1u << 19;
 
 bool hub_rows(const Prepared &pre, uint64_t m) {
@@ -1073,7 +1073,7 @@ static int lock_device_impl(Ctx *c, Csr *A, const uint32_t *rows, const uint32_t
         SPG_TRY(stats.alloc((N_STATS + 1) * sizeof(unsigned), s));
         SPG_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, (N_STATS + 1) * sizeof(unsigned), s));
         if (!A->built) SPG_TRY(pre.off.alloc(csr_off_elems(A->n_rows) * sizeof(uint64_t), s));
-        const bool vec = ((uintptr_t)rows | (uintptr_t)cols) % 16 == 0, hubs = m <= FEW_STAGED;
+        const bool vec = ((uintptr_t)rows | (uintptr_t)cols) % 16 == 0, hubs = m <= FEW_STAGED || A->built;
         auto k = vec ? (hubs ? lock_prepare<true, true> : lock_prepare<true, false>)
                      : (hubs ? lock_prepare<false, true> : lock_prepare<false, false>);
         k<<<grid_for(vec ? (m + 3) / 4 : m, LB, (unsigned)c->n_sms * 16), LB, 0, s>>>(
