@@ -1,5 +1,5 @@
 // spg_spgemm_hash.cu — the row merge of SPG_SPGEMM_ROWMERGE when no row of A
-// has more than SH_H products: C = A * B in Spira's Gustavson order
+// has more than SH_H products (and not many rows few): C = A * B in Spira's Gustavson order
 // (serial/spgemm.hpp:28-48), written to its final place in one pass.
 //
 // Eight lanes take a row. They walk its A entries in ascending k, each lane one
