@@ -44,6 +44,7 @@ int Ctx::wait_word(int k, cudaStream_t s) {
         if (e == cudaSuccess) break;
         if (e != cudaErrorNotReady) SPG_CUDA_TRY(e);
     }
+    std::atomic_thread_fence(std::memory_order_acquire);  // the words stored before it, on a host that reorders loads
     return SPG_OK;
 }
 
